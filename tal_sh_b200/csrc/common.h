@@ -3,6 +3,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <vector>
 
 #include "talsh.h"
 #include "talsh_b200.h"
@@ -50,6 +51,12 @@ inline double contract_flops(int kind, const int *cptrn, int lrank, const int *l
 // sign of the real part (reference cmplx8_to_real8, tensor_algebra_cpu.F90:430-445).
 double cmplx8_to_real8(double re, double im);
 
+// Scratch of one tcTensorContract call: the size that lets it split a long
+// contracted range over CTAs, and in *least (may be null) the size below which
+// the call is refused.
+size_t contract_scratch_bytes(int kind, const int *cptrn, int drank, const int *ddims, int lrank,
+                              const int *ldims, int rrank, const int *rdims, size_t *least);
+
 // Bookkeeping shared by the CUDA translation units.
 void note_launch(unsigned n = 1);
 void note_cuda_error(const char *what, int code);
@@ -63,10 +70,11 @@ int current_sm_count();
 // stays untouched until the launch's upload has run (nullptr refuses: the
 // call returns TRY_LATER).
 using BatchScratchFn = void *(*)(void *ctx, size_t scratch_bytes, size_t stage_bytes, void **stage);
-int batch_launch_with(int ntasks, const tcContractTask *tasks, BatchScratchFn get, void *ctx, void *stream);
+int batch_launch_with(int ntasks, const tcContractTask *tasks, const std::vector<char> *lean, BatchScratchFn get,
+                      void *ctx, void *stream);
 // A batch's scratch is at most batch_fixed_scratch() plus the sum of
-// batch_task_scratch_bound over its tasks.
-size_t batch_task_scratch_bound(const tcContractTask &task);
+// batch_task_scratch_bound over its tasks (lean tasks have no partial sums).
+size_t batch_task_scratch_bound(const tcContractTask &task, bool lean);
 size_t batch_fixed_scratch();
 
 }  // namespace tb

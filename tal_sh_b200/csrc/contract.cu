@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "common.h"
@@ -48,9 +49,13 @@ struct TableParams {
   int64_t hext[kMaxGR], hstrL[kMaxGR], hstrR[kMaxGR], hstrD[kMaxGR];
   int64_t *mL, *mD, *nR, *nD, *kL, *kR;
   int64_t *hL, *hR, *hD;  // used when nh > 0
+  int *cnt;               // arrival counters to zero (split contracted range)
+  int64_t ncnt;
 };
 
 __global__ void build_tables_kernel(const TableParams T) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < T.ncnt; i += (int64_t)gridDim.x * blockDim.x)
+    T.cnt[i] = 0;
   const int64_t mnk = T.M + T.N + T.K;
   const int64_t total = mnk + (T.nh > 0 ? T.H : 0);
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -113,13 +118,31 @@ struct GemmArgs {
   int a_along_m;  // A tile loads: lanes along m (else along k)
   int b_along_n;  // B tile loads: lanes along n (else along k)
   int conj_l, conj_r;
+  // Split contracted range (nsplit > 1): CTA (tile, s) sums k in
+  // [s kchunk, (s+1) kchunk) and the partial tiles meet in `part`.
+  int nsplit, kchunk, gsz;
+  int ncnt;   // arrival counters of this contraction (zeroed by the table kernel)
+  void *part;
+  int *cnt;
 };
 
-// Hyper-index launches: block b runs tile b mod tiles_mn of the GEMM for
-// hyper combination b / tiles_mn, whose operands start at the table offsets.
+// One CTA's work: output tile (tm, tn) of one GEMM, the K range of its split,
+// and the tile's number among all tiles of the launch (partial sums).
+struct TileWork {
+  int tm, tn, split, lin;
+};
+
+// Single-contraction launches: block b runs tile b mod tiles_mn of the GEMM for
+// hyper combination (b / tiles_mn) mod H, whose operands start at the table
+// offsets; the splits of the contracted range are the slowest index, so the
+// CTAs in flight share their operands' k range in L2.
 template <typename T>
-__device__ __forceinline__ int hyper_offsets(const GemmArgs &a, const T *&L, const T *&R, T *&D) {
-  int local = (int)blockIdx.x;
+__device__ __forceinline__ TileWork block_work(const GemmArgs &a, const T *&L, const T *&R, T *&D) {
+  const int per = a.tiles_mn * (a.H > 1 ? a.H : 1);
+  TileWork w;
+  w.split = a.nsplit > 1 ? (int)blockIdx.x / per : 0;
+  w.lin = (int)blockIdx.x - w.split * per;
+  int local = w.lin;
   if (a.hL != nullptr) {
     const int h = local / a.tiles_mn;
     local -= h * a.tiles_mn;
@@ -127,7 +150,64 @@ __device__ __forceinline__ int hyper_offsets(const GemmArgs &a, const T *&L, con
     R += a.hR[h];
     D += a.hD[h];
   }
-  return local;
+  w.tm = local % a.tiles_m;
+  w.tn = local / a.tiles_m;
+  return w;
+}
+
+// Fragment arithmetic of the partial sums.
+__device__ __forceinline__ void vadd(double2 &a, const double2 &b) { a.x += b.x; a.y += b.y; }
+__device__ __forceinline__ void vadd(float4 &a, const float4 &b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; }
+
+// Meeting point of the CTAs that share an output tile (nsplit > 1).  Each CTA
+// stores its partial fragments (16 bytes per slot, coalesced, at the thread's
+// position `pos` in the tile; `mask` drops fragments beyond the tile's extents)
+// and counts itself in; the last
+// CTA of a group of gsz splits adds that group's partials in split order, and
+// the last group adds the group sums in group order, so no CTA ever waits and
+// the sum order does not depend on arrival.  Two levels keep the serial part
+// at about 2 sqrt(nsplit) tile reads: one CTA adding 444 partial 64 x 64 tiles
+// alone would read 14.5 MB.  Returns true in the CTA that holds the final sum.
+// Counters go back to zero, so a recorded launch can be replayed.
+template <int NF, int NT, typename V>
+__device__ __forceinline__ bool split_combine(V (&acc)[NF], uint32_t mask, int pos, const GemmArgs &a, int lin,
+                                              int split) {
+  __shared__ int last;
+  const int tid = threadIdx.x;
+  V *base = (V *)a.part + (int64_t)lin * a.nsplit * (NF * NT) + pos;
+  const int ng = (a.nsplit + a.gsz - 1) / a.gsz, g = split / a.gsz, s0 = g * a.gsz;
+  const int gm = min(a.gsz, a.nsplit - s0);
+  int *cnt = a.cnt + (int64_t)lin * (ng + 1);
+  auto publish = [&](int s, int *c, int want) {
+    V *to = base + (int64_t)s * (NF * NT);
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+      if ((mask >> f) & 1u) __stcg(to + f * NT, acc[f]);
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) last = atomicAdd(c, 1) == want - 1 ? 1 : 0;
+    __syncthreads();
+    if (last && tid == 0) *c = 0;
+    __threadfence();
+    return last != 0;
+  };
+  auto gather = [&](int s, int n, int step) {
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+      if ((mask >> f) & 1u) acc[f] = __ldcg(base + (int64_t)s * (NF * NT) + f * NT);
+    for (int j = 1; j < n; ++j) {
+      const V *from = base + (int64_t)(s + j * step) * (NF * NT);
+#pragma unroll
+      for (int f = 0; f < NF; ++f)
+        if ((mask >> f) & 1u) vadd(acc[f], __ldcg(from + f * NT));
+    }
+  };
+  if (!publish(split, cnt + g, gm)) return false;
+  gather(s0, gm, 1);
+  if (ng == 1) return true;
+  if (!publish(s0, cnt + ng, ng)) return false;
+  gather(0, ng, a.gsz);
+  return true;
 }
 
 // ---------------------------------------------------------------- R8: DMMA
@@ -135,6 +215,10 @@ __device__ __forceinline__ void cp_async8(void *smem_ptr, const void *gptr, bool
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem_ptr);
   const int n = valid ? 8 : 0;
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gptr), "r"(n));
+}
+__device__ __forceinline__ void cp_async8(void *smem_ptr, const void *gptr) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem_ptr);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gptr));
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
@@ -146,58 +230,108 @@ __device__ __forceinline__ void dmma_8x8x4(double &c0, double &c1, double a, dou
                : "d"(a), "d"(b));
 }
 
+constexpr int kKRing = 4;  // slots of the shared k-offset ring
+
 template <int BM, int BN>
 struct DmmaCfg {
-  // warp tile: 32x32, or 16x16 in 32x32 CTA tiles (four warps per small tile)
+  // warp tile: 32x32, or 16x16 in 32x32 CTA tiles (four warps per CTA either way)
   static constexpr int WM = BM <= 32 ? 16 : 32, WN = BN <= 32 ? 16 : 32;
   static constexpr int WARPS_M = BM / WM, WARPS_N = BN / WN;
   static constexpr int THREADS = WARPS_M * WARPS_N * 32;
   static constexpr int BK = 16, STAGES = 3;
-  static constexpr int AP = BM + 8, BP = BN + 8;    // pitches: 2-wavefront fragment loads
+  static constexpr int AP = BM + 4, BP = BN + 4;    // pitches: conflict-free fragment loads
   static constexpr size_t SMEM = (size_t)STAGES * BK * (AP + BP) * sizeof(double) +
-                                 (size_t)(2 * BM + 2 * BN + 2 * STAGES * BK) * sizeof(int64_t);
+                                 (size_t)(2 * BM + 2 * BN + 2 * kKRing * BK) * sizeof(int64_t);
 };
 
-// k-offset tables of the tiles in flight live in a shared ring (slot t % ST
-// holds tile t's BK entries of kL and kR).  The tables of tiles 0..ST-1 are
-// written before the main loop; afterwards warp 0 fetches tile t+ST's entries
-// from global memory during iteration t and stores them at its end, so the
-// address of a cp.async never waits for a global load.
+// k-offset tables of the k-tiles in flight live in a shared ring (slot t % 4
+// holds tile t's BK entries of kL and kR, k counted from the split's first).
+// Tiles 0..ST are fetched before the main loop; iteration t copies tile
+// t+ST+1's entries asynchronously with its own load group, two iterations
+// before the loads that use them, so neither an address nor an iteration waits
+// for a table read (fetched through registers one iteration ahead, the reads'
+// latency bounded every k step of thin tiles).
 template <int BK, int ST>
-__device__ __forceinline__ void kring_init(const GemmArgs &a, int64_t *kLs, int64_t *kRs, int tid, int nt,
-                                           int64_t &pf) {
-  for (int i = tid; i < ST * BK; i += nt) {
-    kLs[i] = i < a.K ? a.kL[i] : 0;
-    kRs[i] = i < a.K ? a.kR[i] : 0;
-  }
-  if (tid < 2 * BK) {
-    const int k = ST * BK + (tid % BK);
-    pf = k < a.K ? (tid < BK ? a.kL[k] : a.kR[k]) : 0;
+__device__ __forceinline__ void kring_init(const int64_t *kL, const int64_t *kR, int K, int64_t *kLs, int64_t *kRs,
+                                           int tid, int nt) {
+  static_assert(ST + 1 <= kKRing, "prefetched tiles fit the ring");
+  for (int i = tid; i < (ST + 1) * BK; i += nt) {
+    kLs[i] = i < K ? kL[i] : 0;
+    kRs[i] = i < K ? kR[i] : 0;
   }
 }
 template <int BK, int ST>
-__device__ __forceinline__ void kring_step(const GemmArgs &a, int64_t *kLs, int64_t *kRs, int tid, int kt,
-                                           int64_t &pf) {
+__device__ __forceinline__ void kring_step(const int64_t *kL, const int64_t *kR, int K, int64_t *kLs, int64_t *kRs,
+                                           int tid, int kt) {
+  static_assert(2 * BK == 32, "one warp copies both tables of a tile");
   if (tid < 2 * BK) {
-    const int j = tid % BK;
-    (tid < BK ? kLs : kRs)[(kt % ST) * BK + j] = pf;
-    const int64_t k = (int64_t)(kt + ST + 1) * BK + j;
-    pf = k < a.K ? (tid < BK ? a.kL[k] : a.kR[k]) : 0;
+    const int j = tid % BK, t = kt + ST + 1;
+    const int64_t k = (int64_t)t * BK + j;
+    const int64_t *from = tid < BK ? kL : kR;
+    cp_async8((tid < BK ? kLs : kRs) + (t % kKRing) * BK + j, from + (k < K ? k : 0), k < K);
   }
 }
 
-// Column swizzle of the FP64 tiles: row k stores column c at c ^ ((k >> 1) & 7)
-// (a permutation inside each aligned group of 8 columns).  Tile loads whose
-// lanes run along k (the operand's stride-1 index is contracted) then hit 16
-// different bank pairs per half-warp instead of 2; fragment loads, which read
-// 8 consecutive columns of one row, are unaffected.
-__device__ __forceinline__ int kswz(int k) { return (k >> 1) & 7; }
+// Column swizzle of the FP64 tiles: row k stores column c at c ^ ((k >> 2) & 3).
+// With rows 8 banks apart (pitch BM + 4 doubles) a fragment load's four k-rows
+// fill all 32 banks, and tile loads whose lanes run along k (the operand's
+// stride-1 index is contracted) hit 16 different bank pairs per half-warp.
+__device__ __forceinline__ int kswz(int k) { return (k >> 2) & 3; }
+
+// Valid 8-row fragments of warp `w` of `W` along one tile dimension with `rem`
+// rows left: fragment i of the warp covers rows (i W + w) 8.  Interleaving the
+// warps' fragments spreads a ragged tile's valid ones over all warps.
+__device__ __forceinline__ int frag_count(int rem, int w, int W, int F) {
+  return max(0, min(F, (rem - w * 8 + 8 * W - 1) / (8 * W)));
+}
+
+// Portion Q of P of one operand's loads of a k-tile: X free-index rows (`rem`
+// of them inside the tensor) by BK k-rows, each element at fs[row] + ks[k].
+// `along`: lanes run along the free index, else along k; the two forms keep
+// their index arithmetic to constant strides, so an element costs an offset
+// read, an add and the copy.  TAIL: k-rows from `klim` on are zero-filled.
+template <int X, int BK, int NT, int PITCH, bool SWZ, int Q, int P, bool TAIL, typename T, typename Put>
+__device__ __forceinline__ void load_side(const T *__restrict__ G, const int64_t *fs, const int64_t *ks, T *dst,
+                                          int along, int rem, int klim, const Put &put) {
+  constexpr int N = (X * BK) / NT;
+  const int tid = threadIdx.x;
+  if (along) {
+    static_assert(NT % X == 0, "a thread keeps its row");
+    constexpr int S = NT / X;  // k-rows between a thread's elements
+    static_assert(!SWZ || S <= 4, "the swizzle does not depend on t0");
+    const int x = tid % X, t0 = tid / X;
+    if (x >= rem) return;
+    const T *g = G + fs[x];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      if (i * P / N != Q) continue;
+      const bool v = !TAIL || t0 + i * S < klim;
+      const int c = SWZ ? x ^ kswz(i * S) : x;  // kswz(t0 + i S): t0 < S <= 4, a power of two
+      put(dst + t0 * PITCH + c + i * S * PITCH, g + (v ? ks[t0 + i * S] : 0), v);
+    }
+  } else {
+    const int kl = tid % BK, t0 = tid / BK;
+    constexpr int S = NT / BK;  // rows between a thread's elements (a multiple of 8)
+    const bool v = !TAIL || kl < klim;
+    const T *g = G + (v ? ks[kl] : 0);
+    T *d = dst + kl * PITCH + (SWZ ? t0 ^ kswz(kl) : t0);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      if (i * P / N != Q) continue;
+      if (t0 + i * S < rem) put(d + i * S, g + fs[t0 + i * S], v);
+    }
+  }
+}
 
 // One BM x BN tile of a gather-GEMM (shared by the single-contraction kernel and
-// the batched one).
+// the batched one) over the k range of its split.  The loads of the tile
+// ST - 1 ahead are issued in BK / 4 portions between the tensor-pipe steps:
+// issued in one block after the barrier they left the pipe idle in every warp
+// at once.  Rows and columns beyond the tensor are neither loaded (their stale
+// shared values only reach outputs that are not stored) nor multiplied.
 template <int BM, int BN>
 __device__ __forceinline__ void dmma_tile(const double *__restrict__ L, const double *__restrict__ R,
-                                          double *D, const GemmArgs &a, int tile_m, int tile_n,
+                                          double *D, const GemmArgs &a, const TileWork &w,
                                           unsigned char *smem) {
   using C = DmmaCfg<BM, BN>;
   constexpr int BK = C::BK, ST = C::STAGES, AP = C::AP, BP = C::BP, NT = C::THREADS;
@@ -208,11 +342,14 @@ __device__ __forceinline__ void dmma_tile(const double *__restrict__ L, const do
   int64_t *nRs = mDs + BM;
   int64_t *nDs = nRs + BN;
   int64_t *kLs = nDs + BN;
-  int64_t *kRs = kLs + ST * BK;
-  int64_t pf = 0;
+  int64_t *kRs = kLs + kKRing * BK;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int m0 = tile_m * BM, n0 = tile_n * BN;
+  const int m0 = w.tm * BM, n0 = w.tn * BN;
+  const int mrem = a.M - m0, nrem = a.N - n0;
+  const int k0 = a.nsplit > 1 ? w.split * a.kchunk : 0;
+  const int K = a.nsplit > 1 ? min(a.kchunk, a.K - k0) : a.K;
+  const int64_t *kLg = a.kL + k0, *kRg = a.kR + k0;
   for (int i = tid; i < BM; i += NT) {
     const int m = m0 + i;
     mLs[i] = m < a.M ? a.mL[m] : 0;
@@ -223,89 +360,115 @@ __device__ __forceinline__ void dmma_tile(const double *__restrict__ L, const do
     nRs[i] = n < a.N ? a.nR[n] : 0;
     nDs[i] = n < a.N ? a.nD[n] : 0;
   }
-  kring_init<BK, ST>(a, kLs, kRs, tid, NT, pf);
+  kring_init<BK, ST>(kLg, kRg, K, kLs, kRs, tid, NT);
   __syncthreads();
 
-  const int numK = (a.K + BK - 1) / BK;
-  auto load_tile = [&](int kt, int s) {
-    double *as = As + s * BK * AP;
-    double *bs = Bs + s * BK * BP;
-#pragma unroll
-    for (int i = 0; i < (BM * BK) / NT; ++i) {
-      const int idx = tid + i * NT;
-      const int ml = a.a_along_m ? (idx % BM) : (idx / BK);
-      const int kl = a.a_along_m ? (idx / BM) : (idx % BK);
-      const int m = m0 + ml, k = kt * BK + kl;
-      const bool v = (m < a.M) && (k < a.K);
-      const double *src = v ? (L + mLs[ml] + kLs[s * BK + kl]) : L;
-      cp_async8(as + kl * AP + (ml ^ kswz(kl)), src, v);
-    }
-#pragma unroll
-    for (int i = 0; i < (BN * BK) / NT; ++i) {
-      const int idx = tid + i * NT;
-      const int nl = a.b_along_n ? (idx % BN) : (idx / BK);
-      const int kl = a.b_along_n ? (idx / BN) : (idx % BK);
-      const int n = n0 + nl, k = kt * BK + kl;
-      const bool v = (n < a.N) && (k < a.K);
-      const double *src = v ? (R + nRs[nl] + kRs[s * BK + kl]) : R;
-      cp_async8(bs + kl * BP + (nl ^ kswz(kl)), src, v);
-    }
+  const int numK = (K + BK - 1) / BK;
+  // Portion Q of P of the loads of k-tile kt into stage s.
+  const int along_a = a.a_along_m, along_b = a.b_along_n;
+  auto load_as = [&](int kt, int s, auto q, auto parts, auto tail) {
+    constexpr int Q = decltype(q)::value, P = decltype(parts)::value;
+    constexpr bool TAIL = decltype(tail)::value;
+    auto put = [](double *dst, const double *src, bool v) {
+      if constexpr (TAIL) cp_async8(dst, src, v);
+      else cp_async8(dst, src);
+    };
+    const int kr = (kt % kKRing) * BK, klim = K - kt * BK;
+    load_side<BM, BK, NT, AP, true, Q, P, TAIL>(L, mLs, kLs + kr, As + s * BK * AP, along_a, mrem, klim, put);
+    load_side<BN, BK, NT, BP, true, Q, P, TAIL>(R, nRs, kRs + kr, Bs + s * BK * BP, along_b, nrem, klim, put);
   };
+  auto load_part = [&](int kt, int s, auto q, auto parts) {
+    if ((kt + 1) * BK <= K) load_as(kt, s, q, parts, std::false_type{});
+    else if (kt * BK < K) load_as(kt, s, q, parts, std::true_type{});
+  };
+  using Int0 = std::integral_constant<int, 0>;
+  using Int1 = std::integral_constant<int, 1>;
+  using Int2 = std::integral_constant<int, 2>;
+  using Int3 = std::integral_constant<int, 3>;
+  using Int4 = std::integral_constant<int, 4>;
 
   constexpr int FM = C::WM / 8, FN = C::WN / 8;
-  double acc[FM][FN][2];
+  double2 acc[FM * FN];
 #pragma unroll
-  for (int i = 0; i < FM; ++i)
-#pragma unroll
-    for (int j = 0; j < FN; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  for (int f = 0; f < FM * FN; ++f) acc[f] = make_double2(0.0, 0.0);
 
-  const int wm0 = (warp % C::WARPS_M) * C::WM, wn0 = (warp / C::WARPS_M) * C::WN;
+  // Ragged tiles give the low warp positions more fragments; rotating the
+  // positions by CTA spreads them over the SM's four tensor pipes.
+  const int wr = (warp + w.lin + w.split) % (C::WARPS_M * C::WARPS_N);
+  const int wm = wr % C::WARPS_M, wn = wr / C::WARPS_M;
   const int fr = lane >> 2, fc = lane & 3;
+  const int fm = frag_count(mrem, wm, C::WARPS_M, FM), fn = frag_count(nrem, wn, C::WARPS_N, FN);
 
 #pragma unroll
   for (int s = 0; s < ST - 1; ++s) {
-    if (s < numK) load_tile(s, s);
+    load_part(s, s, Int0{}, Int1{});
     cp_async_commit();
   }
-  for (int kt = 0; kt < numK; ++kt) {
-    cp_async_wait<ST - 2>();
-    __syncthreads();
-    const int pre = kt + ST - 1;
-    if (pre < numK) load_tile(pre, pre % ST);
-    cp_async_commit();
-    const double *as = As + (kt % ST) * BK * AP;
-    const double *bs = Bs + (kt % ST) * BK * BP;
+  auto main_loop = [&](auto full_c) {
+    constexpr bool FULL = decltype(full_c)::value;
+    int st = 0, ps = ST - 1;  // stage of tile kt, stage filled during iteration kt
+    for (int kt = 0; kt < numK; ++kt) {
+      cp_async_wait<ST - 2>();
+      __syncthreads();
+      const double *as = As + (st * BK + fc) * AP + wm * 8;
+      const double *bs = Bs + (st * BK + fc) * BP + wn * 8;
+      auto step = [&](auto ksc) {
+        constexpr int ks = decltype(ksc)::value;
+        double af[FM], bf[FN];
+        const double *ap = as + (fr ^ ks), *bp = bs + (fr ^ ks);  // kswz(4 ks + fc) = ks
 #pragma unroll
-    for (int ks = 0; ks < BK / 4; ++ks) {
-      double af[FM], bf[FN];
-      const int sw = kswz(ks * 4 + fc);
+        for (int i = 0; i < FM; ++i) af[i] = ap[ks * 4 * AP + i * C::WARPS_M * 8];
 #pragma unroll
-      for (int i = 0; i < FM; ++i) af[i] = as[(ks * 4 + fc) * AP + wm0 + i * 8 + (fr ^ sw)];
+        for (int j = 0; j < FN; ++j) bf[j] = bp[ks * 4 * BP + j * C::WARPS_N * 8];
 #pragma unroll
-      for (int j = 0; j < FN; ++j) bf[j] = bs[(ks * 4 + fc) * BP + wn0 + j * 8 + (fr ^ sw)];
+        for (int i = 0; i < FM; ++i) {
+          if (!FULL && i >= fm) break;
 #pragma unroll
-      for (int i = 0; i < FM; ++i)
-#pragma unroll
-        for (int j = 0; j < FN; ++j) dmma_8x8x4(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+          for (int j = 0; j < FN; ++j)
+            if (FULL || j < fn) dmma_8x8x4(acc[i * FN + j].x, acc[i * FN + j].y, af[i], bf[j]);
+        }
+        load_part(kt + ST - 1, ps, ksc, Int4{});
+      };
+      step(Int0{});
+      step(Int1{});
+      step(Int2{});
+      step(Int3{});
+      kring_step<BK, ST>(kLg, kRg, K, kLs, kRs, tid, kt);
+      cp_async_commit();
+      ps = st;
+      st = st + 1 == ST ? 0 : st + 1;
     }
-    kring_step<BK, ST>(a, kLs, kRs, tid, kt, pf);
-  }
+  };
+  if (fm == FM && fn == FN) main_loop(std::true_type{});
+  else main_loop(std::false_type{});
   cp_async_wait<0>();
 
+  if (a.nsplit > 1) {
+    uint32_t mask = 0;
+#pragma unroll
+    for (int f = 0; f < FM * FN; ++f)
+      if (f / FN < fm && f % FN < fn) mask |= 1u << f;
+    if (!split_combine<FM * FN, NT>(acc, mask, wr * 32 + lane, a, w.lin, w.split)) return;
+  }
+  // Epilogue: the D values of a fragment row are all loaded before any is
+  // stored (the compiler cannot move a load above a store that may alias it).
   const double alpha = a.alpha_re;
 #pragma unroll
   for (int i = 0; i < FM; ++i) {
-    const int ml = wm0 + i * 8 + fr;
-    if (m0 + ml >= a.M) continue;
+    const int ml = (i * C::WARPS_M + wm) * 8 + fr;
+    if (ml >= mrem) continue;
+    double *p[FN * 2];
+    double d[FN * 2];
 #pragma unroll
-    for (int j = 0; j < FN; ++j) {
+    for (int j = 0; j < FN * 2; ++j) {
+      const int nl = ((j / 2) * C::WARPS_N + wn) * 8 + fc * 2 + (j & 1);
+      p[j] = nl < nrem ? D + mDs[ml] + nDs[nl] : nullptr;
+      d[j] = (a.beta && p[j]) ? *p[j] : 0.0;
+    }
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int nl = wn0 + j * 8 + fc * 2 + h;
-        if (n0 + nl >= a.N) continue;
-        double *p = D + mDs[ml] + nDs[nl];
-        *p = a.beta ? fma(alpha, acc[i][j][h], *p) : alpha * acc[i][j][h];
-      }
+    for (int j = 0; j < FN * 2; ++j) {
+      const double v = (j & 1) ? acc[i * FN + j / 2].y : acc[i * FN + j / 2].x;
+      if (p[j]) *p[j] = a.beta ? fma(alpha, v, d[j]) : alpha * v;
     }
   }
 }
@@ -326,7 +489,7 @@ struct ZmmaCfg {
   static constexpr int BK = 16, STAGES = BM <= 32 ? 2 : 3;  // two stages keep five small CTAs per SM
   static constexpr int AP = BM + 2, BP = BN + 2;           // in complex elements
   static constexpr size_t SMEM = (size_t)STAGES * BK * (AP + BP) * sizeof(double2) +
-                                 (size_t)(2 * BM + 2 * BN + 2 * STAGES * BK) * sizeof(int64_t);
+                                 (size_t)(2 * BM + 2 * BN + 2 * kKRing * BK) * sizeof(int64_t);
 };
 
 __device__ __forceinline__ void cp_async16(void *smem_ptr, const void *gptr, bool valid) {
@@ -338,7 +501,7 @@ __device__ __forceinline__ void cp_async16(void *smem_ptr, const void *gptr, boo
 
 template <int BM, int BN>
 __device__ __forceinline__ void zmma_tile(const double2 *__restrict__ L, const double2 *__restrict__ R,
-                                          double2 *D, const GemmArgs &a, int tile_m, int tile_n,
+                                          double2 *D, const GemmArgs &a, const TileWork &w,
                                           unsigned char *smem) {
   using C = ZmmaCfg<BM, BN>;
   constexpr int BK = C::BK, ST = C::STAGES, AP = C::AP, BP = C::BP, NT = C::THREADS;
@@ -349,10 +512,13 @@ __device__ __forceinline__ void zmma_tile(const double2 *__restrict__ L, const d
   int64_t *nRs = mDs + BM;
   int64_t *nDs = nRs + BN;
   int64_t *kLs = nDs + BN;
-  int64_t *kRs = kLs + ST * BK;
-  int64_t pf = 0;
+  int64_t *kRs = kLs + kKRing * BK;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int m0 = tile_m * BM, n0 = tile_n * BN;
+  const int m0 = w.tm * BM, n0 = w.tn * BN;
+  const int mrem = a.M - m0, nrem = a.N - n0;
+  const int k0 = a.nsplit > 1 ? w.split * a.kchunk : 0;
+  const int K = a.nsplit > 1 ? min(a.kchunk, a.K - k0) : a.K;
+  const int64_t *kLg = a.kL + k0, *kRg = a.kR + k0;
   for (int i = tid; i < BM; i += NT) {
     const int m = m0 + i;
     mLs[i] = m < a.M ? a.mL[m] : 0;
@@ -363,126 +529,151 @@ __device__ __forceinline__ void zmma_tile(const double2 *__restrict__ L, const d
     nRs[i] = n < a.N ? a.nR[n] : 0;
     nDs[i] = n < a.N ? a.nD[n] : 0;
   }
-  kring_init<BK, ST>(a, kLs, kRs, tid, NT, pf);
+  kring_init<BK, ST>(kLg, kRg, K, kLs, kRs, tid, NT);
   __syncthreads();
-  const int numK = (a.K + BK - 1) / BK;
-  auto load_tile = [&](int kt, int s) {
-#pragma unroll
-    for (int i = 0; i < (BM * BK) / NT; ++i) {
-      const int idx = tid + i * NT;
-      const int ml = a.a_along_m ? (idx % BM) : (idx / BK);
-      const int kl = a.a_along_m ? (idx / BM) : (idx % BK);
-      const int m = m0 + ml, k = kt * BK + kl;
-      const bool v = (m < a.M) && (k < a.K);
-      const double2 *src = v ? (L + mLs[ml] + kLs[s * BK + kl]) : L;
-      cp_async16(As + (s * BK + kl) * AP + ml, src, v);
-    }
-#pragma unroll
-    for (int i = 0; i < (BN * BK) / NT; ++i) {
-      const int idx = tid + i * NT;
-      const int nl = a.b_along_n ? (idx % BN) : (idx / BK);
-      const int kl = a.b_along_n ? (idx / BN) : (idx % BK);
-      const int n = n0 + nl, k = kt * BK + kl;
-      const bool v = (n < a.N) && (k < a.K);
-      const double2 *src = v ? (R + nRs[nl] + kRs[s * BK + kl]) : R;
-      cp_async16(Bs + (s * BK + kl) * BP + nl, src, v);
-    }
+  const int numK = (K + BK - 1) / BK;
+  const int along_a = a.a_along_m, along_b = a.b_along_n;
+  auto load_as = [&](int kt, int s, auto q, auto parts, auto tail) {
+    constexpr int Q = decltype(q)::value, P = decltype(parts)::value;
+    constexpr bool TAIL = decltype(tail)::value;
+    auto put = [](double2 *dst, const double2 *src, bool v) { cp_async16(dst, src, v); };
+    const int kr = (kt % kKRing) * BK, klim = K - kt * BK;
+    load_side<BM, BK, NT, AP, false, Q, P, TAIL>(L, mLs, kLs + kr, As + s * BK * AP, along_a, mrem, klim, put);
+    load_side<BN, BK, NT, BP, false, Q, P, TAIL>(R, nRs, kRs + kr, Bs + s * BK * BP, along_b, nrem, klim, put);
   };
+  auto load_part = [&](int kt, int s, auto q, auto parts) {
+    if ((kt + 1) * BK <= K) load_as(kt, s, q, parts, std::false_type{});
+    else if (kt * BK < K) load_as(kt, s, q, parts, std::true_type{});
+  };
+  using Int0 = std::integral_constant<int, 0>;
+  using Int1 = std::integral_constant<int, 1>;
+  using Int2 = std::integral_constant<int, 2>;
+  using Int3 = std::integral_constant<int, 3>;
+  using Int4 = std::integral_constant<int, 4>;
   constexpr int FM = C::WM / 8, FN = C::WN / 8;
-  double cr[FM][FN][2], ci[FM][FN][2];
+  double2 acc[2 * FM * FN];  // fragment f: real parts at 2 f, imaginary parts at 2 f + 1
 #pragma unroll
-  for (int i = 0; i < FM; ++i)
-#pragma unroll
-    for (int j = 0; j < FN; ++j) cr[i][j][0] = cr[i][j][1] = ci[i][j][0] = ci[i][j][1] = 0.0;
-  const int wm0 = (warp % C::WARPS_M) * C::WM, wn0 = (warp / C::WARPS_M) * C::WN;
+  for (int f = 0; f < 2 * FM * FN; ++f) acc[f] = make_double2(0.0, 0.0);
+  // Ragged tiles give the low warp positions more fragments; rotating the
+  // positions by CTA spreads them over the SM's four tensor pipes.
+  const int wr = (warp + w.lin + w.split) % (C::WARPS_M * C::WARPS_N);
+  const int wm = wr % C::WARPS_M, wn = wr / C::WARPS_M;
   const int fr = lane >> 2, fc = lane & 3;
+  const int fm = frag_count(mrem, wm, C::WARPS_M, FM), fn = frag_count(nrem, wn, C::WARPS_N, FN);
   const double sl = a.conj_l ? -1.0 : 1.0, sr = a.conj_r ? -1.0 : 1.0;
 #pragma unroll
   for (int s = 0; s < ST - 1; ++s) {
-    if (s < numK) load_tile(s, s);
+    load_part(s, s, Int0{}, Int1{});
     cp_async_commit();
   }
-  for (int kt = 0; kt < numK; ++kt) {
-    cp_async_wait<ST - 2>();
-    __syncthreads();
-    const int pre = kt + ST - 1;
-    if (pre < numK) load_tile(pre, pre % ST);
-    cp_async_commit();
-    const int so = (kt % ST);
+  auto main_loop = [&](auto full_c) {
+    constexpr bool FULL = decltype(full_c)::value;
+    int st = 0, ps = ST - 1;
+    for (int kt = 0; kt < numK; ++kt) {
+      cp_async_wait<ST - 2>();
+      __syncthreads();
+      const double2 *as = As + (st * BK + fc) * AP + wm * 8 + fr;
+      const double2 *bs = Bs + (st * BK + fc) * BP + wn * 8 + fr;
+      auto step = [&](auto ksc) {
+        constexpr int ks = decltype(ksc)::value;
+        double ar[FM], ai[FM], nai[FM], br[FN], bi[FN];
 #pragma unroll
-    for (int ks = 0; ks < BK / 4; ++ks) {
-      double ar[FM], ai[FM], nai[FM], br[FN], bi[FN];
-#pragma unroll
-      for (int i = 0; i < FM; ++i) {
-        const double2 v = As[(so * BK + ks * 4 + fc) * AP + wm0 + i * 8 + fr];
-        ar[i] = v.x;
-        ai[i] = sl * v.y;
-        nai[i] = -ai[i];
-      }
-#pragma unroll
-      for (int j = 0; j < FN; ++j) {
-        const double2 v = Bs[(so * BK + ks * 4 + fc) * BP + wn0 + j * 8 + fr];
-        br[j] = v.x;
-        bi[j] = sr * v.y;
-      }
-#pragma unroll
-      for (int i = 0; i < FM; ++i)
+        for (int i = 0; i < FM; ++i) {
+          const double2 v = as[ks * 4 * AP + i * C::WARPS_M * 8];
+          ar[i] = v.x;
+          ai[i] = sl * v.y;
+          nai[i] = -ai[i];
+        }
 #pragma unroll
         for (int j = 0; j < FN; ++j) {
-          dmma_8x8x4(cr[i][j][0], cr[i][j][1], ar[i], br[j]);
-          dmma_8x8x4(cr[i][j][0], cr[i][j][1], nai[i], bi[j]);
-          dmma_8x8x4(ci[i][j][0], ci[i][j][1], ar[i], bi[j]);
-          dmma_8x8x4(ci[i][j][0], ci[i][j][1], ai[i], br[j]);
+          const double2 v = bs[ks * 4 * BP + j * C::WARPS_N * 8];
+          br[j] = v.x;
+          bi[j] = sr * v.y;
         }
+#pragma unroll
+        for (int i = 0; i < FM; ++i) {
+          if (!FULL && i >= fm) break;
+#pragma unroll
+          for (int j = 0; j < FN; ++j) {
+            if (!FULL && j >= fn) break;
+            double2 &cr = acc[2 * (i * FN + j)], &ci = acc[2 * (i * FN + j) + 1];
+            dmma_8x8x4(cr.x, cr.y, ar[i], br[j]);
+            dmma_8x8x4(cr.x, cr.y, nai[i], bi[j]);
+            dmma_8x8x4(ci.x, ci.y, ar[i], bi[j]);
+            dmma_8x8x4(ci.x, ci.y, ai[i], br[j]);
+          }
+        }
+        load_part(kt + ST - 1, ps, ksc, Int4{});
+      };
+      step(Int0{});
+      step(Int1{});
+      step(Int2{});
+      step(Int3{});
+      kring_step<BK, ST>(kLg, kRg, K, kLs, kRs, tid, kt);
+      cp_async_commit();
+      ps = st;
+      st = st + 1 == ST ? 0 : st + 1;
     }
-    kring_step<BK, ST>(a, kLs, kRs, tid, kt, pf);
-  }
+  };
+  if (fm == FM && fn == FN) main_loop(std::true_type{});
+  else main_loop(std::false_type{});
   cp_async_wait<0>();
+  if (a.nsplit > 1) {
+    uint32_t mask = 0;
+#pragma unroll
+    for (int f = 0; f < FM * FN; ++f)
+      if (f / FN < fm && f % FN < fn) mask |= 3u << (2 * f);
+    if (!split_combine<2 * FM * FN, NT>(acc, mask, wr * 32 + lane, a, w.lin, w.split)) return;
+  }
   const double alr = a.alpha_re, ali = a.alpha_im;
 #pragma unroll
   for (int i = 0; i < FM; ++i) {
-    const int ml = wm0 + i * 8 + fr;
-    if (m0 + ml >= a.M) continue;
+    const int ml = (i * C::WARPS_M + wm) * 8 + fr;
+    if (ml >= mrem) continue;
+    double2 *p[FN * 2];
+    double2 d[FN * 2];
 #pragma unroll
-    for (int j = 0; j < FN; ++j) {
+    for (int j = 0; j < FN * 2; ++j) {
+      const int nl = ((j / 2) * C::WARPS_N + wn) * 8 + fc * 2 + (j & 1);
+      p[j] = nl < nrem ? D + mDs[ml] + nDs[nl] : nullptr;
+      d[j] = (a.beta && p[j]) ? *p[j] : make_double2(0.0, 0.0);
+    }
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int nl = wn0 + j * 8 + fc * 2 + h;
-        if (n0 + nl >= a.N) continue;
-        double2 *p = D + mDs[ml] + nDs[nl];
-        const double vr = cr[i][j][h] * alr - ci[i][j][h] * ali;
-        const double vi = cr[i][j][h] * ali + ci[i][j][h] * alr;
-        if (a.beta) {
-          const double2 d = *p;
-          *p = make_double2(d.x + vr, d.y + vi);
-        } else {
-          *p = make_double2(vr, vi);
-        }
-      }
+    for (int j = 0; j < FN * 2; ++j) {
+      const double2 fr2 = acc[2 * (i * FN + j / 2)], fi2 = acc[2 * (i * FN + j / 2) + 1];
+      const double cr = (j & 1) ? fr2.y : fr2.x, ci = (j & 1) ? fi2.y : fi2.x;
+      const double vr = cr * alr - ci * ali;
+      const double vi = cr * ali + ci * alr;
+      if (p[j]) *p[j] = a.beta ? make_double2(d[j].x + vr, d[j].y + vi) : make_double2(vr, vi);
     }
   }
 }
 
+// Resident CTAs per SM asked of the compiler.
+template <int BM, int BN> struct GemmOcc { static constexpr int D = 1, Z = 1; };
+template <> struct GemmOcc<64, 64> { static constexpr int D = 4, Z = 2; };
+template <> struct GemmOcc<32, 32> { static constexpr int D = 6, Z = 5; };
+
 template <int BM, int BN>
-__global__ void __launch_bounds__(ZmmaCfg<BM, BN>::THREADS)
+__global__ void __launch_bounds__(ZmmaCfg<BM, BN>::THREADS, GemmOcc<BM, BN>::Z)
     zgemm_gather_kernel(const double2 *__restrict__ L, const double2 *__restrict__ R, double2 *D,
                         const GemmArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const double2 *Lp = L, *Rp = R;
   double2 *Dp = D;
-  const int local = hyper_offsets(a, Lp, Rp, Dp);
-  zmma_tile<BM, BN>(Lp, Rp, Dp, a, local % a.tiles_m, local / a.tiles_m, smem);
+  const TileWork w = block_work(a, Lp, Rp, Dp);
+  zmma_tile<BM, BN>(Lp, Rp, Dp, a, w, smem);
 }
 
 template <int BM, int BN>
-__global__ void __launch_bounds__(DmmaCfg<BM, BN>::THREADS)
+__global__ void __launch_bounds__(DmmaCfg<BM, BN>::THREADS, GemmOcc<BM, BN>::D)
     dgemm_gather_kernel(const double *__restrict__ L, const double *__restrict__ R, double *D,
                         const GemmArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const double *Lp = L, *Rp = R;
   double *Dp = D;
-  const int local = hyper_offsets(a, Lp, Rp, Dp);
-  dmma_tile<BM, BN>(Lp, Rp, Dp, a, local % a.tiles_m, local / a.tiles_m, smem);
+  const TileWork w = block_work(a, Lp, Rp, Dp);
+  dmma_tile<BM, BN>(Lp, Rp, Dp, a, w, smem);
 }
 
 // ------------------------------------------------- R4 / C4 / C8: SIMT FMA
@@ -612,8 +803,8 @@ __global__ void __launch_bounds__(kSThreads)
     gemm_gather_simt_kernel(const T *__restrict__ L, const T *__restrict__ R, T *D, const GemmArgs a) {
   const T *Lp = L, *Rp = R;
   T *Dp = D;
-  const int local = hyper_offsets(a, Lp, Rp, Dp);
-  simt_tile<T>(Lp, Rp, Dp, a, local % a.tiles_m, local / a.tiles_m);
+  const TileWork w = block_work(a, Lp, Rp, Dp);
+  simt_tile<T>(Lp, Rp, Dp, a, w.tm, w.tn);
 }
 
 // ------------------------------------------------------ full contraction
@@ -817,22 +1008,67 @@ int analyze(const int *cptrn, int drank, const int *ddims, int lrank, const int 
   return TALSH_SUCCESS;
 }
 
+int sm_count_dev() { return current_sm_count(); }
+
 size_t table_bytes(const TableParams &T) {
   return (size_t)align_up(8 * (2 * T.M + 2 * T.N + 2 * T.K + (T.nh > 0 ? 3 * T.H : 0)), 256);
 }
 
-// Grid of a gather-GEMM launch: tiles of one GEMM times hyper combinations.
+// Split of the contracted range.  A contraction with few output tiles and a
+// long contracted range leaves most SMs idle (a 40 x 40 output with K = 501760
+// ran on one CTA: 44 ms); its K is cut so that as many CTAs per SM have work as
+// fit at once (R8 four: 217 / 193 / 185 us there with two / three / four; C8
+// two), each at least 256 long (16 pipeline steps; 512 makes short ranges up to
+// 15 % slower).  The cut depends on the
+// shape alone, so the same contraction sums in the same order alone and in any
+// batch, whatever tile runs it.
+struct KSplit {
+  int nsplit = 1, kchunk = 0, gsz = 1;
+};
+constexpr int kSplitMinK = 256;
+KSplit k_split(int kind, int64_t M, int64_t N, int64_t K, int64_t H) {
+  KSplit s;
+  if (kind != R8 && kind != C8) return s;
+  const int64_t tiles = ((M + 63) / 64) * ((N + 63) / 64) * std::max<int64_t>(H, 1);
+  const int64_t want = std::min((kind == R8 ? 4 : 2) * 148 / tiles, K / kSplitMinK);
+  if (want < 2) return s;
+  s.kchunk = (int)(((K + want - 1) / want + 15) / 16 * 16);
+  s.nsplit = (int)((K + s.kchunk - 1) / s.kchunk);
+  s.gsz = s.nsplit;
+  if (s.nsplit > 8)
+    for (s.gsz = 1; s.gsz * s.gsz < s.nsplit; ++s.gsz) {}
+  return s;
+}
+int64_t split_counters(const KSplit &s, int64_t tiles) {
+  return s.nsplit > 1 ? tiles * ((s.nsplit + s.gsz - 1) / s.gsz + 1) : 0;
+}
+// Bytes of the partial tiles (edge x edge) and of the arrival counters.
+int64_t split_bytes(const KSplit &s, int kind, int64_t M, int64_t N, int64_t H, int edge) {
+  if (s.nsplit <= 1) return 0;
+  const int64_t tiles = ((M + edge - 1) / edge) * ((N + edge - 1) / edge) * std::max<int64_t>(H, 1);
+  return tiles * s.nsplit * edge * edge * kind_size(kind) + align_up(4 * split_counters(s, tiles), 256);
+}
+
+// CTA tile edge of a single FP64 contraction: 64, or 32 when even the split
+// 64 x 64 tiles do not give every SM one.  (128 x 128 tiles, one CTA of 16
+// warps per SM, were 1.5 % slower than four 64 x 64 CTAs on 3072 x 3072 x 3072:
+// independent CTAs fill each other's barrier gaps.)  Results do not depend on it.
+int gemm_edge(int64_t M, int64_t N, int64_t H, const KSplit &s) {
+  const int64_t tiles = ((M + 63) / 64) * ((N + 63) / 64) * std::max<int64_t>(H, 1);
+  return tiles * s.nsplit >= sm_count_dev() ? 64 : 32;
+}
+
+// Grid of a gather-GEMM launch: tiles of one GEMM times hyper combinations
+// times splits.
 int gemm_grid(GemmArgs &ga, int bm, int bn, int64_t *blocks) {
   ga.tiles_m = (ga.M + bm - 1) / bm;
   const int64_t per = (int64_t)ga.tiles_m * ((ga.N + bn - 1) / bn);
-  const int64_t all = per * std::max(ga.H, 1);
+  const int64_t all = per * std::max(ga.H, 1) * std::max(ga.nsplit, 1);
   if (per > 0x7fffffffLL || all > 0x7fffffffLL) return TALSH_LIMIT_EXCEEDED;
   ga.tiles_mn = (int)per;
   *blocks = all;
   return TALSH_SUCCESS;
 }
-
-int sm_count_dev() { return current_sm_count(); }
 
 template <int BM, int BN>
 int launch_dmma(const double *L, const double *R, double *D, GemmArgs ga, cudaStream_t st) {
@@ -919,16 +1155,28 @@ int check_args(int kind, const int *cptrn, int drank, const int *ddims, int lran
 
 }  // namespace
 
-// Scratch bytes needed by tcTensorContract for this shape (0 when none).
+// Scratch bytes of tcTensorContract for this shape (0 when none): the offset
+// tables and, for a split contracted range, the partial sums and counters.
+// `least`, when given, receives what the unsplit form needs: a call with less
+// than the full size but at least that runs unsplit.
 size_t contract_scratch_bytes(int kind, const int *cptrn, int drank, const int *ddims, int lrank,
-                              const int *ldims, int rrank, const int *rdims) {
+                              const int *ldims, int rrank, const int *rdims, size_t *least) {
+  if (least) *least = 0;
   if (check_args(kind, cptrn, drank, ddims, lrank, ldims, rrank, rdims)) return 0;
   if (lrank == 0 || rrank == 0) return 0;
   Analysis an;
   if (analyze(cptrn, drank, ddims, lrank, ldims, rrank, rdims, an)) return 0;
-  size_t b = table_bytes(an.T);
-  if (drank == 0) b += (size_t)dot_blocks(an.T.K) * sizeof(double2);
-  return b;
+  const TableParams &T = an.T;
+  size_t b = table_bytes(T);
+  if (drank == 0) b += (size_t)dot_blocks(T.K) * sizeof(double2);
+  if (least) *least = b;
+  if (drank == 0) return b;
+  const KSplit ks = k_split(kind, T.M, T.N, T.K, T.H);
+  return b + (size_t)split_bytes(ks, kind, T.M, T.N, T.H, gemm_edge(T.M, T.N, T.H, ks));
+}
+size_t contract_scratch_bytes(int kind, const int *cptrn, int drank, const int *ddims, int lrank,
+                              const int *ldims, int rrank, const int *rdims) {
+  return contract_scratch_bytes(kind, cptrn, drank, ddims, lrank, ldims, rrank, rdims, nullptr);
 }
 
 // The argument checks of contract_launch without launching anything.
@@ -1005,6 +1253,20 @@ int contract_launch(int kind, const int *cptrn, int drank, const int *ddims, int
   if (T.nh > 0) {
     T.hL = T.kR + T.K; T.hR = T.hL + T.H; T.hD = T.hR + T.H;
   }
+  KSplit ks;
+  int edge = 64;
+  if (drank > 0) {
+    ks = k_split(kind, T.M, T.N, T.K, T.H);
+    edge = gemm_edge(T.M, T.N, T.H, ks);
+    const int64_t extra = split_bytes(ks, kind, T.M, T.N, T.H, edge);
+    if (scratch_bytes < need + (size_t)extra) {  // no room for partial sums: one CTA per tile
+      ks = KSplit();
+      edge = gemm_edge(T.M, T.N, T.H, ks);
+    }
+    const int64_t tiles = ((T.M + edge - 1) / edge) * ((T.N + edge - 1) / edge) * T.H;
+    T.ncnt = split_counters(ks, tiles);
+    T.cnt = (int *)((char *)scratch + need);
+  }
   {
     const int64_t total = T.M + T.N + T.K + (T.nh > 0 ? T.H : 0);
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((total + 255) / 256, 4096));
@@ -1033,16 +1295,20 @@ int contract_launch(int kind, const int *cptrn, int drank, const int *ddims, int
   if (T.nh > 0) {
     ga.hL = T.hL; ga.hR = T.hR; ga.hD = T.hD;
   }
+  ga.nsplit = ks.nsplit; ga.kchunk = ks.kchunk; ga.gsz = ks.gsz;
+  ga.cnt = T.cnt;
+  ga.part = (char *)scratch + need + align_up(4 * T.ncnt, 256);
   switch (kind) {
     case R8: {
-      const int64_t big_tiles = ((T.M + 127) / 128) * ((T.N + 127) / 128) * T.H;
-      if (big_tiles >= 2 * sm_count_dev())
-        return launch_dmma<128, 128>((const double *)L, (const double *)R, (double *)D, ga, st);
-      return launch_dmma<64, 64>((const double *)L, (const double *)R, (double *)D, ga, st);
+      const double *l = (const double *)L, *r = (const double *)R;
+      if (edge == 64) return launch_dmma<64, 64>(l, r, (double *)D, ga, st);
+      return launch_dmma<32, 32>(l, r, (double *)D, ga, st);
     }
     case R4: return launch_simt<float>(L, R, D, ga, st);
     case C4: return launch_simt<float2>(L, R, D, ga, st);
-    default: return launch_zmma<64, 64>((const double2 *)L, (const double2 *)R, (double2 *)D, ga, st);
+    default:
+      if (edge == 64) return launch_zmma<64, 64>((const double2 *)L, (const double2 *)R, (double2 *)D, ga, st);
+      return launch_zmma<32, 32>((const double2 *)L, (const double2 *)R, (double2 *)D, ga, st);
   }
 }
 
@@ -1129,6 +1395,7 @@ __global__ void __launch_bounds__(256) batch_tables_kernel(const BatchDesc *desc
   const BatchDesc &d = descs[blockIdx.y];
   const int64_t M = d.a.M, N = d.a.N, K = d.a.K;
   const int64_t total = M + N + K;
+  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < d.a.ncnt; i += (int64_t)gridDim.x * 256) d.a.cnt[i] = 0;
   int64_t *mL = const_cast<int64_t *>(d.a.mL), *mD = const_cast<int64_t *>(d.a.mD);
   int64_t *nR = const_cast<int64_t *>(d.a.nR), *nD = const_cast<int64_t *>(d.a.nD);
   int64_t *kL = const_cast<int64_t *>(d.a.kL), *kR = const_cast<int64_t *>(d.a.kR);
@@ -1177,6 +1444,25 @@ __device__ __forceinline__ int find_task(const int64_t *prefix, int n, int64_t w
   return lo;
 }
 
+// Item i of a task: its tiles, repeated for every split of the contracted range.
+__device__ __forceinline__ TileWork item_work(const GemmArgs &a, int i) {
+  TileWork w;
+  w.split = i / a.tiles_mn;
+  w.lin = i - w.split * a.tiles_mn;
+  w.tm = w.lin % a.tiles_m;
+  w.tn = w.lin / a.tiles_m;
+  return w;
+}
+
+// The item's GEMM arguments, kept in shared memory (in registers they spilled).
+__device__ __forceinline__ void stage_args(GemmArgs &to, const GemmArgs &from) {
+  static_assert(sizeof(GemmArgs) % 4 == 0, "copied as words");
+  const uint32_t *f = reinterpret_cast<const uint32_t *>(&from);
+  uint32_t *t = reinterpret_cast<uint32_t *>(&to);
+  for (int i = threadIdx.x; i < (int)(sizeof(GemmArgs) / 4); i += blockDim.x) t[i] = f[i];
+  __syncthreads();
+}
+
 // Dynamic work distribution: CTAs take the next flat tile from a counter; the
 // host orders the tasks by decreasing K (longest tiles first).
 __device__ __forceinline__ int64_t next_item(unsigned long long *ctr) {
@@ -1187,38 +1473,33 @@ __device__ __forceinline__ int64_t next_item(unsigned long long *ctr) {
   return item;
 }
 
-// Resident CTAs per SM asked of the compiler for the persistent batch kernels.
-template <int BM, int BN> struct BatchOcc { static constexpr int D = 1, Z = 1; };
-template <> struct BatchOcc<64, 64> { static constexpr int D = 3, Z = 2; };
-template <> struct BatchOcc<32, 32> { static constexpr int D = 6, Z = 5; };
-
 template <int BM, int BN>
-__global__ void __launch_bounds__(DmmaCfg<BM, BN>::THREADS, BatchOcc<BM, BN>::D)
+__global__ void __launch_bounds__(DmmaCfg<BM, BN>::THREADS, GemmOcc<BM, BN>::D)
     dmma_batch_kernel(const BatchDesc *descs, const int32_t *list, const int64_t *prefix, int n,
                       int64_t total, unsigned long long *ctr) {
   extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ GemmArgs a;
   for (int64_t w = next_item(ctr); w < total; w = next_item(ctr)) {
     const int j = find_task(prefix, n, w);
     const BatchDesc &d = descs[list[j]];
-    const GemmArgs a = d.a;
-    const int local = (int)(w - prefix[j]);
-    dmma_tile<BM, BN>((const double *)d.L, (const double *)d.R, (double *)d.D, a, local % a.tiles_m,
-                      local / a.tiles_m, smem);
+    stage_args(a, d.a);
+    dmma_tile<BM, BN>((const double *)d.L, (const double *)d.R, (double *)d.D, a, item_work(a, (int)(w - prefix[j])),
+                      smem);
   }
 }
 
 template <int BM, int BN>
-__global__ void __launch_bounds__(ZmmaCfg<BM, BN>::THREADS, BatchOcc<BM, BN>::Z)
+__global__ void __launch_bounds__(ZmmaCfg<BM, BN>::THREADS, GemmOcc<BM, BN>::Z)
     zmma_batch_kernel(const BatchDesc *descs, const int32_t *list, const int64_t *prefix, int n,
                       int64_t total, unsigned long long *ctr) {
   extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ GemmArgs a;
   for (int64_t w = next_item(ctr); w < total; w = next_item(ctr)) {
     const int j = find_task(prefix, n, w);
     const BatchDesc &d = descs[list[j]];
-    const GemmArgs a = d.a;
-    const int local = (int)(w - prefix[j]);
-    zmma_tile<BM, BN>((const double2 *)d.L, (const double2 *)d.R, (double2 *)d.D, a, local % a.tiles_m,
-                      local / a.tiles_m, smem);
+    stage_args(a, d.a);
+    zmma_tile<BM, BN>((const double2 *)d.L, (const double2 *)d.R, (double2 *)d.D, a,
+                      item_work(a, (int)(w - prefix[j])), smem);
   }
 }
 
@@ -1239,6 +1520,8 @@ struct BatchPlan {
   std::vector<BatchDesc> descs;
   std::vector<int> cfg;          // per task: configuration, or -1 = single-task fallback
   std::vector<int64_t> tab_off;  // per task: offset of its tables (int64 elements)
+  std::vector<size_t> part_off;  // per task: offset of its partial sums and counters (bytes, from off_part)
+  size_t off_part = 0;
   std::vector<size_t> fb_scratch;
   std::vector<size_t> fb_off;
   std::vector<int32_t> list[kNumCfg];
@@ -1269,14 +1552,18 @@ int batch_cfg_of(int kind, int64_t M, int64_t N) {
   }
 }
 
-int batch_plan(int ntasks, const tcContractTask *tasks, BatchPlan &bp) {
+// `lean` (one flag per task, or null): no partial sums for that task, whose
+// contracted range then is not split.
+int batch_plan(int ntasks, const tcContractTask *tasks, BatchPlan &bp, const std::vector<char> *lean = nullptr) {
   if (ntasks < 0 || ntasks > 65535 || (ntasks > 0 && tasks == nullptr)) return TALSH_INVALID_ARGS;
   bp.descs.assign(ntasks, BatchDesc());
   bp.cfg.assign(ntasks, -1);
   bp.tab_off.assign(ntasks, 0);
   bp.fb_scratch.assign(ntasks, 0);
   bp.fb_off.assign(ntasks, 0);
+  bp.part_off.assign(ntasks, 0);
   int64_t tab = 0;
+  size_t part = 0;
   for (int t = 0; t < ntasks; ++t) {
     const tcContractTask &x = tasks[t];
     if (x.drank > TC_BATCH_MAX_RANK || x.lrank > TC_BATCH_MAX_RANK || x.rrank > TC_BATCH_MAX_RANK)
@@ -1293,8 +1580,10 @@ int batch_plan(int ntasks, const tcContractTask *tasks, BatchPlan &bp) {
                   an.T.M <= 0x7fffffffLL && an.T.N <= 0x7fffffffLL && an.T.K <= 0x7fffffffLL;
     }
     if (!batchable) {  // scalar operands, hyper-indices: single-task path
+      size_t least = 0;
       bp.fb_scratch[t] = contract_scratch_bytes(x.data_kind, x.cptrn, x.drank, x.ddims, x.lrank, x.ldims,
-                                                x.rrank, x.rdims);
+                                                x.rrank, x.rdims, &least);
+      if (lean && (*lean)[t]) bp.fb_scratch[t] = least;
       continue;
     }
     const TableParams &T = an.T;
@@ -1324,23 +1613,35 @@ int batch_plan(int ntasks, const tcContractTask *tasks, BatchPlan &bp) {
     const int bm = cfg_tile(c), bn = bm;
     a.tiles_m = (int)((T.M + bm - 1) / bm);
     const int64_t tiles = (int64_t)a.tiles_m * ((T.N + bn - 1) / bn);
+    if (tiles > 0x7fffffffLL) return TALSH_LIMIT_EXCEEDED;
+    a.tiles_mn = (int)tiles;
+    a.nsplit = 1;
+    if (!(lean && (*lean)[t])) {
+      const KSplit ks = k_split(x.data_kind, T.M, T.N, T.K, 1);
+      a.nsplit = ks.nsplit; a.kchunk = ks.kchunk; a.gsz = ks.gsz;
+      a.ncnt = (int)split_counters(ks, tiles);
+      bp.part_off[t] = part;
+      part += (size_t)align_up(split_bytes(ks, x.data_kind, T.M, T.N, 1, bm), 256);
+    }
     bp.cfg[t] = c;
     bp.tab_off[t] = tab;
     tab += 2 * (T.M + T.N + T.K);
     bp.list[c].push_back(t);
-    (void)tiles;
   }
-  // Longest tiles (largest K) first, then the tile prefix sums.
+  // Longest items (largest K, or K chunk) first, then the item prefix sums.
+  auto span = [&](int t) {
+    const GemmArgs &a = bp.descs[t].a;
+    return a.nsplit > 1 ? a.kchunk : a.K;
+  };
   for (int c = 0; c < kNumCfg; ++c) {
     auto &l = bp.list[c];
-    std::stable_sort(l.begin(), l.end(), [&](int x, int y) { return bp.descs[x].a.K > bp.descs[y].a.K; });
+    std::stable_sort(l.begin(), l.end(), [&](int x, int y) { return span(x) > span(y); });
     auto &pl = bp.prefix[c];
     if (l.empty()) continue;
     pl.push_back(0);
     for (int t : l) {
       const GemmArgs &a = bp.descs[t].a;
-      const int bn = cfg_tile(c);
-      pl.push_back(pl.back() + (int64_t)a.tiles_m * ((a.N + bn - 1) / bn));
+      pl.push_back(pl.back() + (int64_t)a.tiles_mn * a.nsplit);
     }
   }
   size_t off = 0;
@@ -1354,6 +1655,7 @@ int batch_plan(int ntasks, const tcContractTask *tasks, BatchPlan &bp) {
   bp.off_ctr = take(sizeof(unsigned long long) * kNumCfg);
   for (int t = 0; t < ntasks; ++t)
     if (bp.cfg[t] < 0) bp.fb_off[t] = take(bp.fb_scratch[t]);
+  bp.off_part = take(part);
   bp.total = off;
   return TALSH_SUCCESS;
 }
@@ -1422,6 +1724,34 @@ int launch_simt_batch(const BatchPlan &bp, int c, char *base, cudaStream_t st) {
 namespace tb {
 namespace {
 
+// The plan for a scratch block of `bytes`: without the partial sums of split
+// contracted ranges when those do not fit (batch_run refuses what is smaller
+// still).
+int batch_plan_for(int ntasks, const tcContractTask *tasks, BatchPlan &bp, size_t bytes) {
+  const int rc = batch_plan(ntasks, tasks, bp);
+  if (rc || bytes >= bp.total) return rc;
+  bp = BatchPlan();
+  const std::vector<char> lean((size_t)ntasks, 1);
+  return batch_plan(ntasks, tasks, bp, &lean);
+}
+
+// Points the descriptors at their tables, counters and partial sums in the
+// scratch block; returns the largest number of table entries of a task.
+int64_t batch_bind(BatchPlan &bp, char *base) {
+  int64_t *tabs = (int64_t *)(base + bp.off_tab);
+  int64_t max_entries = 0;
+  for (size_t t = 0; t < bp.descs.size(); ++t) {
+    if (bp.cfg[t] < 0) continue;
+    GemmArgs &a = bp.descs[t].a;
+    int64_t *p = tabs + bp.tab_off[t];
+    a.mL = p; a.mD = p + a.M; a.nR = a.mD + a.M; a.nD = a.nR + a.N; a.kL = a.nD + a.N; a.kR = a.kL + a.K;
+    a.cnt = (int *)(base + bp.off_part + bp.part_off[t]);
+    a.part = (char *)a.cnt + align_up(4 * (int64_t)a.ncnt, 256);
+    max_entries = std::max<int64_t>(max_entries, (int64_t)a.M + a.N + a.K);
+  }
+  return max_entries;
+}
+
 // Uploads the descriptors, work lists and prefix sums (the scratch bytes below
 // off_tab) as one copy, then launches the table build, one persistent kernel
 // per configuration and the single-task fallbacks.  `stage`, when given, is a
@@ -1431,15 +1761,7 @@ int batch_run(int ntasks, const tcContractTask *tasks, BatchPlan &bp, void *scra
               void *stage, cudaStream_t st) {
   if (scratch == nullptr || scratch_bytes < bp.total) return TALSH_INVALID_ARGS;
   char *base = (char *)scratch;
-  int64_t *tabs = (int64_t *)(base + bp.off_tab);
-  int64_t max_entries = 0;
-  for (int t = 0; t < ntasks; ++t) {
-    if (bp.cfg[t] < 0) continue;
-    GemmArgs &a = bp.descs[t].a;
-    int64_t *p = tabs + bp.tab_off[t];
-    a.mL = p; a.mD = p + a.M; a.nR = a.mD + a.M; a.nD = a.nR + a.N; a.kL = a.nD + a.N; a.kR = a.kL + a.K;
-    max_entries = std::max<int64_t>(max_entries, (int64_t)a.M + a.N + a.K);
-  }
+  const int64_t max_entries = batch_bind(bp, base);
   std::vector<char> pageable;
   char *host = (char *)stage;
   if (host == nullptr) {
@@ -1487,9 +1809,21 @@ int batch_run(int ntasks, const tcContractTask *tasks, BatchPlan &bp, void *scra
 // Upper bound of one task's share of a batch's scratch: its descriptor, work
 // list and prefix entries, and its offset tables or single-task fallback
 // scratch.  A batch needs the sum over its tasks plus batch_fixed_scratch().
-size_t batch_task_scratch_bound(const tcContractTask &x) {
-  const size_t fb = contract_scratch_bytes(x.data_kind, x.cptrn, x.drank, x.ddims, x.lrank, x.ldims, x.rrank,
-                                           x.rdims);
+// `lean` leaves out the partial sums of a split contracted range.
+size_t batch_task_scratch_bound(const tcContractTask &x, bool lean) {
+  size_t fb = 0;
+  const size_t full = contract_scratch_bytes(x.data_kind, x.cptrn, x.drank, x.ddims, x.lrank, x.ldims, x.rrank,
+                                             x.rdims, &fb);
+  Analysis an;
+  if (!lean && full > 0 && analyze(x.cptrn, x.drank, x.ddims, x.lrank, x.ldims, x.rrank, x.rdims, an) == 0) {
+    const TableParams &T = an.T;
+    if (an.hyper) {  // single-task path inside the batch
+      fb = full;
+    } else {         // either tile edge of the batch kernels
+      const KSplit ks = k_split(x.data_kind, T.M, T.N, T.K, 1);
+      fb += (size_t)std::max(split_bytes(ks, x.data_kind, T.M, T.N, 1, 32), split_bytes(ks, x.data_kind, T.M, T.N, 1, 64)) + 256;
+    }
+  }
   return sizeof(BatchDesc) + sizeof(int32_t) + sizeof(int64_t) + fb + 256;
 }
 
@@ -1498,11 +1832,12 @@ size_t batch_fixed_scratch() { return (size_t)(2 * kNumCfg + 4) * 256 + sizeof(u
 // Plans a batch, asks `get` for device scratch and a pinned staging block of
 // the sizes the plan needs (get returns nullptr to refuse: TRY_LATER), and
 // launches it on `stream`.
-int batch_launch_with(int ntasks, const tcContractTask *tasks, BatchScratchFn get, void *ctx, void *stream) {
+int batch_launch_with(int ntasks, const tcContractTask *tasks, const std::vector<char> *lean, BatchScratchFn get,
+                      void *ctx, void *stream) {
   cudaStream_t st = (cudaStream_t)stream;
   if (ntasks == 0) return TALSH_SUCCESS;
   BatchPlan bp;
-  int rc = batch_plan(ntasks, tasks, bp);
+  int rc = batch_plan(ntasks, tasks, bp, lean);
   if (rc) return rc;
   void *stage = nullptr;
   void *scratch = get(ctx, bp.total, bp.off_tab, &stage);
@@ -1522,7 +1857,7 @@ extern "C" int tcTensorContractBatch(int ntasks, const tcContractTask *tasks, vo
                                      size_t scratch_bytes, void *stream) {
   if (ntasks == 0) return TALSH_SUCCESS;
   tb::BatchPlan bp;
-  const int rc = tb::batch_plan(ntasks, tasks, bp);
+  const int rc = tb::batch_plan_for(ntasks, tasks, bp, scratch_bytes);
   if (rc) return rc;
   return tb::batch_run(ntasks, tasks, bp, scratch, scratch_bytes, nullptr, (cudaStream_t)stream);
 }
@@ -1550,21 +1885,13 @@ extern "C" int tcContractBatchGraphCreate(int ntasks, const tcContractTask *task
   *out = nullptr;
   if (ntasks < 1) return TALSH_INVALID_ARGS;
   BatchPlan bp;
-  int rc = batch_plan(ntasks, tasks, bp);
+  int rc = batch_plan_for(ntasks, tasks, bp, scratch_bytes);
   if (rc) return rc;
   if (scratch == nullptr || scratch_bytes < bp.total) return TALSH_INVALID_ARGS;
   cudaStream_t st = (cudaStream_t)stream;
   char *base = (char *)scratch;
   // Descriptors, lists and prefix sums, then the offset tables, once.
-  int64_t *tabs = (int64_t *)(base + bp.off_tab);
-  int64_t max_entries = 0;
-  for (int t = 0; t < ntasks; ++t) {
-    if (bp.cfg[t] < 0) continue;
-    GemmArgs &a = bp.descs[t].a;
-    int64_t *p = tabs + bp.tab_off[t];
-    a.mL = p; a.mD = p + a.M; a.nR = a.mD + a.M; a.nD = a.nR + a.N; a.kL = a.nD + a.N; a.kR = a.kL + a.K;
-    max_entries = std::max<int64_t>(max_entries, (int64_t)a.M + a.N + a.K);
-  }
+  const int64_t max_entries = batch_bind(bp, base);
   std::vector<char> host(bp.off_tab, 0);
   std::memcpy(host.data() + bp.off_desc, bp.descs.data(), sizeof(BatchDesc) * ntasks);
   for (int c = 0; c < kNumCfg; ++c) {

@@ -17,8 +17,6 @@
 #include "common.h"
 
 namespace tb {
-size_t contract_scratch_bytes(int kind, const int *cptrn, int drank, const int *ddims, int lrank,
-                              const int *ldims, int rrank, const int *rdims);
 int contract_launch(int kind, const int *cptrn, int drank, const int *ddims, int lrank,
                     const int *ldims, int rrank, const int *rdims, void *D, const void *L,
                     const void *R, double alpha_re, double alpha_im, int conj_bits,
@@ -78,8 +76,8 @@ extern "C" int tcTensorContractNoAlloc(int data_kind, const int *cptrn, int dran
                                        int accumulative, void *stream) {
   // The scratch need is a function of the shapes only; reject what does not fit
   // before touching the device.
-  const size_t need = tb::contract_scratch_bytes(data_kind, cptrn, drank, ddims, lrank, ldims,
-                                                 rrank, rdims);
+  size_t need = 0;  // without partial sums: a split contracted range uses what is left of the array
+  tb::contract_scratch_bytes(data_kind, cptrn, drank, ddims, lrank, ldims, rrank, rdims, &need);
   if (need > tb::kNoAllocScratchBytes) {
     char msg[200];
     std::snprintf(msg, sizeof(msg),

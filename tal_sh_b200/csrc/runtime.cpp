@@ -44,8 +44,6 @@
 namespace tb {
 int norm1_launch(int data_kind, size_t vol, const void *src, double *result_dev, double *partial,
                  cudaStream_t st);
-size_t contract_scratch_bytes(int kind, const int *cptrn, int drank, const int *ddims, int lrank,
-                              const int *ldims, int rrank, const int *rdims);
 size_t contract_split_scratch(int kind, const int *cptrn, int drank, const int *ddims, int lrank,
                               const int *ldims, int rrank, const int *rdims, int slices);
 int contract_split_launch(int kind, const int *cptrn, int drank, const int *ddims, int lrank,
@@ -619,7 +617,7 @@ int schedule(OpSpec &op, int dev_id, int dev_kind, talsh_task_t *user_task) {
       a.copy_back = a.output && (a.coh == COPY_T || a.coh == COPY_K);
     }
   }
-  size_t scratch = 0;
+  size_t scratch = 0, scratch_least = 0;  // a contraction may run with the smaller size
   if (op.kind == kOpContract) {
     int dd[MAX_TENSOR_RANK], ld[MAX_TENSOR_RANK], rd[MAX_TENSOR_RANK];
     for (int i = 0; i < op.drank; ++i) dd[i] = op.t[0]->shape_p->dims[i];
@@ -642,13 +640,17 @@ int schedule(OpSpec &op, int dev_id, int dev_kind, talsh_task_t *user_task) {
       scratch = split;
       tr->split_slices = sl;
     } else {
-      scratch = contract_scratch_bytes(dkind, op.dig, op.drank, dd, op.lrank, ld, op.rrank, rd);
+      scratch = contract_scratch_bytes(dkind, op.dig, op.drank, dd, op.lrank, ld, op.rrank, rd, &scratch_least);
     }
   } else if (op.kind == kOpNorm1) {
     scratch = tcTensorNorm1Scratch(shape_volume(op.t[0]->shape_p)) + 256;
   }
   if (scratch > 0) {
-    const int rc = dev_alloc(gpu, scratch, &tr->scratch);
+    int rc = dev_alloc(gpu, scratch, &tr->scratch);
+    if (rc != TALSH_SUCCESS && scratch_least > 0 && scratch_least < scratch) {
+      scratch = scratch_least;
+      rc = dev_alloc(gpu, scratch, &tr->scratch);
+    }
     if (rc != TALSH_SUCCESS) {
       for (int j = 0; j < op.nt; ++j) if (tr->a[j].dalloc) mem_free(tr->a[j].dptr);
       delete tr;
@@ -2476,7 +2478,7 @@ int talshTensorContractXL(const char *cptrn, talsh_tens_t *d, talsh_tens_t *l, t
   std::vector<XLBlock> ops;
   if ((rc = xl_decompose(op.dig, rank, full, es, avail, kXLMaxOps, ops)) != TALSH_SUCCESS) return rc;
   // Device buffers sized for the largest block of each argument, and scratch.
-  size_t bb[3] = {0, 0, 0}, scratch_bytes = 0;
+  size_t bb[3] = {0, 0, 0}, scratch_bytes = 0, scratch_least = 0;
   const int sl = g_r8_slices.load();
   bool hyper = false;
   for (int i = 0; i < op.lrank && !hyper; ++i)
@@ -2485,11 +2487,13 @@ int talshTensorContractXL(const char *cptrn, talsh_tens_t *d, talsh_tens_t *l, t
   const bool split = sl > 0 && kind == R8 && op.conj == 0 && !hyper && op.drank > 0 && op.lrank > 0 && op.rrank > 0;
   for (const XLBlock &b : ops) {
     for (int a = 0; a < 3; ++a) bb[a] = std::max(bb[a], xl_bytes(b, a, rank[a], es));
+    size_t least = 0;
     const size_t sc = split ? contract_split_scratch(kind, op.dig, op.drank, b.dims[0], op.lrank, b.dims[1], op.rrank,
                                                      b.dims[2], sl)
                             : contract_scratch_bytes(kind, op.dig, op.drank, b.dims[0], op.lrank, b.dims[1],
-                                                     op.rrank, b.dims[2]);
+                                                     op.rrank, b.dims[2], &least);
     scratch_bytes = std::max(scratch_bytes, sc);
+    scratch_least = std::max(scratch_least, split ? sc : least);
   }
   void *db[3] = {nullptr, nullptr, nullptr}, *scr = nullptr;
   bool reg[3] = {false, false, false};
@@ -2505,7 +2509,13 @@ int talshTensorContractXL(const char *cptrn, talsh_tens_t *d, talsh_tens_t *l, t
   };
   cudaSetDevice(gpu);
   for (int a = 0; a < 3 && rc == TALSH_SUCCESS; ++a) rc = dev_alloc(gpu, bb[a], &db[a]);
-  if (rc == TALSH_SUCCESS && scratch_bytes) rc = dev_alloc(gpu, scratch_bytes, &scr);
+  if (rc == TALSH_SUCCESS && scratch_bytes) {
+    rc = dev_alloc(gpu, scratch_bytes, &scr);
+    if (rc != TALSH_SUCCESS && scratch_least < scratch_bytes) {
+      scratch_bytes = scratch_least;
+      rc = dev_alloc(gpu, scratch_bytes, &scr);
+    }
+  }
   for (int a = 0; a < 3 && rc == TALSH_SUCCESS; ++a) {
     const size_t whole = shape_volume(ts[a]->shape_p) * (size_t)es;
     mp[a] = xl_map(hp[a], whole, reg[a]);

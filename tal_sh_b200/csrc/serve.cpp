@@ -37,8 +37,6 @@
 #include "common.h"
 
 namespace tb {
-size_t contract_scratch_bytes(int kind, const int *cptrn, int drank, const int *ddims, int lrank,
-                              const int *ldims, int rrank, const int *rdims);
 size_t contract_split_scratch(int kind, const int *cptrn, int drank, const int *ddims, int lrank,
                               const int *ldims, int rrank, const int *rdims, int slices);
 int contract_split_launch(int kind, const int *cptrn, int drank, const int *ddims, int lrank,
@@ -76,6 +74,7 @@ struct STask {
   size_t out_bytes = 0;    // server-held output bytes (0: caller's D)
   void *scratch = nullptr; // large tasks: scratch allocated at admission
   size_t scratch_bytes = 0;
+  bool lean = false;       // no room in the budget for partial sums: contracted range not split
   size_t reserve = 0;      // small tasks: budget held for their share of a batch's scratch
   int consumers_left = 0;  // declared consumers that have not completed
   int readers = 0;         // submitted consumers that have not completed
@@ -253,7 +252,10 @@ size_t large_scratch(const STask &t, int slices) {
   if (t.split)
     return tb::contract_split_scratch(x.data_kind, x.cptrn, x.drank, x.ddims, x.lrank, x.ldims, x.rrank, x.rdims,
                                       slices);
-  return tb::contract_scratch_bytes(x.data_kind, x.cptrn, x.drank, x.ddims, x.lrank, x.ldims, x.rrank, x.rdims);
+  size_t least = 0;
+  const size_t full = tb::contract_scratch_bytes(x.data_kind, x.cptrn, x.drank, x.ddims, x.lrank, x.ldims, x.rrank,
+                                                 x.rdims, &least);
+  return t.lean ? least : full;
 }
 
 void admit(tcServer *s, int cls) {
@@ -270,9 +272,20 @@ void admit(tcServer *s, int cls) {
     // Admitted tasks always leave room for the batch scratch of every admitted,
     // unlaunched small task plus one batch's fixed part, so a launch never
     // waits for memory that only a later launch could free.
-    const size_t resv = t.large ? 0 : round_bytes(tb::batch_task_scratch_bound(t.spec.op));
-    const size_t need = (t.own_out ? round_bytes(t.out_bytes) : 0) +
-                        (t.scratch_bytes ? round_bytes(t.scratch_bytes) : 0) + resv + tb::batch_fixed_scratch();
+    size_t resv = 0, need = 0;
+    auto size_up = [&]() {
+      resv = t.large ? 0 : round_bytes(tb::batch_task_scratch_bound(t.spec.op, t.lean));
+      need = (t.own_out ? round_bytes(t.out_bytes) : 0) + (t.scratch_bytes ? round_bytes(t.scratch_bytes) : 0) + resv +
+             tb::batch_fixed_scratch();
+    };
+    size_up();
+    if (need > s->cfg.budget_bytes && !t.lean) {
+      // A task that fits only without partial sums runs unsplit.  This depends
+      // on the budget alone, so its result does not depend on the other tasks.
+      t.lean = true;
+      if (t.large) t.scratch_bytes = large_scratch(t, s->cfg.r8_slices);
+      size_up();
+    }
     if (need > s->cfg.budget_bytes) {
       q.pop_front();
       tb::note_error_text("served task needs more device memory than the server budget");
@@ -392,15 +405,18 @@ void launch_batches(tcServer *s) {
     int rc = TRY_LATER;
     ScratchCtx ctx{s};
     std::vector<tcContractTask> ops;
+    std::vector<char> lean;
     while (n > 0) {
       ops.clear();
+      lean.clear();
       size_t resv = 0;
       for (size_t i = 0; i < n; ++i) {
         ops.push_back(resolve(s, s->tasks[sel[i]]));
+        lean.push_back(s->tasks[sel[i]].lean ? 1 : 0);
         resv += s->tasks[sel[i]].reserve;
       }
       s->reserved -= resv;  // the reservations become this batch's scratch
-      rc = tb::batch_launch_with((int)n, ops.data(), batch_scratch, &ctx, s->st[0]);
+      rc = tb::batch_launch_with((int)n, ops.data(), &lean, batch_scratch, &ctx, s->st[0]);
       if (rc != TRY_LATER) {
         for (size_t i = 0; i < n; ++i) s->tasks[sel[i]].reserve = 0;
         break;
