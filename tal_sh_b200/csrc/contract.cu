@@ -47,8 +47,9 @@ struct TableParams {
   int64_t kext[kMaxGR], kstrL[kMaxGR], kstrR[kMaxGR];
   // hyper-indices (in D, L and R): one independent GEMM per combination
   int64_t hext[kMaxGR], hstrL[kMaxGR], hstrR[kMaxGR], hstrD[kMaxGR];
-  int64_t *mL, *mD, *nR, *nD, *kL, *kR;
-  int64_t *hL, *hR, *hD;  // used when nh > 0
+  int64_t *mL, *mD, *nR, *nD, *kL, *kR;  // L and R offsets in bytes, D offsets in elements
+  int64_t *hL, *hR, *hD;  // used when nh > 0 (all in elements)
+  int es;                 // bytes per element of L and R
   int *cnt;               // arrival counters to zero (split contracted range)
   int64_t ncnt;
 };
@@ -80,7 +81,7 @@ __global__ void build_tables_kernel(const TableParams T) {
         a += c * T.mstrL[d];
         b += c * T.mstrD[d];
       }
-      T.mL[i] = a;
+      T.mL[i] = a * T.es;
       T.mD[i] = b;
     } else if (i < T.M + T.N) {
       int64_t r = i - T.M, a = 0, b = 0;
@@ -90,7 +91,7 @@ __global__ void build_tables_kernel(const TableParams T) {
         a += c * T.nstrR[d];
         b += c * T.nstrD[d];
       }
-      T.nR[i - T.M] = a;
+      T.nR[i - T.M] = a * T.es;
       T.nD[i - T.M] = b;
     } else {
       int64_t r = i - T.M - T.N, a = 0, b = 0;
@@ -100,8 +101,8 @@ __global__ void build_tables_kernel(const TableParams T) {
         a += c * T.kstrL[d];
         b += c * T.kstrR[d];
       }
-      T.kL[i - T.M - T.N] = a;
-      T.kR[i - T.M - T.N] = b;
+      T.kL[i - T.M - T.N] = a * T.es;
+      T.kR[i - T.M - T.N] = b * T.es;
     }
   }
 }
@@ -211,15 +212,6 @@ __device__ __forceinline__ bool split_combine(V (&acc)[NF], uint32_t mask, int p
 }
 
 // ---------------------------------------------------------------- R8: DMMA
-__device__ __forceinline__ void cp_async8(void *smem_ptr, const void *gptr, bool valid) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem_ptr);
-  const int n = valid ? 8 : 0;
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gptr), "r"(n));
-}
-__device__ __forceinline__ void cp_async8(void *smem_ptr, const void *gptr) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem_ptr);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gptr));
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
@@ -260,17 +252,26 @@ __device__ __forceinline__ void kring_init(const int64_t *kL, const int64_t *kR,
     kRs[i] = i < K ? kR[i] : 0;
   }
 }
+// The copies of one warp: lane l < BK the kL entries of a tile, the others kR's.
 template <int BK, int ST>
-__device__ __forceinline__ void kring_step(const int64_t *kL, const int64_t *kR, int K, int64_t *kLs, int64_t *kRs,
-                                           int tid, int kt) {
+struct KRing {
   static_assert(2 * BK == 32, "one warp copies both tables of a tile");
-  if (tid < 2 * BK) {
-    const int j = tid % BK, t = kt + ST + 1;
-    const int64_t k = (int64_t)t * BK + j;
-    const int64_t *from = tid < BK ? kL : kR;
-    cp_async8((tid < BK ? kLs : kRs) + (t % kKRing) * BK + j, from + (k < K ? k : 0), k < K);
+  const int64_t *from;
+  uint32_t to;
+  __device__ __forceinline__ void init(const int64_t *kL, const int64_t *kR, int64_t *kLs, int64_t *kRs) {
+    const int j = threadIdx.x % BK;
+    from = (threadIdx.x % 32 < BK ? kL : kR) + j;
+    to = (uint32_t)__cvta_generic_to_shared((threadIdx.x % 32 < BK ? kLs : kRs) + j);
   }
-}
+  __device__ __forceinline__ void step(int kt, int K) const {
+    if (threadIdx.x < 32) {
+      const int t = kt + ST + 1, k = t * BK;
+      const int n = k + (int)(threadIdx.x % BK) < K ? 8 : 0;
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(to + (t % kKRing) * (BK * 8)),
+                   "l"(from + (n ? k : 0)), "r"(n));
+    }
+  }
+};
 
 // Column swizzle of the FP64 tiles: row k stores column c at c ^ ((k >> 2) & 3).
 // With rows 8 banks apart (pitch BM + 4 doubles) a fragment load's four k-rows
@@ -285,49 +286,96 @@ __device__ __forceinline__ int frag_count(int rem, int w, int W, int F) {
   return max(0, min(F, (rem - w * 8 + 8 * W - 1) / (8 * W)));
 }
 
-// Portion Q of P of one operand's loads of a k-tile: X free-index rows (`rem`
-// of them inside the tensor) by BK k-rows, each element at fs[row] + ks[k].
-// `along`: lanes run along the free index, else along k; the two forms keep
-// their index arithmetic to constant strides, so an element costs an offset
-// read, an add and the copy.  TAIL: k-rows from `klim` on are zero-filled.
-template <int X, int BK, int NT, int PITCH, bool SWZ, int Q, int P, bool TAIL, typename T, typename Put>
-__device__ __forceinline__ void load_side(const T *__restrict__ G, const int64_t *fs, const int64_t *ks, T *dst,
-                                          int along, int rem, int klim, const Put &put) {
-  constexpr int N = (X * BK) / NT;
-  const int tid = threadIdx.x;
-  if (along) {
-    static_assert(NT % X == 0, "a thread keeps its row");
-    constexpr int S = NT / X;  // k-rows between a thread's elements
-    static_assert(!SWZ || S <= 4, "the swizzle does not depend on t0");
-    const int x = tid % X, t0 = tid / X;
-    if (x >= rem) return;
-    const T *g = G + fs[x];
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      if (i * P / N != Q) continue;
-      const bool v = !TAIL || t0 + i * S < klim;
-      const int c = SWZ ? x ^ kswz(i * S) : x;  // kswz(t0 + i S): t0 < S <= 4, a power of two
-      put(dst + t0 * PITCH + c + i * S * PITCH, g + (v ? ks[t0 + i * S] : 0), v);
-    }
+// Shared-memory reads by 32-bit address, and the copy of one ES-byte element.
+__device__ __forceinline__ int64_t lds64(uint32_t a) {
+  int64_t v;
+  asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(a));
+  return v;
+}
+template <int ES, bool TAIL>
+__device__ __forceinline__ void cp_elem(uint32_t s, const char *g, bool v) {
+  if constexpr (TAIL) {
+    const int n = v ? ES : 0;
+    if constexpr (ES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(g), "r"(n));
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(s), "l"(g), "n"(ES), "r"(n));
   } else {
-    const int kl = tid % BK, t0 = tid / BK;
-    constexpr int S = NT / BK;  // rows between a thread's elements (a multiple of 8)
-    const bool v = !TAIL || kl < klim;
-    const T *g = G + (v ? ks[kl] : 0);
-    T *d = dst + kl * PITCH + (SWZ ? t0 ^ kswz(kl) : t0);
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      if (i * P / N != Q) continue;
-      if (t0 + i * S < rem) put(d + i * S, g + fs[t0 + i * S], v);
-    }
+    if constexpr (ES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(g));
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(s), "l"(g), "n"(ES));
   }
 }
 
+// One operand's k-tile loads: X free-index rows (`rem` of them inside the
+// tensor) by BK k-rows, element (x, k) at G + fs[x] + ks[k] bytes and at column
+// x (XOR kswz(k) if SWZ) of shared row k.  `along`: a thread keeps one free
+// index and steps through k, its lanes along the free index; else it keeps one
+// k and steps through the free index.  Everything that does not change with the
+// k-tile is kept here, so an element costs an offset read, an add and the copy
+// (with the index arithmetic in the loop, about 25 instructions per element
+// bounded thin tiles and took issue slots from the tensor pipe in full ones).
+template <int X, int BK, int NT, int PITCH, int ES, bool SWZ>
+struct Side {
+  static constexpr int N = X * BK / NT;    // elements per thread and k-tile
+  static constexpr int SF = NT / X;        // k step of a thread along its free index
+  static constexpr int SK = NT / BK;       // free-index step of a thread along its k
+  static_assert(NT % X == 0 && NT % BK == 0 && X * BK % NT == 0, "whole elements per thread");
+  static_assert(!SWZ || (SF <= 4 && 4 % SF == 0 && SK % 4 == 0), "the swizzle is constant per element slot");
+  const char *g;   // along: the row's base, else the operand
+  uint32_t s;      // shared address of the thread's first element in stage 0
+  uint32_t u;      // along: column (swizzled per element); else shared address of its first row offset
+  int k0, lim;     // first k-row; along: rows left (> 0: loads), else rows it may load
+  bool along;
+
+  __device__ __forceinline__ void init(const void *G, const int64_t *fs_, const void *stage0, bool along_, int rem) {
+    const int tid = threadIdx.x;
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(stage0);
+    along = along_;
+    if (along) {
+      const int x0 = tid % X;
+      k0 = tid / X;
+      g = (const char *)G + fs_[x0];
+      s = base + (uint32_t)(k0 * PITCH + (SWZ ? 0 : x0)) * ES;
+      lim = rem - x0;
+      u = (uint32_t)x0;
+    } else {
+      const int x0 = tid / BK;
+      k0 = tid % BK;
+      g = (const char *)G;
+      s = base + (uint32_t)(k0 * PITCH + (SWZ ? x0 ^ kswz(k0) : x0)) * ES;
+      lim = rem - x0;
+      u = (uint32_t)__cvta_generic_to_shared(fs_ + x0);
+    }
+  }
+  // Loads of one k-tile: `so` bytes to its stage, k offsets at shared address
+  // ks, k-rows from klim on zero-filled (TAIL).
+  template <bool TAIL>
+  __device__ __forceinline__ void load(uint32_t so, uint32_t ks, int klim) const {
+    if (along) {
+      if (lim <= 0) return;
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        const bool v = !TAIL || k0 + i * SF < klim;
+        const uint32_t c = SWZ ? (u ^ kswz(i * SF)) * ES : 0u;
+        cp_elem<ES, TAIL>(s + so + c + (uint32_t)(i * SF * PITCH * ES), g + (v ? lds64(ks + (k0 + i * SF) * 8) : 0), v);
+      }
+    } else {
+      const bool v = !TAIL || k0 < klim;
+      const char *gk = g + (v ? lds64(ks + k0 * 8) : 0);
+#pragma unroll
+      for (int i = 0; i < N; ++i)
+        if (i * SK < lim) cp_elem<ES, TAIL>(s + so + (uint32_t)(i * SK * ES), gk + lds64(u + i * SK * 8), v);
+    }
+  }
+  __device__ __forceinline__ void load_tile(uint32_t so, uint32_t ks, int klim) const {
+    if (klim >= BK) load<false>(so, ks, klim);
+    else if (klim > 0) load<true>(so, ks, klim);
+  }
+};
+
 // One BM x BN tile of a gather-GEMM (shared by the single-contraction kernel and
 // the batched one) over the k range of its split.  The loads of the tile
-// ST - 1 ahead are issued in BK / 4 portions between the tensor-pipe steps:
-// issued in one block after the barrier they left the pipe idle in every warp
-// at once.  Rows and columns beyond the tensor are neither loaded (their stale
+// ST - 1 ahead are issued between the tensor-pipe steps (A's after the first,
+// B's after the third): issued in one block after the barrier they left the
+// pipe idle in every warp at once.  Rows and columns beyond the tensor are neither loaded (their stale
 // shared values only reach outputs that are not stored) nor multiplied.
 template <int BM, int BN>
 __device__ __forceinline__ void dmma_tile(const double *__restrict__ L, const double *__restrict__ R,
@@ -365,27 +413,20 @@ __device__ __forceinline__ void dmma_tile(const double *__restrict__ L, const do
 
   const int numK = (K + BK - 1) / BK;
   // Portion Q of P of the loads of k-tile kt into stage s.
-  const int along_a = a.a_along_m, along_b = a.b_along_n;
-  auto load_as = [&](int kt, int s, auto q, auto parts, auto tail) {
-    constexpr int Q = decltype(q)::value, P = decltype(parts)::value;
-    constexpr bool TAIL = decltype(tail)::value;
-    auto put = [](double *dst, const double *src, bool v) {
-      if constexpr (TAIL) cp_async8(dst, src, v);
-      else cp_async8(dst, src);
-    };
-    const int kr = (kt % kKRing) * BK, klim = K - kt * BK;
-    load_side<BM, BK, NT, AP, true, Q, P, TAIL>(L, mLs, kLs + kr, As + s * BK * AP, along_a, mrem, klim, put);
-    load_side<BN, BK, NT, BP, true, Q, P, TAIL>(R, nRs, kRs + kr, Bs + s * BK * BP, along_b, nrem, klim, put);
-  };
-  auto load_part = [&](int kt, int s, auto q, auto parts) {
-    if ((kt + 1) * BK <= K) load_as(kt, s, q, parts, std::false_type{});
-    else if (kt * BK < K) load_as(kt, s, q, parts, std::true_type{});
-  };
+  Side<BM, BK, NT, AP, 8, true> sa;
+  Side<BN, BK, NT, BP, 8, true> sb;
+  sa.init(L, mLs, As, a.a_along_m, mrem);
+  sb.init(R, nRs, Bs, a.b_along_n, nrem);
+  constexpr uint32_t SAB = BK * AP * 8, SBB = BK * BP * 8;  // bytes per stage
+  KRing<BK, ST> ring;
+  ring.init(kLg, kRg, kLs, kRs);
+  const uint32_t ksa = (uint32_t)__cvta_generic_to_shared(kLs), ksb = (uint32_t)__cvta_generic_to_shared(kRs);
+  auto load_a = [&](int kt, int s) { sa.load_tile(s * SAB, ksa + (kt % kKRing) * (BK * 8), K - kt * BK); };
+  auto load_b = [&](int kt, int s) { sb.load_tile(s * SBB, ksb + (kt % kKRing) * (BK * 8), K - kt * BK); };
   using Int0 = std::integral_constant<int, 0>;
   using Int1 = std::integral_constant<int, 1>;
   using Int2 = std::integral_constant<int, 2>;
   using Int3 = std::integral_constant<int, 3>;
-  using Int4 = std::integral_constant<int, 4>;
 
   constexpr int FM = C::WM / 8, FN = C::WN / 8;
   double2 acc[FM * FN];
@@ -401,7 +442,8 @@ __device__ __forceinline__ void dmma_tile(const double *__restrict__ L, const do
 
 #pragma unroll
   for (int s = 0; s < ST - 1; ++s) {
-    load_part(s, s, Int0{}, Int1{});
+    load_a(s, s);
+    load_b(s, s);
     cp_async_commit();
   }
   auto main_loop = [&](auto full_c) {
@@ -427,13 +469,14 @@ __device__ __forceinline__ void dmma_tile(const double *__restrict__ L, const do
           for (int j = 0; j < FN; ++j)
             if (FULL || j < fn) dmma_8x8x4(acc[i * FN + j].x, acc[i * FN + j].y, af[i], bf[j]);
         }
-        load_part(kt + ST - 1, ps, ksc, Int4{});
+        if constexpr (ks == 0) load_a(kt + ST - 1, ps);
+        if constexpr (ks == 2) load_b(kt + ST - 1, ps);
       };
       step(Int0{});
       step(Int1{});
       step(Int2{});
       step(Int3{});
-      kring_step<BK, ST>(kLg, kRg, K, kLs, kRs, tid, kt);
+      ring.step(kt, K);
       cp_async_commit();
       ps = st;
       st = st + 1 == ST ? 0 : st + 1;
@@ -476,7 +519,7 @@ __device__ __forceinline__ void dmma_tile(const double *__restrict__ L, const do
 // Complex-double tile on the FP64 tensor pipe: complex elements stay
 // interleaved in shared memory (one 16-byte cp.async per element, one 128-bit
 // load per fragment element), and
-// C_re += A_re B_re - A_im B_im, C_im += A_re B_im + A_im B_re run as four
+// C_re += A_re B_re + A_im (-B_im), C_im += A_re B_im + A_im B_re run as four
 // DMMA products.  Row pitches of BM + 2 elements put the four k-rows of a
 // fragment load in different bank groups.
 // Warp tiles are 32 x 16 (16 x 16 in 32x32 CTA tiles): two accumulator sets
@@ -491,13 +534,6 @@ struct ZmmaCfg {
   static constexpr size_t SMEM = (size_t)STAGES * BK * (AP + BP) * sizeof(double2) +
                                  (size_t)(2 * BM + 2 * BN + 2 * kKRing * BK) * sizeof(int64_t);
 };
-
-__device__ __forceinline__ void cp_async16(void *smem_ptr, const void *gptr, bool valid) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem_ptr);
-  const int n = valid ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gptr), "r"(n));
-}
-
 
 template <int BM, int BN>
 __device__ __forceinline__ void zmma_tile(const double2 *__restrict__ L, const double2 *__restrict__ R,
@@ -532,24 +568,21 @@ __device__ __forceinline__ void zmma_tile(const double2 *__restrict__ L, const d
   kring_init<BK, ST>(kLg, kRg, K, kLs, kRs, tid, NT);
   __syncthreads();
   const int numK = (K + BK - 1) / BK;
-  const int along_a = a.a_along_m, along_b = a.b_along_n;
-  auto load_as = [&](int kt, int s, auto q, auto parts, auto tail) {
-    constexpr int Q = decltype(q)::value, P = decltype(parts)::value;
-    constexpr bool TAIL = decltype(tail)::value;
-    auto put = [](double2 *dst, const double2 *src, bool v) { cp_async16(dst, src, v); };
-    const int kr = (kt % kKRing) * BK, klim = K - kt * BK;
-    load_side<BM, BK, NT, AP, false, Q, P, TAIL>(L, mLs, kLs + kr, As + s * BK * AP, along_a, mrem, klim, put);
-    load_side<BN, BK, NT, BP, false, Q, P, TAIL>(R, nRs, kRs + kr, Bs + s * BK * BP, along_b, nrem, klim, put);
-  };
-  auto load_part = [&](int kt, int s, auto q, auto parts) {
-    if ((kt + 1) * BK <= K) load_as(kt, s, q, parts, std::false_type{});
-    else if (kt * BK < K) load_as(kt, s, q, parts, std::true_type{});
-  };
+  Side<BM, BK, NT, AP, 16, false> sa;
+  Side<BN, BK, NT, BP, 16, false> sb;
+  sa.init(L, mLs, As, a.a_along_m, mrem);
+  sb.init(R, nRs, Bs, a.b_along_n, nrem);
+  constexpr uint32_t SAB = BK * AP * 16, SBB = BK * BP * 16;  // bytes per stage
+  KRing<BK, ST> ring;
+  ring.init(kLg, kRg, kLs, kRs);
+  const uint32_t ksa = (uint32_t)__cvta_generic_to_shared(kLs), ksb = (uint32_t)__cvta_generic_to_shared(kRs);
+  auto load_a = [&](int kt, int s) { sa.load_tile(s * SAB, ksa + (kt % kKRing) * (BK * 8), K - kt * BK); };
+  auto load_b = [&](int kt, int s) { sb.load_tile(s * SBB, ksb + (kt % kKRing) * (BK * 8), K - kt * BK); };
   using Int0 = std::integral_constant<int, 0>;
   using Int1 = std::integral_constant<int, 1>;
   using Int2 = std::integral_constant<int, 2>;
   using Int3 = std::integral_constant<int, 3>;
-  using Int4 = std::integral_constant<int, 4>;
+
   constexpr int FM = C::WM / 8, FN = C::WN / 8;
   double2 acc[2 * FM * FN];  // fragment f: real parts at 2 f, imaginary parts at 2 f + 1
 #pragma unroll
@@ -560,10 +593,13 @@ __device__ __forceinline__ void zmma_tile(const double2 *__restrict__ L, const d
   const int wm = wr % C::WARPS_M, wn = wr / C::WARPS_M;
   const int fr = lane >> 2, fc = lane & 3;
   const int fm = frag_count(mrem, wm, C::WARPS_M, FM), fn = frag_count(nrem, wn, C::WARPS_N, FN);
-  const double sl = a.conj_l ? -1.0 : 1.0, sr = a.conj_r ? -1.0 : 1.0;
+  // conjugation flips the sign bit of the imaginary part
+  const int ml = a.conj_l ? (int)0x80000000 : 0, mr = a.conj_r ? (int)0x80000000 : 0;
+  auto flip = [](double x, int m) { return __hiloint2double(__double2hiint(x) ^ m, __double2loint(x)); };
 #pragma unroll
   for (int s = 0; s < ST - 1; ++s) {
-    load_part(s, s, Int0{}, Int1{});
+    load_a(s, s);
+    load_b(s, s);
     cp_async_commit();
   }
   auto main_loop = [&](auto full_c) {
@@ -576,19 +612,19 @@ __device__ __forceinline__ void zmma_tile(const double2 *__restrict__ L, const d
       const double2 *bs = Bs + (st * BK + fc) * BP + wn * 8 + fr;
       auto step = [&](auto ksc) {
         constexpr int ks = decltype(ksc)::value;
-        double ar[FM], ai[FM], nai[FM], br[FN], bi[FN];
+        double ar[FM], ai[FM], br[FN], bi[FN], nbi[FN];
 #pragma unroll
         for (int i = 0; i < FM; ++i) {
           const double2 v = as[ks * 4 * AP + i * C::WARPS_M * 8];
           ar[i] = v.x;
-          ai[i] = sl * v.y;
-          nai[i] = -ai[i];
+          ai[i] = flip(v.y, ml);
         }
 #pragma unroll
         for (int j = 0; j < FN; ++j) {
           const double2 v = bs[ks * 4 * BP + j * C::WARPS_N * 8];
           br[j] = v.x;
-          bi[j] = sr * v.y;
+          bi[j] = flip(v.y, mr);
+          nbi[j] = -bi[j];
         }
 #pragma unroll
         for (int i = 0; i < FM; ++i) {
@@ -598,18 +634,19 @@ __device__ __forceinline__ void zmma_tile(const double2 *__restrict__ L, const d
             if (!FULL && j >= fn) break;
             double2 &cr = acc[2 * (i * FN + j)], &ci = acc[2 * (i * FN + j) + 1];
             dmma_8x8x4(cr.x, cr.y, ar[i], br[j]);
-            dmma_8x8x4(cr.x, cr.y, nai[i], bi[j]);
+            dmma_8x8x4(cr.x, cr.y, ai[i], nbi[j]);
             dmma_8x8x4(ci.x, ci.y, ar[i], bi[j]);
             dmma_8x8x4(ci.x, ci.y, ai[i], br[j]);
           }
         }
-        load_part(kt + ST - 1, ps, ksc, Int4{});
+        if constexpr (ks == 0) load_a(kt + ST - 1, ps);
+        if constexpr (ks == 2) load_b(kt + ST - 1, ps);
       };
       step(Int0{});
       step(Int1{});
       step(Int2{});
       step(Int3{});
-      kring_step<BK, ST>(kLg, kRg, K, kLs, kRs, tid, kt);
+      ring.step(kt, K);
       cp_async_commit();
       ps = st;
       st = st + 1 == ST ? 0 : st + 1;
@@ -759,7 +796,7 @@ __device__ __forceinline__ void simt_tile(const T *__restrict__ L, const T *__re
       const int ml = a.a_along_m ? (idx % kSBM) : (idx / kSBK);
       const int kl = a.a_along_m ? (idx / kSBM) : (idx % kSBK);
       const int m = m0 + ml, k = k0 + kl;
-      As[kl][ml] = (m < a.M && k < a.K) ? Num<T>::load(L[mLs[ml] + a.kL[k]], a.conj_l) : Num<T>::zero();
+      As[kl][ml] = (m < a.M && k < a.K) ? Num<T>::load(*(const T *)((const char *)L + mLs[ml] + a.kL[k]), a.conj_l) : Num<T>::zero();
     }
 #pragma unroll
     for (int i = 0; i < (kSBN * kSBK) / kSThreads; ++i) {
@@ -767,7 +804,7 @@ __device__ __forceinline__ void simt_tile(const T *__restrict__ L, const T *__re
       const int nl = a.b_along_n ? (idx % kSBN) : (idx / kSBK);
       const int kl = a.b_along_n ? (idx / kSBN) : (idx % kSBK);
       const int n = n0 + nl, k = k0 + kl;
-      Bs[kl][nl] = (n < a.N && k < a.K) ? Num<T>::load(R[nRs[nl] + a.kR[k]], a.conj_r) : Num<T>::zero();
+      Bs[kl][nl] = (n < a.N && k < a.K) ? Num<T>::load(*(const T *)((const char *)R + nRs[nl] + a.kR[k]), a.conj_r) : Num<T>::zero();
     }
     __syncthreads();
 #pragma unroll
@@ -851,7 +888,8 @@ __global__ void __launch_bounds__(kDotThreads)
   const int64_t beg = (int64_t)blockIdx.x * chunk, end = min(K, beg + chunk);
   double2 acc = make_double2(0.0, 0.0);
   for (int64_t k = beg + threadIdx.x; k < end; k += kDotThreads) {
-    const double2 x = as_c<T>(L[kL[k]], cl), y = as_c<T>(R[kR[k]], cr);
+    const double2 x = as_c<T>(*(const T *)((const char *)L + kL[k]), cl);
+    const double2 y = as_c<T>(*(const T *)((const char *)R + kR[k]), cr);
     acc.x += x.x * y.x - x.y * y.y;
     acc.y += x.x * y.y + x.y * y.x;
   }
@@ -1249,6 +1287,7 @@ int contract_launch(int kind, const int *cptrn, int drank, const int *ddims, int
   if (T.M > 0x7fffffffLL || T.N > 0x7fffffffLL || T.K > 0x7fffffffLL || T.H > 0x7fffffffLL)
     return TALSH_LIMIT_EXCEEDED;
   int64_t *base = (int64_t *)scratch;
+  T.es = kind_size(kind);
   T.mL = base; T.mD = T.mL + T.M; T.nR = T.mD + T.M; T.nD = T.nR + T.N; T.kL = T.nD + T.N; T.kR = T.kL + T.K;
   if (T.nh > 0) {
     T.hL = T.kR + T.K; T.hR = T.hL + T.H; T.hD = T.hR + T.H;
@@ -1334,6 +1373,7 @@ int contract_build_tables(const int *cptrn, int drank, const int *ddims, int lra
   if (an.hyper) return TALSH_NOT_IMPLEMENTED;
   TableParams T = an.T;
   int64_t *base = (int64_t *)tables;
+  T.es = kind_size(R8);
   T.mL = base; T.mD = T.mL + T.M; T.nR = T.mD + T.M; T.nD = T.nR + T.N; T.kL = T.nD + T.N; T.kR = T.kL + T.K;
   const int64_t total = T.M + T.N + T.K;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((total + 255) / 256, 4096));
@@ -1377,7 +1417,7 @@ namespace {
 constexpr int kBMaxG = 8;  // max dimensions per index group of a batched task
 
 struct BatchDesc {
-  int nm, nn, nk;
+  int nm, nn, nk, es;
   int32_t mext[kBMaxG], next[kBMaxG], kext[kBMaxG];
   int64_t mstrL[kBMaxG], mstrD[kBMaxG], nstrR[kBMaxG], nstrD[kBMaxG], kstrL[kBMaxG], kstrR[kBMaxG];
   GemmArgs a;
@@ -1408,7 +1448,7 @@ __global__ void __launch_bounds__(256) batch_tables_kernel(const BatchDesc *desc
         x += c * d.mstrL[g];
         y += c * d.mstrD[g];
       }
-      mL[i] = x;
+      mL[i] = x * d.es;
       mD[i] = y;
     } else if (i < M + N) {
       int64_t r = i - M, x = 0, y = 0;
@@ -1418,7 +1458,7 @@ __global__ void __launch_bounds__(256) batch_tables_kernel(const BatchDesc *desc
         x += c * d.nstrR[g];
         y += c * d.nstrD[g];
       }
-      nR[i - M] = x;
+      nR[i - M] = x * d.es;
       nD[i - M] = y;
     } else {
       int64_t r = i - M - N, x = 0, y = 0;
@@ -1428,8 +1468,8 @@ __global__ void __launch_bounds__(256) batch_tables_kernel(const BatchDesc *desc
         x += c * d.kstrL[g];
         y += c * d.kstrR[g];
       }
-      kL[i - M - N] = x;
-      kR[i - M - N] = y;
+      kL[i - M - N] = x * d.es;
+      kR[i - M - N] = y * d.es;
     }
   }
 }
@@ -1588,7 +1628,7 @@ int batch_plan(int ntasks, const tcContractTask *tasks, BatchPlan &bp, const std
     }
     const TableParams &T = an.T;
     BatchDesc &d = bp.descs[t];
-    d.nm = T.nm; d.nn = T.nn; d.nk = T.nk;
+    d.nm = T.nm; d.nn = T.nn; d.nk = T.nk; d.es = kind_size(x.data_kind);
     for (int g = 0; g < T.nm; ++g) { d.mext[g] = (int32_t)T.mext[g]; d.mstrL[g] = T.mstrL[g]; d.mstrD[g] = T.mstrD[g]; }
     for (int g = 0; g < T.nn; ++g) { d.next[g] = (int32_t)T.next[g]; d.nstrR[g] = T.nstrR[g]; d.nstrD[g] = T.nstrD[g]; }
     for (int g = 0; g < T.nk; ++g) { d.kext[g] = (int32_t)T.kext[g]; d.kstrL[g] = T.kstrL[g]; d.kstrR[g] = T.kstrR[g]; }
