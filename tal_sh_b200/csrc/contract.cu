@@ -15,7 +15,8 @@
 // mapped so that the operand's stride-1 index runs across the lanes.
 //  * R8: warp-level DMMA (mma.sync m8n8k4 f64) on a multistage cp.async
 //    pipeline, FP64 end to end.
-//  * R4 / C4 / C8: register-blocked SIMT FMA kernel on the same tables.
+//  * C8: four DMMA products per complex product; R4 / C4: register-blocked packed
+//    FP32 FMA; all on the same tables and pipeline.
 //  * Degenerate patterns: full contraction (dot, deterministic two-pass),
 //    scalar x tensor (the permute-add kernel with a device-side scale) and
 //    scalar x scalar.
@@ -315,6 +316,8 @@ __device__ __forceinline__ void cp_elem(uint32_t s, const char *g, bool v) {
 template <int X, int BK, int NT, int PITCH, int ES, bool SWZ>
 struct Side {
   static constexpr int N = X * BK / NT;    // elements per thread and k-tile
+  static constexpr int W = 4;              // offsets read before the copies that use them: the reads
+                                           // overlap instead of costing a shared-memory latency each
   static constexpr int SF = NT / X;        // k step of a thread along its free index
   static constexpr int SK = NT / BK;       // free-index step of a thread along its k
   static_assert(NT % X == 0 && NT % BK == 0 && X * BK % NT == 0, "whole elements per thread");
@@ -337,6 +340,7 @@ struct Side {
       lim = rem - x0;
       u = (uint32_t)x0;
     } else {
+      static_assert(N % W == 0, "whole groups of offset reads");
       const int x0 = tid / BK;
       k0 = tid % BK;
       g = (const char *)G;
@@ -352,17 +356,29 @@ struct Side {
     if (along) {
       if (lim <= 0) return;
 #pragma unroll
-      for (int i = 0; i < N; ++i) {
-        const bool v = !TAIL || k0 + i * SF < klim;
-        const uint32_t c = SWZ ? (u ^ kswz(i * SF)) * ES : 0u;
-        cp_elem<ES, TAIL>(s + so + c + (uint32_t)(i * SF * PITCH * ES), g + (v ? lds64(ks + (k0 + i * SF) * 8) : 0), v);
+      for (int i0 = 0; i0 < N; i0 += W) {
+        int64_t o[W];
+#pragma unroll
+        for (int i = 0; i < W; ++i) o[i] = lds64(ks + (k0 + (i0 + i) * SF) * 8);  // zero past the range
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+          const bool v = !TAIL || k0 + (i0 + i) * SF < klim;
+          const uint32_t c = SWZ ? (u ^ kswz((i0 + i) * SF)) * ES : 0u;
+          cp_elem<ES, TAIL>(s + so + c + (uint32_t)((i0 + i) * SF * PITCH * ES), g + o[i], v);
+        }
       }
     } else {
       const bool v = !TAIL || k0 < klim;
-      const char *gk = g + (v ? lds64(ks + k0 * 8) : 0);
+      const char *gk = g + lds64(ks + k0 * 8);
 #pragma unroll
-      for (int i = 0; i < N; ++i)
-        if (i * SK < lim) cp_elem<ES, TAIL>(s + so + (uint32_t)(i * SK * ES), gk + lds64(u + i * SK * 8), v);
+      for (int i0 = 0; i0 < N; i0 += W) {
+        int64_t o[W];
+#pragma unroll
+        for (int i = 0; i < W; ++i) o[i] = lds64(u + (i0 + i) * SK * 8);
+#pragma unroll
+        for (int i = 0; i < W; ++i)
+          if ((i0 + i) * SK < lim) cp_elem<ES, TAIL>(s + so + (uint32_t)((i0 + i) * SK * ES), gk + o[i], v);
+      }
     }
   }
   __device__ __forceinline__ void load_tile(uint32_t so, uint32_t ks, int klim) const {
@@ -713,135 +729,244 @@ __global__ void __launch_bounds__(DmmaCfg<BM, BN>::THREADS, GemmOcc<BM, BN>::D)
   dmma_tile<BM, BN>(Lp, Rp, Dp, a, w, smem);
 }
 
-// ------------------------------------------------- R4 / C4 / C8: SIMT FMA
-template <typename T> struct Num;
-template <> struct Num<float> {
-  using A = float;
-  __device__ static A zero() { return 0.f; }
-  __device__ static A load(const float &x, bool) { return x; }
-  __device__ static void fma_acc(A &c, A x, A y) { c = fmaf(x, y, c); }
-  __device__ static float out(A acc, float d, double ar, double, int beta) {
-    const float v = acc * (float)ar;
-    return beta ? d + v : v;
-  }
-};
-template <> struct Num<double> {
-  using A = double;
-  __device__ static A zero() { return 0.0; }
-  __device__ static A load(const double &x, bool) { return x; }
-  __device__ static void fma_acc(A &c, A x, A y) { c = fma(x, y, c); }
-  __device__ static double out(A acc, double d, double ar, double, int beta) {
-    return beta ? fma(ar, acc, d) : ar * acc;
-  }
-};
-template <> struct Num<float2> {
-  using A = float2;
-  __device__ static A zero() { return make_float2(0.f, 0.f); }
-  __device__ static A load(const float2 &x, bool cj) { return cj ? make_float2(x.x, -x.y) : x; }
-  __device__ static void fma_acc(A &c, A x, A y) {
-    c.x = fmaf(x.x, y.x, c.x); c.x = fmaf(-x.y, y.y, c.x);
-    c.y = fmaf(x.x, y.y, c.y); c.y = fmaf(x.y, y.x, c.y);
-  }
-  __device__ static float2 out(A acc, float2 d, double ar, double ai, int beta) {
-    const float vr = acc.x * (float)ar - acc.y * (float)ai, vi = acc.x * (float)ai + acc.y * (float)ar;
-    return beta ? make_float2(d.x + vr, d.y + vi) : make_float2(vr, vi);
-  }
-};
-template <> struct Num<double2> {
-  using A = double2;
-  __device__ static A zero() { return make_double2(0.0, 0.0); }
-  __device__ static A load(const double2 &x, bool cj) { return cj ? make_double2(x.x, -x.y) : x; }
-  __device__ static void fma_acc(A &c, A x, A y) {
-    c.x = fma(x.x, y.x, c.x); c.x = fma(-x.y, y.y, c.x);
-    c.y = fma(x.x, y.y, c.y); c.y = fma(x.y, y.x, c.y);
-  }
-  __device__ static double2 out(A acc, double2 d, double ar, double ai, int beta) {
-    const double vr = acc.x * ar - acc.y * ai, vi = acc.x * ai + acc.y * ar;
-    return beta ? make_double2(d.x + vr, d.y + vi) : make_double2(vr, vi);
-  }
+// ------------------------------------------------- R4 / C4: packed FP32 FMA
+// Bound by the FP32 pipe (74 TFLOP/s nominal).  The packed form
+// fma.rn.f32x2 does two FMAs per instruction, so a k step of a thread's
+// sub-tile leaves issue slots for its shared-memory reads and for the tile
+// loads, which are the asynchronous gathers of the FP64 kernels (Side).  Each
+// accumulator is one chain of FMAs in k order, whatever the tile.
+__device__ __forceinline__ void ffma2(uint64_t &c, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+
+// A thread's sub-tile: MC x NC blocks of VE x VE elements (VE elements per
+// 16-byte shared read); block (c, d) covers rows c TMN VE + tm VE + 0..VE-1.
+template <typename T, int BM, int BN>
+struct FmmaCfg {
+  static constexpr int VE = 16 / (int)sizeof(T);
+  static constexpr int MC = sizeof(T) == 4 ? 2 : 4, NC = 2;
+  static constexpr int TMN = BM / (MC * VE), TNN = BN / (NC * VE);  // threads along m and n
+  static constexpr int THREADS = TMN * TNN;
+  static constexpr int BK = 16, STAGES = 3;
+  static constexpr int AP = BM + VE, BP = BN + VE;
+  static constexpr size_t SMEM = (size_t)STAGES * BK * (AP + BP) * sizeof(T) +
+                                 (size_t)(2 * BM + 2 * BN + 2 * kKRing * BK) * sizeof(int64_t);
 };
 
-constexpr int kSBM = 64, kSBN = 64, kSBK = 16, kSThreads = 256;
-
-template <typename T>
-__device__ __forceinline__ void simt_tile(const T *__restrict__ L, const T *__restrict__ R, T *D,
-                                          const GemmArgs &a, int tile_m, int tile_n) {
-  using A = typename Num<T>::A;
-  __shared__ A As[kSBK][kSBM + 1];
-  __shared__ A Bs[kSBK][kSBN + 1];
-  __shared__ int64_t mLs[kSBM], mDs[kSBM], nRs[kSBN], nDs[kSBN];
-  const int tid = threadIdx.x;
-  const int m0 = tile_m * kSBM, n0 = tile_n * kSBN;
-  for (int i = tid; i < kSBM; i += kSThreads) {
+template <typename T, int BM, int BN>
+__device__ __forceinline__ void fmma_tile(const T *__restrict__ L, const T *__restrict__ R, T *D, const GemmArgs &a,
+                                          const TileWork &w, unsigned char *smem) {
+  using C = FmmaCfg<T, BM, BN>;
+  constexpr int BK = C::BK, ST = C::STAGES, AP = C::AP, BP = C::BP, NT = C::THREADS, VE = C::VE;
+  constexpr int TM = C::MC * VE, TN = C::NC * VE, ES = (int)sizeof(T);
+  constexpr bool CPLX = sizeof(T) == 8;
+  T *As = reinterpret_cast<T *>(smem);
+  T *Bs = As + ST * BK * AP;
+  int64_t *mLs = reinterpret_cast<int64_t *>(Bs + ST * BK * BP);
+  int64_t *mDs = mLs + BM;
+  int64_t *nRs = mDs + BM;
+  int64_t *nDs = nRs + BN;
+  int64_t *kLs = nDs + BN;
+  int64_t *kRs = kLs + kKRing * BK;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int m0 = w.tm * BM, n0 = w.tn * BN;
+  const int mrem = a.M - m0, nrem = a.N - n0;
+  const int k0 = a.nsplit > 1 ? w.split * a.kchunk : 0;
+  const int K = a.nsplit > 1 ? min(a.kchunk, a.K - k0) : a.K;
+  const int64_t *kLg = a.kL + k0, *kRg = a.kR + k0;
+  for (int i = tid; i < BM; i += NT) {
     const int m = m0 + i;
     mLs[i] = m < a.M ? a.mL[m] : 0;
     mDs[i] = m < a.M ? a.mD[m] : 0;
   }
-  for (int i = tid; i < kSBN; i += kSThreads) {
+  for (int i = tid; i < BN; i += NT) {
     const int n = n0 + i;
     nRs[i] = n < a.N ? a.nR[n] : 0;
     nDs[i] = n < a.N ? a.nD[n] : 0;
   }
-  const int tr = tid % 16, tc = tid / 16;  // 16 x 16 threads, 4 x 4 outputs each
-  A acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = Num<T>::zero();
+  kring_init<BK, ST>(kLg, kRg, K, kLs, kRs, tid, NT);
   __syncthreads();
-  for (int k0 = 0; k0 < a.K; k0 += kSBK) {
+  const int numK = (K + BK - 1) / BK;
+  Side<BM, BK, NT, AP, ES, false> sa;
+  Side<BN, BK, NT, BP, ES, false> sb;
+  sa.init(L, mLs, As, a.a_along_m, mrem);
+  sb.init(R, nRs, Bs, a.b_along_n, nrem);
+  constexpr uint32_t SAB = BK * AP * ES, SBB = BK * BP * ES;
+  KRing<BK, ST> ring;
+  ring.init(kLg, kRg, kLs, kRs);
+  const uint32_t ksa = (uint32_t)__cvta_generic_to_shared(kLs), ksb = (uint32_t)__cvta_generic_to_shared(kRs);
+  auto load_a = [&](int kt, int s) { sa.load_tile(s * SAB, ksa + (kt % kKRing) * (BK * 8), K - kt * BK); };
+  auto load_b = [&](int kt, int s) { sb.load_tile(s * SBB, ksb + (kt % kKRing) * (BK * 8), K - kt * BK); };
+
+  const int tm = (lane & 3) + 4 * (warp % (C::TMN / 4)), tn = (lane >> 2) + 8 * (warp / (C::TMN / 4));
+  // Accumulator pairs.  Complex: acc[i][j] is element (i, j), (re, im).  Real:
+  // a pair of rows meets a pair of columns as they come from shared memory, and
+  // the pair of columns swapped: for rows i, i+1 and columns j, j+1 (all even i,
+  // j) acc[i][j/2] = (c(i,j), c(i+1,j+1)) and acc[i+1][j/2] = (c(i,j+1), c(i+1,j)).
+  // That costs one swap per column pair where pairs of equal row values would
+  // cost two moves per row.
+  constexpr int NP = CPLX ? TN : TN / 2;
+  uint64_t acc[TM][NP];
 #pragma unroll
-    for (int i = 0; i < (kSBM * kSBK) / kSThreads; ++i) {
-      const int idx = tid + i * kSThreads;
-      const int ml = a.a_along_m ? (idx % kSBM) : (idx / kSBK);
-      const int kl = a.a_along_m ? (idx / kSBM) : (idx % kSBK);
-      const int m = m0 + ml, k = k0 + kl;
-      As[kl][ml] = (m < a.M && k < a.K) ? Num<T>::load(*(const T *)((const char *)L + mLs[ml] + a.kL[k]), a.conj_l) : Num<T>::zero();
-    }
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int i = 0; i < (kSBN * kSBK) / kSThreads; ++i) {
-      const int idx = tid + i * kSThreads;
-      const int nl = a.b_along_n ? (idx % kSBN) : (idx / kSBK);
-      const int kl = a.b_along_n ? (idx / kSBN) : (idx % kSBK);
-      const int n = n0 + nl, k = k0 + kl;
-      Bs[kl][nl] = (n < a.N && k < a.K) ? Num<T>::load(*(const T *)((const char *)R + nRs[nl] + a.kR[k]), a.conj_r) : Num<T>::zero();
-    }
-    __syncthreads();
+    for (int j = 0; j < NP; ++j) acc[i][j] = 0;
+  const uint32_t cl = a.conj_l ? 0x80000000u : 0u, cr = a.conj_r ? 0x80000000u : 0u;
 #pragma unroll
-    for (int kk = 0; kk < kSBK; ++kk) {
-      A av[4], bv[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) av[i] = As[kk][tr + 16 * i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) bv[j] = Bs[kk][tc + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) Num<T>::fma_acc(acc[i][j], av[i], bv[j]);
-    }
-    __syncthreads();
+  for (int s = 0; s < ST - 1; ++s) {
+    load_a(s, s);
+    load_b(s, s);
+    cp_async_commit();
   }
+  int st = 0, ps = ST - 1;
+  for (int kt = 0; kt < numK; ++kt) {
+    cp_async_wait<ST - 2>();
+    __syncthreads();
+    const T *as = As + st * BK * AP + tm * VE;
+    const T *bs = Bs + st * BK * BP + tn * VE;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int ml = tr + 16 * i;
-    if (m0 + ml >= a.M) continue;
+    for (int k = 0; k < BK; ++k) {
+      uint64_t av[C::MC * 2], bv[C::NC * 2];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int nl = tc + 16 * j;
-      if (n0 + nl >= a.N) continue;
-      T *p = D + mDs[ml] + nDs[nl];
-      *p = Num<T>::out(acc[i][j], a.beta ? *p : T(), a.alpha_re, a.alpha_im, a.beta);
+      for (int c = 0; c < C::MC; ++c) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(as + k * AP + c * (C::TMN * VE));
+        av[2 * c] = v.x;
+        av[2 * c + 1] = v.y;
+      }
+#pragma unroll
+      for (int c = 0; c < C::NC; ++c) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(bs + k * BP + c * (C::TNN * VE));
+        bv[2 * c] = v.x;
+        bv[2 * c + 1] = v.y;
+      }
+      if constexpr (CPLX) {
+        // (re, im) += x.re (y.re, y.im), then += x.im (-y.im, y.re)
+        uint64_t by[TN], bx[TN];
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+          const float2 y = unpack2(bv[j]);
+          const float yi = __uint_as_float(__float_as_uint(y.y) ^ cr);
+          by[j] = pack2(y.x, yi);
+          bx[j] = pack2(-yi, y.x);
+        }
+#pragma unroll
+        for (int i = 0; i < TM; ++i) {
+          const float2 x = unpack2(av[i]);
+          const float xi = __uint_as_float(__float_as_uint(x.y) ^ cl);
+          const uint64_t xr2 = pack2(x.x, x.x), xi2 = pack2(xi, xi);
+#pragma unroll
+          for (int j = 0; j < TN; ++j) {
+            ffma2(acc[i][j], xr2, by[j]);
+            ffma2(acc[i][j], xi2, bx[j]);
+          }
+        }
+      } else {
+        uint64_t bs2[NP];
+#pragma unroll
+        for (int j = 0; j < NP; ++j) {
+          const float2 y = unpack2(bv[j]);
+          bs2[j] = pack2(y.y, y.x);
+        }
+#pragma unroll
+        for (int i = 0; i < TM; i += 2)
+#pragma unroll
+          for (int j = 0; j < NP; ++j) {
+            ffma2(acc[i][j], av[i / 2], bv[j]);
+            ffma2(acc[i + 1][j], av[i / 2], bs2[j]);
+          }
+      }
+      if (k == 1) load_a(kt + ST - 1, ps);
+      if (k == BK / 2 + 1) load_b(kt + ST - 1, ps);
+    }
+    ring.step(kt, K);
+    cp_async_commit();
+    ps = st;
+    st = st + 1 == ST ? 0 : st + 1;
+  }
+  cp_async_wait<0>();
+
+  if constexpr (!CPLX) {  // back to rows: acc[i][j/2] = (c(i,j), c(i,j+1))
+#pragma unroll
+    for (int i = 0; i < TM; i += 2)
+#pragma unroll
+      for (int j = 0; j < NP; ++j) {
+        const float2 d = unpack2(acc[i][j]), x = unpack2(acc[i + 1][j]);
+        acc[i][j] = pack2(d.x, x.x);
+        acc[i + 1][j] = pack2(x.y, d.y);
+      }
+  }
+  auto row_of = [&](int i) { return (i / VE) * (C::TMN * VE) + tm * VE + i % VE; };
+  auto col_of = [&](int j) { return (j / VE) * (C::TNN * VE) + tn * VE + j % VE; };
+  if (a.nsplit > 1) {
+    constexpr int NF = TM * NP / 2;  // 16-byte units: two accumulator pairs of a row
+    float4 part[NF];
+    uint32_t mask = 0;
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      const int i = f / (NP / 2), j = f % (NP / 2);
+      const float2 u = unpack2(acc[i][2 * j]), v = unpack2(acc[i][2 * j + 1]);
+      part[f] = make_float4(u.x, u.y, v.x, v.y);
+      if (row_of(i) < mrem && col_of(j * (TN * 2 / NP)) < nrem) mask |= 1u << f;
+    }
+    if (!split_combine<NF, NT>(part, mask, tid, a, w.lin, w.split)) return;
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      const int i = f / (NP / 2), j = f % (NP / 2);
+      acc[i][2 * j] = pack2(part[f].x, part[f].y);
+      acc[i][2 * j + 1] = pack2(part[f].z, part[f].w);
+    }
+  }
+  const float alr = (float)a.alpha_re, ali = (float)a.alpha_im;
+#pragma unroll
+  for (int i = 0; i < TM; ++i) {
+    const int ml = row_of(i);
+    if (ml >= mrem) continue;
+    T *p[TN], d[TN];
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+      const int nl = col_of(j);
+      p[j] = nl < nrem ? D + mDs[ml] + nDs[nl] : nullptr;
+      d[j] = (a.beta && p[j]) ? *p[j] : T();
+    }
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+      if (!p[j]) continue;
+      if constexpr (CPLX) {
+        const float2 c = unpack2(acc[i][j]);
+        const float vr = c.x * alr - c.y * ali, vi = c.x * ali + c.y * alr;
+        *p[j] = a.beta ? make_float2(d[j].x + vr, d[j].y + vi) : make_float2(vr, vi);
+      } else {
+        const float2 c = unpack2(acc[i][j / 2]);
+        const float v = ((j & 1) ? c.y : c.x) * alr;
+        *p[j] = a.beta ? d[j] + v : v;
+      }
     }
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kSThreads)
-    gemm_gather_simt_kernel(const T *__restrict__ L, const T *__restrict__ R, T *D, const GemmArgs a) {
+// Resident CTAs per SM asked of the compiler.
+template <typename T, int BM> struct FmmaOcc { static constexpr int N = 4; };
+template <> struct FmmaOcc<float, 64> { static constexpr int N = 7; };
+template <> struct FmmaOcc<float, 128> { static constexpr int N = 2; };
+
+template <typename T, int BM, int BN>
+__global__ void __launch_bounds__(FmmaCfg<T, BM, BN>::THREADS, FmmaOcc<T, BM>::N)
+    fgemm_gather_kernel(const T *__restrict__ L, const T *__restrict__ R, T *D, const GemmArgs a) {
+  extern __shared__ __align__(16) unsigned char smem[];
   const T *Lp = L, *Rp = R;
   T *Dp = D;
   const TileWork w = block_work(a, Lp, Rp, Dp);
-  simt_tile<T>(Lp, Rp, Dp, a, w.tm, w.tn);
+  fmma_tile<T, BM, BN>(Lp, Rp, Dp, a, w, smem);
 }
 
 // ------------------------------------------------------ full contraction
@@ -1066,9 +1191,21 @@ struct KSplit {
 constexpr int kSplitMinK = 256;
 KSplit k_split(int kind, int64_t M, int64_t N, int64_t K, int64_t H) {
   KSplit s;
-  if (kind != R8 && kind != C8) return s;
   const int64_t tiles = ((M + 63) / 64) * ((N + 63) / 64) * std::max<int64_t>(H, 1);
-  const int64_t want = std::min((kind == R8 ? 4 : 2) * 148 / tiles, K / kSplitMinK);
+  const int64_t most = K / kSplitMinK;
+  if (most < 2 || tiles >= 8 * 148) return s;
+  int64_t want = std::min((kind == C8 ? 2 : kind == R4 ? 6 : 4) * 148 / tiles, most);
+  if (tiles >= 148) {
+    // Every SM has a tile, but not the same number of them: cut K when that
+    // evens them out.  Cost of n cuts: items of the fullest SM times an item's
+    // length, plus about 48 k for its start and end and 32 k for its partial sums.
+    double best = 0.0;
+    want = 1;
+    for (int64_t n = 1; n <= std::min<int64_t>(most, 6); ++n) {
+      const double cost = (double)((tiles * n + 147) / 148) * ((double)K / n + (n > 1 ? 80 : 48));
+      if (n == 1 || cost < 0.97 * best) { best = cost; want = n; }
+    }
+  }
   if (want < 2) return s;
   s.kchunk = (int)(((K + want - 1) / want + 15) / 16 * 16);
   s.nsplit = (int)((K + s.kchunk - 1) / s.kchunk);
@@ -1087,13 +1224,17 @@ int64_t split_bytes(const KSplit &s, int kind, int64_t M, int64_t N, int64_t H, 
   return tiles * s.nsplit * edge * edge * kind_size(kind) + align_up(4 * split_counters(s, tiles), 256);
 }
 
-// CTA tile edge of a single FP64 contraction: 64, or 32 when even the split
-// 64 x 64 tiles do not give every SM one.  (128 x 128 tiles, one CTA of 16
+// CTA tile edge of a single contraction.  R8, C8: 64, or 32 when even the split
+// 64 x 64 tiles do not give every SM one.  (128 x 128 R8 tiles, one CTA of 16
 // warps per SM, were 1.5 % slower than four 64 x 64 CTAs on 3072 x 3072 x 3072:
-// independent CTAs fill each other's barrier gaps.)  Results do not depend on it.
-int gemm_edge(int64_t M, int64_t N, int64_t H, const KSplit &s) {
-  const int64_t tiles = ((M + 63) / 64) * ((N + 63) / 64) * std::max<int64_t>(H, 1);
-  return tiles * s.nsplit >= sm_count_dev() ? 64 : 32;
+// independent CTAs fill each other's barrier gaps.)  R4: 128 when two of those
+// per SM exist and are mostly filled, else 64.  Results do not depend on it.
+int gemm_edge(int kind, int64_t M, int64_t N, int64_t H, const KSplit &s) {
+  auto tiles = [&](int64_t e) { return ((M + e - 1) / e) * ((N + e - 1) / e) * std::max<int64_t>(H, 1); };
+  const int64_t sms = sm_count_dev();
+  if (kind == R4) return tiles(128) >= 2 * sms && tiles(64) >= 3 * tiles(128) ? 128 : 64;
+  if (kind == C4) return 64;
+  return tiles(64) * s.nsplit >= sms ? 64 : 32;
 }
 
 // Grid of a gather-GEMM launch: tiles of one GEMM times hyper combinations
@@ -1138,14 +1279,18 @@ int launch_zmma(const double2 *L, const double2 *R, double2 *D, GemmArgs ga, cud
   return check_launch("zgemm_gather_kernel");
 }
 
-template <typename T>
-int launch_simt(const void *L, const void *R, void *D, GemmArgs ga, cudaStream_t st) {
+template <typename T, int BM, int BN>
+int launch_fmma(const void *L, const void *R, void *D, GemmArgs ga, cudaStream_t st) {
+  using C = FmmaCfg<T, BM, BN>;
+  static std::atomic<uint64_t> attr_set{0};
+  once_per_device(attr_set, [] {
+    cudaFuncSetAttribute(fgemm_gather_kernel<T, BM, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+  });
   int64_t tiles = 0;
-  if (gemm_grid(ga, kSBM, kSBN, &tiles)) return TALSH_LIMIT_EXCEEDED;
-  gemm_gather_simt_kernel<T><<<(unsigned)tiles, kSThreads, 0, st>>>((const T *)L, (const T *)R,
-                                                                     (T *)D, ga);
+  if (gemm_grid(ga, BM, BN, &tiles)) return TALSH_LIMIT_EXCEEDED;
+  fgemm_gather_kernel<T, BM, BN><<<(unsigned)tiles, C::THREADS, C::SMEM, st>>>((const T *)L, (const T *)R, (T *)D, ga);
   note_launch();
-  return check_launch("gemm_gather_simt_kernel");
+  return check_launch("fgemm_gather_kernel");
 }
 
 template <typename T>
@@ -1210,7 +1355,7 @@ size_t contract_scratch_bytes(int kind, const int *cptrn, int drank, const int *
   if (least) *least = b;
   if (drank == 0) return b;
   const KSplit ks = k_split(kind, T.M, T.N, T.K, T.H);
-  return b + (size_t)split_bytes(ks, kind, T.M, T.N, T.H, gemm_edge(T.M, T.N, T.H, ks));
+  return b + (size_t)split_bytes(ks, kind, T.M, T.N, T.H, gemm_edge(kind, T.M, T.N, T.H, ks));
 }
 size_t contract_scratch_bytes(int kind, const int *cptrn, int drank, const int *ddims, int lrank,
                               const int *ldims, int rrank, const int *rdims) {
@@ -1296,11 +1441,11 @@ int contract_launch(int kind, const int *cptrn, int drank, const int *ddims, int
   int edge = 64;
   if (drank > 0) {
     ks = k_split(kind, T.M, T.N, T.K, T.H);
-    edge = gemm_edge(T.M, T.N, T.H, ks);
+    edge = gemm_edge(kind, T.M, T.N, T.H, ks);
     const int64_t extra = split_bytes(ks, kind, T.M, T.N, T.H, edge);
     if (scratch_bytes < need + (size_t)extra) {  // no room for partial sums: one CTA per tile
       ks = KSplit();
-      edge = gemm_edge(T.M, T.N, T.H, ks);
+      edge = gemm_edge(kind, T.M, T.N, T.H, ks);
     }
     const int64_t tiles = ((T.M + edge - 1) / edge) * ((T.N + edge - 1) / edge) * T.H;
     T.ncnt = split_counters(ks, tiles);
@@ -1343,8 +1488,10 @@ int contract_launch(int kind, const int *cptrn, int drank, const int *ddims, int
       if (edge == 64) return launch_dmma<64, 64>(l, r, (double *)D, ga, st);
       return launch_dmma<32, 32>(l, r, (double *)D, ga, st);
     }
-    case R4: return launch_simt<float>(L, R, D, ga, st);
-    case C4: return launch_simt<float2>(L, R, D, ga, st);
+    case R4:
+      if (edge == 128) return launch_fmma<float, 128, 128>(L, R, D, ga, st);
+      return launch_fmma<float, 64, 64>(L, R, D, ga, st);
+    case C4: return launch_fmma<float2, 64, 64>(L, R, D, ga, st);
     default:
       if (edge == 64) return launch_zmma<64, 64>((const double2 *)L, (const double2 *)R, (double2 *)D, ga, st);
       return launch_zmma<32, 32>((const double2 *)L, (const double2 *)R, (double2 *)D, ga, st);
@@ -1426,7 +1573,7 @@ struct BatchDesc {
 };
 
 // Tile configurations of the batch: 0 = DMMA 64x64, 1 = DMMA 32x32 (R8),
-// 2 = SIMT 64x64 (R4, C4, C8: one list per kind).
+// Z = complex on the DMMA pipe, S4 / S14 = packed FP32 FMA 64x64 (R4 / C4).
 enum : int { kCfgD64 = 0, kCfgD32 = 1, kCfgZ64 = 2, kCfgZ32 = 3, kCfgS4 = 4, kCfgS14 = 5, kNumCfg = 6 };
 // Square tile edge of a configuration.
 inline int cfg_tile(int c) { return (c == kCfgD32 || c == kCfgZ32) ? 32 : 64; }
@@ -1544,15 +1691,16 @@ __global__ void __launch_bounds__(ZmmaCfg<BM, BN>::THREADS, GemmOcc<BM, BN>::Z)
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kSThreads)
-    simt_batch_kernel(const BatchDesc *descs, const int32_t *list, const int64_t *prefix, int n,
+__global__ void __launch_bounds__(FmmaCfg<T, 64, 64>::THREADS, FmmaOcc<T, 64>::N)
+    fmma_batch_kernel(const BatchDesc *descs, const int32_t *list, const int64_t *prefix, int n,
                       int64_t total, unsigned long long *ctr) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ GemmArgs a;
   for (int64_t w = next_item(ctr); w < total; w = next_item(ctr)) {
     const int j = find_task(prefix, n, w);
     const BatchDesc &d = descs[list[j]];
-    const GemmArgs a = d.a;
-    const int local = (int)(w - prefix[j]);
-    simt_tile<T>((const T *)d.L, (const T *)d.R, (T *)d.D, a, local % a.tiles_m, local / a.tiles_m);
+    stage_args(a, d.a);
+    fmma_tile<T, 64, 64>((const T *)d.L, (const T *)d.R, (T *)d.D, a, item_work(a, (int)(w - prefix[j])), smem);
   }
 }
 
@@ -1742,20 +1890,14 @@ int launch_zmma_batch(const BatchPlan &bp, int c, char *base, cudaStream_t st) {
 }
 
 template <typename T>
-int launch_simt_batch(const BatchPlan &bp, int c, char *base, cudaStream_t st) {
-  const int64_t total = bp.prefix[c].back();
-  int bps = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, simt_batch_kernel<T>, kSThreads, 0) != cudaSuccess ||
-      bps < 1)
-    bps = 1;
-  cudaGetLastError();
-  const int64_t grid = std::min<int64_t>(total, (int64_t)sm_count_dev() * bps);
-  simt_batch_kernel<T><<<(unsigned)grid, kSThreads, 0, st>>>(
-      (const BatchDesc *)(base + bp.off_desc), (const int32_t *)(base + bp.off_list[c]),
-      (const int64_t *)(base + bp.off_prefix[c]), (int)bp.list[c].size(), total,
-      (unsigned long long *)(base + bp.off_ctr) + c);
-  note_launch();
-  return check_launch("simt_batch_kernel");
+int launch_fmma_batch(const BatchPlan &bp, int c, char *base, cudaStream_t st) {
+  using C = FmmaCfg<T, 64, 64>;
+  static std::atomic<uint64_t> attr{0};
+  once_per_device(attr, [] {
+    cudaFuncSetAttribute(fmma_batch_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+    cudaFuncSetAttribute(fmma_batch_kernel<T>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+  });
+  return launch_tc_batch(fmma_batch_kernel<T>, C::THREADS, C::SMEM, "fmma_batch_kernel", bp, c, base, st);
 }
 
 }  // namespace
@@ -1831,8 +1973,8 @@ int batch_run(int ntasks, const tcContractTask *tasks, BatchPlan &bp, void *scra
   if (!bp.list[kCfgD32].empty() && (rc = launch_dmma_batch<32, 32>(bp, kCfgD32, base, st)) != 0) return rc;
   if (!bp.list[kCfgZ64].empty() && (rc = launch_zmma_batch<64, 64>(bp, kCfgZ64, base, st)) != 0) return rc;
   if (!bp.list[kCfgZ32].empty() && (rc = launch_zmma_batch<32, 32>(bp, kCfgZ32, base, st)) != 0) return rc;
-  if (!bp.list[kCfgS4].empty() && (rc = launch_simt_batch<float>(bp, kCfgS4, base, st)) != 0) return rc;
-  if (!bp.list[kCfgS14].empty() && (rc = launch_simt_batch<float2>(bp, kCfgS14, base, st)) != 0) return rc;
+  if (!bp.list[kCfgS4].empty() && (rc = launch_fmma_batch<float>(bp, kCfgS4, base, st)) != 0) return rc;
+  if (!bp.list[kCfgS14].empty() && (rc = launch_fmma_batch<float2>(bp, kCfgS14, base, st)) != 0) return rc;
   for (int t = 0; t < ntasks; ++t) {
     if (bp.cfg[t] >= 0) continue;
     const tcContractTask &x = tasks[t];
@@ -1993,8 +2135,8 @@ extern "C" int tcContractBatchGraphCreate(int ntasks, const tcContractTask *task
       case kCfgD32: rc = launch_dmma_batch<32, 32>(bp, c, base, s2); break;
       case kCfgZ64: rc = launch_zmma_batch<64, 64>(bp, c, base, s2); break;
       case kCfgZ32: rc = launch_zmma_batch<32, 32>(bp, c, base, s2); break;
-      case kCfgS4: rc = launch_simt_batch<float>(bp, c, base, s2); break;
-      default: rc = launch_simt_batch<float2>(bp, c, base, s2); break;
+      case kCfgS4: rc = launch_fmma_batch<float>(bp, c, base, s2); break;
+      default: rc = launch_fmma_batch<float2>(bp, c, base, s2); break;
     }
   }
   for (int t = 0; t < ntasks && fallbacks && rc == TALSH_SUCCESS && e == cudaSuccess; ++t) {
