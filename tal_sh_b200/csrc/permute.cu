@@ -75,7 +75,7 @@ constexpr int kStages = 3;              // tile buffers per CTA of permute_tiled
 #endif
 constexpr bool kAddPrefetch = TB_ADD_PREFETCH != 0;
 __host__ __device__ constexpr int reg_stages(int esize, int op) {
-  return op == 1 ? (esize <= 4 ? TB_STAGES_ADD4 : TB_STAGES_ADD8)
+  return (op == 1 || op == 3) ? (esize <= 4 ? TB_STAGES_ADD4 : TB_STAGES_ADD8)
                  : (esize <= 4 ? TB_STAGES_COPY4 : TB_STAGES_COPY8);
 }
 
@@ -114,6 +114,8 @@ struct PermParams {
   uint32_t mg_lip, sh_lip;  // magic divisor of Li_pad
   int64_t num_tiles;
   double s_re, s_im;
+  double2 *dot_part;  // kOpDot: one partial sum per CTA
+  int dot_conj;       // kOpDot: the destination-side operand is conjugated
   const void *sdev;  // optional device scalar multiplying the scale (rank-0 operand)
   int sdev_kind, sdev_conj;
   int64_t ext[kMaxFR];
@@ -236,7 +238,7 @@ template <> struct CplxTraits<float2> { static constexpr bool value = true; };
 template <> struct CplxTraits<double2> { static constexpr bool value = true; };
 
 // Operation applied in the write phase.
-enum : int { kOpCopy = 0, kOpAdd = 1, kOpScaleCopy = 2 };
+enum : int { kOpCopy = 0, kOpAdd = 1, kOpScaleCopy = 2, kOpDot = 3 };
 
 // Effective scale when a device-resident scalar multiplies alpha (scalar x
 // tensor contractions): s = scalar * alpha as a complex(8) product, reduced to
@@ -263,6 +265,36 @@ __device__ __forceinline__ void effective_scale(const void *sdev, int sdev_kind,
     sr = fr;
     si = fi;
   }
+}
+
+// acc += d * x in double precision (complex kinds: the complex product).
+__device__ __forceinline__ void dot_acc(double2 &acc, float d, float x, bool) { acc.x = fma((double)d, (double)x, acc.x); }
+__device__ __forceinline__ void dot_acc(double2 &acc, double d, double x, bool) { acc.x = fma(d, x, acc.x); }
+__device__ __forceinline__ void dot_acc(double2 &acc, double2 d, double2 x, bool cd) {
+  const double di = cd ? -d.y : d.y;
+  acc.x = fma(-di, x.y, fma(d.x, x.x, acc.x));
+  acc.y = fma(di, x.x, fma(d.x, x.y, acc.y));
+}
+__device__ __forceinline__ void dot_acc(double2 &acc, float2 d, float2 x, bool cd) {
+  dot_acc(acc, make_double2(d.x, d.y), make_double2(x.x, x.y), cd);
+}
+
+// Sum over the CTA in a fixed order; the result is in thread 0.
+__device__ double2 cta_sum(double2 v) {
+  __shared__ double2 ws[kThreads / 32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    v.x += __shfl_down_sync(0xffffffffu, v.x, o);
+    v.y += __shfl_down_sync(0xffffffffu, v.y, o);
+  }
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int i = 1; i < kThreads / 32; ++i) {
+      v.x += ws[i].x;
+      v.y += ws[i].y;
+    }
+  return v;
 }
 
 template <typename T, int N>
@@ -434,7 +466,7 @@ __global__ void __launch_bounds__(kThreads, K <= 4 ? 4 : TB_MIN_BLOCKS8)
     permute_reg_kernel(const T *__restrict__ src, T *dst, const PermParams P) {
   constexpr int KW = K / VOUT;  // write vectors per thread
   constexpr int S = reg_stages((int)sizeof(T), OP);
-  constexpr bool DPF = OP == kOpAdd && kAddPrefetch;  // D vectors prefetched into shared slots
+  constexpr bool DPF = (OP == kOpAdd && kAddPrefetch) || OP == kOpDot;  // D vectors prefetched into shared slots
   using V = Pack<T, VOUT>;
   extern __shared__ __align__(16) unsigned char smem[];
   T *buf0 = reinterpret_cast<T *>(smem);
@@ -551,6 +583,7 @@ __global__ void __launch_bounds__(kThreads, K <= 4 ? 4 : TB_MIN_BLOCKS8)
     }
   };
 
+  double2 dot = make_double2(0.0, 0.0);
   int64_t t = blockIdx.x;
 #pragma unroll
   for (int k = 0; k < S - 1; ++k) {
@@ -595,15 +628,24 @@ __global__ void __launch_bounds__(kThreads, K <= 4 ? 4 : TB_MIN_BLOCKS8)
         for (int u = 0; u < WB; ++u) {
           if (!ok[u]) continue;
           V d = *reinterpret_cast<const V *>(ds + (size_t)((c0 + u) * kThreads) * sizeof(V));
+          if constexpr (OP == kOpDot) {
 #pragma unroll
-          for (int j = 0; j < VOUT; ++j) d.v[j] = Arith<T>::axpy(d.v[j], v[u].v[j], sr, si);
-          st_pack<T, VOUT>(gp[u], d);
+            for (int j = 0; j < VOUT; ++j) dot_acc(dot, d.v[j], v[u].v[j], P.dot_conj != 0);
+          } else {
+#pragma unroll
+            for (int j = 0; j < VOUT; ++j) d.v[j] = Arith<T>::axpy(d.v[j], v[u].v[j], sr, si);
+            st_pack<T, VOUT>(gp[u], d);
+          }
         }
       } else {
         emit_masked<T, VOUT, OP, WB>(gp, v, ok, sr, si);
       }
     }
     __syncthreads();
+  }
+  if constexpr (OP == kOpDot) {
+    dot = cta_sum(dot);
+    if (tid == 0) P.dot_part[blockIdx.x] = dot;
   }
 }
 
@@ -960,6 +1002,38 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     }
     __syncthreads();
   }
+}
+
+// Dot product of two tensors stored alike: 16-byte loads, four per operand in
+// flight, one partial sum per CTA.
+template <typename T, int VEC>
+__global__ void __launch_bounds__(kThreads) dot_linear_kernel(const T *__restrict__ src, const T *__restrict__ dst,
+                                                              int64_t nvec, int64_t vol, int conj_src,
+                                                              int conj_dst, double2 *part) {
+  double2 acc = make_double2(0.0, 0.0);
+  const int64_t step = (int64_t)gridDim.x * kThreads;
+  constexpr int U = 4;
+  auto one = [&](T d, T x) {
+    if (conj_src) x = Arith<T>::conj(x);
+    dot_acc(acc, d, x, conj_dst != 0);
+  };
+  for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < nvec; i += U * step) {
+    Pack<T, VEC> x[U], d[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i + u * step < nvec) {
+        x[u] = ld_pack<T, VEC>(src + (i + u * step) * VEC);
+        d[u] = ld_pack<T, VEC>(dst + (i + u * step) * VEC);
+      }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i + u * step < nvec)
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) one(d[u].v[j], x[u].v[j]);
+  }
+  for (int64_t i = nvec * VEC + (int64_t)blockIdx.x * kThreads + threadIdx.x; i < vol; i += step) one(dst[i], src[i]);
+  acc = cta_sum(acc);
+  if (threadIdx.x == 0) part[blockIdx.x] = acc;
 }
 
 // Identity permutation after fusion: straight streaming copy / add.
@@ -1804,6 +1878,76 @@ extern "C" void tcTensorPermuteTuneReset(void) {
 }
 
 namespace tb {
+namespace {
+template <typename T>
+int launch_dot_typed(Plan &plan, const void *src, const void *dst, int conj_src, int conj_dst,
+                     double2 *part, int64_t max_parts, int *nparts, cudaStream_t st) {
+  constexpr int VEC = 16 / sizeof(T);
+  const int sms = current_sm_count();
+  if (plan.linear) {
+    const bool aligned = ((uintptr_t)src % 16 == 0) && ((uintptr_t)dst % 16 == 0);
+    const int64_t nvec = aligned ? plan.vol / VEC : 0;
+    const int64_t want = (std::max<int64_t>(nvec, plan.vol - nvec * VEC) + 4 * kThreads - 1) / (4 * kThreads);
+    const int64_t grid = std::min<int64_t>(std::min<int64_t>(want, (int64_t)sms * 8), max_parts);
+    dot_linear_kernel<T, VEC><<<(unsigned)grid, kThreads, 0, st>>>((const T *)src, (const T *)dst, nvec, plan.vol,
+                                                                  conj_src, conj_dst, part);
+    *nparts = (int)grid;
+    note_launch();
+    return check_launch("dot_linear_kernel");
+  }
+  PermParams &P = plan.P;
+  if (!P.reg) return TALSH_NOT_IMPLEMENTED;
+  P.conj = conj_src;
+  P.dot_conj = conj_dst;
+  P.dot_part = part;
+  int vout = plan.vout == VEC && (uintptr_t)dst % 16 == 0 ? VEC : 1;
+  P.y_step = (P.ymap.n >= 1 && P.ymap.ext[0] % vout == 0) ? 1 : 0;
+  P.nv = P.Lo / vout;
+  make_magic((uint32_t)P.nv, P.mg_nv, P.sh_nv);
+  constexpr int K = sizeof(T) >= 16 ? 4 : 8;
+  const size_t bufs = (size_t)reg_stages((int)sizeof(T), kOpDot) * (P.buf_elems + K * kThreads) * sizeof(T);
+  const size_t smem = std::max(plan.smem, bufs);
+  auto run = [&](auto kern) {
+    const int64_t grid = std::min<int64_t>(std::min<int64_t>(P.num_tiles, (int64_t)sms * blocks_per_sm((const void *)kern, smem)),
+                                           max_parts);
+    kern<<<(unsigned)grid, kThreads, smem, st>>>((const T *)src, const_cast<T *>((const T *)dst), P);
+    *nparts = (int)grid;
+  };
+  if (vout == VEC) {
+    if (P.swz) run(permute_reg_kernel<T, K, VEC, kOpDot, true>);
+    else run(permute_reg_kernel<T, K, VEC, kOpDot, false>);
+  } else {
+    if (P.swz) run(permute_reg_kernel<T, K, 1, kOpDot, true>);
+    else run(permute_reg_kernel<T, K, 1, kOpDot, false>);
+  }
+  note_launch();
+  return check_launch("permute_reg_kernel (dot)");
+}
+}  // namespace
+
+// Partial sums of sum_i dst[O2N(i)] * src[i] over all elements, in double: the
+// full contraction of two tensors, read once each along their own runs by the
+// transpose-add kernel (its destination prefetch supplies the other factor;
+// nothing is written).  One partial per CTA, at most max_parts of them, in
+// part[0 .. *nparts).  TALSH_NOT_IMPLEMENTED: no register-table plan.
+int permute_dot_launch(int kind, int rank, const int *dims, const int *o2n, const void *src, const void *dst,
+                       int conj_src, int conj_dst, double2 *part, int64_t max_parts, int *nparts, cudaStream_t st) {
+  int rc = validate(kind, rank, dims, o2n);
+  if (rc) return rc;
+  Fused F;
+  if ((rc = fuse_dims(rank, dims, o2n, F)) != 0) return rc;
+  Plan plan;
+  PlanCfg cfg;
+  cfg.bulk = 0;
+  if ((rc = build_plan(kind_size(kind), F, plan, kOpAdd, cfg)) != 0) return TALSH_NOT_IMPLEMENTED;
+  switch (kind) {
+    case R4: return launch_dot_typed<float>(plan, src, dst, conj_src, conj_dst, part, max_parts, nparts, st);
+    case R8: return launch_dot_typed<double>(plan, src, dst, conj_src, conj_dst, part, max_parts, nparts, st);
+    case C4: return launch_dot_typed<float2>(plan, src, dst, conj_src, conj_dst, part, max_parts, nparts, st);
+    default: return launch_dot_typed<double2>(plan, src, dst, conj_src, conj_dst, part, max_parts, nparts, st);
+  }
+}
+
 // dst = permute(src) on a given stream, for the library's own staging steps.
 int permute_launch_o2n(int kind, int rank, const int *dims, const int *o2n, const void *src, void *dst,
                        cudaStream_t st) {
