@@ -42,17 +42,40 @@ template <> struct ScaleOp<double2> {
   __device__ static double absd(double2 x) { return hypot(x.x, x.y); }
 };
 
+// Elements move as 16-byte units wherever the body is 16-byte aligned (Pack),
+// four units in flight per thread.
+template <typename T> struct alignas(16) Pack { T v[16 / sizeof(T)]; };
+template <typename T> constexpr int kVec = 16 / (int)sizeof(T);
+
 template <typename T>
-__global__ void __launch_bounds__(kThreads) init_kernel(T *dst, int64_t vol, T val) {
-  const int64_t stride = (int64_t)gridDim.x * kThreads;
-  for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < vol; i += stride) dst[i] = val;
+__global__ void __launch_bounds__(kThreads) init_kernel(T *dst, int64_t nvec, int64_t vol, T val) {
+  const int64_t stride = (int64_t)gridDim.x * kThreads, t = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  Pack<T> p;
+#pragma unroll
+  for (int j = 0; j < kVec<T>; ++j) p.v[j] = val;
+  for (int64_t i = t; i < nvec; i += stride) reinterpret_cast<Pack<T> *>(dst)[i] = p;
+  for (int64_t i = nvec * kVec<T> + t; i < vol; i += stride) dst[i] = val;
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads) scale_kernel(T *dst, int64_t vol, double sr, double si) {
-  const int64_t stride = (int64_t)gridDim.x * kThreads;
-  for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < vol; i += stride)
-    dst[i] = ScaleOp<T>::apply(dst[i], sr, si);
+__global__ void __launch_bounds__(kThreads) scale_kernel(T *dst, int64_t nvec, int64_t vol, double sr, double si) {
+  const int64_t stride = (int64_t)gridDim.x * kThreads, t = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  Pack<T> *d = reinterpret_cast<Pack<T> *>(dst);
+  constexpr int U = 4;
+  for (int64_t i = t; i < nvec; i += U * stride) {
+    Pack<T> p[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i + u * stride < nvec) p[u] = d[i + u * stride];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (i + u * stride >= nvec) continue;
+#pragma unroll
+      for (int j = 0; j < kVec<T>; ++j) p[u].v[j] = ScaleOp<T>::apply(p[u].v[j], sr, si);
+      d[i + u * stride] = p[u];
+    }
+  }
+  for (int64_t i = nvec * kVec<T> + t; i < vol; i += stride) dst[i] = ScaleOp<T>::apply(dst[i], sr, si);
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -76,15 +99,37 @@ __device__ double block_sum(double v) {
   return r;  // valid in thread 0
 }
 
-// Pass 1: block b sums the contiguous chunk [b*chunk, min((b+1)*chunk, vol)).
-template <typename T>
+// Pass 1: block b sums the units [b*chunk, min((b+1)*chunk, units)), a unit
+// being 16 bytes of elements; the same elements go to the same thread in the
+// same order whether or not the body allows 16-byte loads.
+template <typename T, bool VECTOR>
 __global__ void __launch_bounds__(kThreads) norm1_partial_kernel(const T *__restrict__ src,
                                                                  int64_t vol, int64_t chunk,
                                                                  double *partial) {
-  const int64_t beg = (int64_t)blockIdx.x * chunk;
-  const int64_t end = min(vol, beg + chunk);
+  constexpr int V = kVec<T>, U = 4;
+  const int64_t units = (vol + V - 1) / V, whole = vol / V;
+  const int64_t beg = (int64_t)blockIdx.x * chunk, end = min(units, beg + chunk);
   double acc = 0.0;
-  for (int64_t i = beg + threadIdx.x; i < end; i += kThreads) acc += ScaleOp<T>::absd(src[i]);
+  for (int64_t i = beg + threadIdx.x; i < end; i += U * kThreads) {
+    Pack<T> p[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t k = i + u * kThreads;
+      if (k >= end) continue;
+      if (VECTOR && k < whole) {
+        p[u] = reinterpret_cast<const Pack<T> *>(src)[k];
+      } else {
+#pragma unroll
+        for (int j = 0; j < V; ++j) p[u].v[j] = k * V + j < vol ? src[k * V + j] : T();
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (i + u * kThreads >= end) continue;
+#pragma unroll
+      for (int j = 0; j < V; ++j) acc += ScaleOp<T>::absd(p[u].v[j]);
+    }
+  }
   const double s = block_sum(acc);
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }
@@ -97,6 +142,9 @@ __global__ void __launch_bounds__(kThreads) norm1_final_kernel(const double *par
   const double s = block_sum(acc);
   if (threadIdx.x == 0) *result = s;
 }
+
+// 16-byte units of a body (0 when it is not aligned for them).
+template <typename T> int64_t vec_units(const void *p, int64_t vol) { return (uintptr_t)p % 16 == 0 ? vol / kVec<T> : 0; }
 
 int grid_for(int64_t n) {
   const int64_t g = (n + kThreads - 1) / kThreads;
@@ -129,17 +177,17 @@ extern "C" int tcTensorInit(int data_kind, size_t vol, void *dst, double val_re,
   if (vol > 0 && !elem_aligned(data_kind, dst)) return TALSH_INVALID_ARGS;
   if (vol == 0) return TALSH_SUCCESS;
   cudaStream_t st = (cudaStream_t)stream;
-  const int grid = grid_for((int64_t)vol);
+  const int64_t n = (int64_t)vol;
+  auto go = [&](auto val) {
+    using T = decltype(val);
+    const int64_t nv = vec_units<T>(dst, n);
+    init_kernel<T><<<grid_for(std::max(nv, n - nv * kVec<T>)), kThreads, 0, st>>>((T *)dst, nv, n, val);
+  };
   switch (data_kind) {
-    case R4: init_kernel<float><<<grid, kThreads, 0, st>>>((float *)dst, vol, (float)val_re); break;
-    case R8: init_kernel<double><<<grid, kThreads, 0, st>>>((double *)dst, vol, val_re); break;
-    case C4:
-      init_kernel<float2><<<grid, kThreads, 0, st>>>((float2 *)dst, vol,
-                                                     make_float2((float)val_re, (float)val_im));
-      break;
-    case C8:
-      init_kernel<double2><<<grid, kThreads, 0, st>>>((double2 *)dst, vol, make_double2(val_re, val_im));
-      break;
+    case R4: go((float)val_re); break;
+    case R8: go(val_re); break;
+    case C4: go(make_float2((float)val_re, (float)val_im)); break;
+    case C8: go(make_double2(val_re, val_im)); break;
   }
   note_launch();
   return check_launch("init_kernel");
@@ -151,14 +199,19 @@ extern "C" int tcTensorScale(int data_kind, size_t vol, void *dst, double alpha_
   if (vol > 0 && !elem_aligned(data_kind, dst)) return TALSH_INVALID_ARGS;
   if (vol == 0) return TALSH_SUCCESS;
   cudaStream_t st = (cudaStream_t)stream;
-  const int grid = grid_for((int64_t)vol);
+  const int64_t n = (int64_t)vol;
   double sr = alpha_re, si = alpha_im;
   if (!kind_is_complex(data_kind)) { sr = cmplx8_to_real8(alpha_re, alpha_im); si = 0.0; }
+  auto go = [&](auto zero) {
+    using T = decltype(zero);
+    const int64_t nv = vec_units<T>(dst, n);
+    scale_kernel<T><<<grid_for(std::max((nv + 3) / 4, n - nv * kVec<T>)), kThreads, 0, st>>>((T *)dst, nv, n, sr, si);
+  };
   switch (data_kind) {
-    case R4: scale_kernel<float><<<grid, kThreads, 0, st>>>((float *)dst, vol, sr, si); break;
-    case R8: scale_kernel<double><<<grid, kThreads, 0, st>>>((double *)dst, vol, sr, si); break;
-    case C4: scale_kernel<float2><<<grid, kThreads, 0, st>>>((float2 *)dst, vol, sr, si); break;
-    case C8: scale_kernel<double2><<<grid, kThreads, 0, st>>>((double2 *)dst, vol, sr, si); break;
+    case R4: go(float()); break;
+    case R8: go(double()); break;
+    case C4: go(float2()); break;
+    case C8: go(double2()); break;
   }
   note_launch();
   return check_launch("scale_kernel");
@@ -171,12 +224,17 @@ namespace tb {
 int norm1_launch(int data_kind, size_t vol, const void *src, double *result_dev, double *partial,
                  cudaStream_t st) {
   const int nb = norm1_blocks(vol);
-  const int64_t chunk = (int64_t)((vol + nb - 1) / nb);
+  auto go = [&](auto zero) {
+    using T = decltype(zero);
+    const int64_t n = (int64_t)vol, units = (n + kVec<T> - 1) / kVec<T>, chunk = (units + nb - 1) / nb;
+    if ((uintptr_t)src % 16 == 0) norm1_partial_kernel<T, true><<<nb, kThreads, 0, st>>>((const T *)src, n, chunk, partial);
+    else norm1_partial_kernel<T, false><<<nb, kThreads, 0, st>>>((const T *)src, n, chunk, partial);
+  };
   switch (data_kind) {
-    case R4: norm1_partial_kernel<float><<<nb, kThreads, 0, st>>>((const float *)src, vol, chunk, partial); break;
-    case R8: norm1_partial_kernel<double><<<nb, kThreads, 0, st>>>((const double *)src, vol, chunk, partial); break;
-    case C4: norm1_partial_kernel<float2><<<nb, kThreads, 0, st>>>((const float2 *)src, vol, chunk, partial); break;
-    case C8: norm1_partial_kernel<double2><<<nb, kThreads, 0, st>>>((const double2 *)src, vol, chunk, partial); break;
+    case R4: go(float()); break;
+    case R8: go(double()); break;
+    case C4: go(float2()); break;
+    case C8: go(double2()); break;
     default: return TALSH_INVALID_ARGS;
   }
   note_launch();

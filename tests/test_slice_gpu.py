@@ -99,3 +99,37 @@ def test_talsh_slice_and_insert(talsh, kind):
     assert Lb.talshTensorSlice(dt.ref, lt.ref, T.ivec([13, 0, 0]), 0, T.DEV_NVIDIA_GPU, T.COPY_TT, T.NOPE,
                                None) == T.TALSH_INVALID_ARGS
     dt.destruct(); lt.destruct()
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_slice_insert_units(talsh, kind):
+    """Every copy unit (16, 8 bytes, one element): runs, origins, strides or bodies that only the narrower ones
+    divide, against numpy, bit-exact; fully covered middle dimensions continue the one before."""
+    torch = pytest.importorskip("torch")
+    L, rng = T.lib(), np.random.default_rng(77)
+    s = torch.cuda.current_stream().cuda_stream
+    cases = [([64, 9, 5], [32, 9, 5], [16, 0, 0]), ([64, 9, 5], [32, 4, 5], [2, 1, 0]), ([62, 9, 5], [31, 4, 2], [3, 1, 0]),
+             ([12, 7, 6, 4], [8, 7, 6, 2], [4, 0, 0, 1]), ([2051], [1026], [1]), ([5, 1, 7], [4, 1, 7], [0, 0, 0]),
+             ([6, 8, 3, 3], [6, 8, 1, 2], [0, 0, 2, 1])]
+    for (full, sl, off), shift in [(c, k) for c in cases for k in (0, 1)]:
+        F, S = rand(full, kind, rng), rand(sl, kind, rng)
+        where = tuple(slice(o, o + n) for o, n in zip(off, sl))
+        for insert in (False, True):
+            for acc in (0, 1):
+                a, b = (S, F) if insert else (F, S)
+                ref = b.copy(order="F")
+                if insert:
+                    ref[where] = ref[where] + a if acc else a
+                else:
+                    ref[...] = ref + a[where] if acc else a[where]
+                bufs = []
+                for x in (a, b):
+                    t = torch.empty(x.size + shift, dtype=_dev(torch, x).dtype, device="cuda")[shift:]
+                    t.copy_(_dev(torch, x))
+                    bufs.append(t)
+                fn = L.tcTensorInsert if insert else L.tcTensorSlice
+                rc = fn(kind, len(full), T.ivec(full), T.ivec(sl), T.ivec(off), bufs[0].data_ptr(), bufs[1].data_ptr(),
+                        acc, s)
+                torch.cuda.synchronize()
+                assert rc == 0 and bufs[1].cpu().numpy().tobytes() == ref.tobytes(order="F"), (full, sl, off, shift,
+                                                                                                  insert, acc)
