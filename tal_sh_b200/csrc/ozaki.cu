@@ -532,8 +532,9 @@ constexpr int kWsDiagPerPass = 3;             // accumulators per pass: 3 x 128 
 // format (bits 4-5: 1 F32, 2 S32), A/B formats (bits 7-9, 10-12: signed int8
 // 1; bf16 1 and tf32 2 of kind::f16/tf32; e4m3 0 of kind::f8f6f4).
 constexpr uint32_t kIdescMN128 = ((uint32_t)(kWsBN >> 3) << 17) | ((uint32_t)(kOzBM >> 4) << 24);
-// M = 256 (a CTA pair, cta_group::2), N = 256.
-constexpr uint32_t kIdescPair = ((uint32_t)(256 >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+// M = 256 (a CTA pair, cta_group::2); the N field is added at run time.
+constexpr uint32_t kIdescPair = (uint32_t)(256 >> 4) << 24;
+inline __host__ __device__ uint32_t idesc_n(int n) { return (uint32_t)(n >> 3) << 17; }
 template <int FORM> struct FormMma;
 template <> struct FormMma<kFormInt8> {
   static constexpr uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | kIdescMN128;
@@ -544,11 +545,11 @@ template <> struct FormMma<kFormInt8> {
         "l"(a), "l"(b), "r"(idesc), "r"(acc));
   }
   static constexpr uint32_t idesc_pair = (2u << 4) | (1u << 7) | (1u << 10) | kIdescPair;
-  __device__ static void mma_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t acc) {
+  __device__ static void mma_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t n, uint32_t acc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
-        "l"(a), "l"(b), "r"(idesc_pair), "r"(acc));
+        "l"(a), "l"(b), "r"(idesc_pair | n), "r"(acc));
   }
 };
 template <> struct FormMma<kFormBF16> {
@@ -560,11 +561,11 @@ template <> struct FormMma<kFormBF16> {
         "l"(a), "l"(b), "r"(idesc), "r"(acc));
   }
   static constexpr uint32_t idesc_pair = (1u << 4) | (1u << 7) | (1u << 10) | kIdescPair;
-  __device__ static void mma_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t acc) {
+  __device__ static void mma_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t n, uint32_t acc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
-        "l"(a), "l"(b), "r"(idesc_pair), "r"(acc));
+        "l"(a), "l"(b), "r"(idesc_pair | n), "r"(acc));
   }
 };
 template <> struct FormMma<kFormTF32> {
@@ -576,11 +577,11 @@ template <> struct FormMma<kFormTF32> {
         "l"(a), "l"(b), "r"(idesc), "r"(acc));
   }
   static constexpr uint32_t idesc_pair = (1u << 4) | (2u << 7) | (2u << 10) | kIdescPair;
-  __device__ static void mma_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t acc) {
+  __device__ static void mma_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t n, uint32_t acc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
-        "l"(a), "l"(b), "r"(idesc_pair), "r"(acc));
+        "l"(a), "l"(b), "r"(idesc_pair | n), "r"(acc));
   }
 };
 template <> struct FormMma<kFormFP8> {
@@ -592,11 +593,11 @@ template <> struct FormMma<kFormFP8> {
         "l"(a), "l"(b), "r"(idesc), "r"(acc));
   }
   static constexpr uint32_t idesc_pair = (1u << 4) | (0u << 7) | (0u << 10) | kIdescPair;
-  __device__ static void mma_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t acc) {
+  __device__ static void mma_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t n, uint32_t acc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
-        "l"(a), "l"(b), "r"(idesc_pair), "r"(acc));
+        "l"(a), "l"(b), "r"(idesc_pair | n), "r"(acc));
   }
 };
 
@@ -891,14 +892,18 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity
   return false;
 }
 
-constexpr int kPairBN = 256;                 // tile columns of the pair (UMMA N)
+// Tile columns of the pair (UMMA N): at most 256, in steps of 32.  A launch
+// takes the width that gives the least work per SM (pair_tile_n): 256-wide
+// tiles leave most of the last wave empty when there are few of them.
+constexpr int kPairBN = 256;
 constexpr int kPairDiag = 2;                 // accumulators per pass: 2 x 256 TMEM columns
-constexpr int kPairBTile = 128 * kWsBox;     // 8 KB: this CTA's 128 rows of a B slice box
+constexpr int kPairBTile = 128 * kWsBox;     // 8 KB: room for this CTA's nt / 2 rows of a B slice box
 
 struct OzPairArgs {
   uint32_t spin_limit;
   int64_t Mp, Np;
-  int tiles_m2, tiles_n;  // 256-row and 128-column tiles
+  int tiles_m2, tiles_n;  // 256-row and nt-column tiles
+  int nt;
   int group_m;            // pair tiles along m per raster group
   int64_t kb0, kb1;
   int S, nst;
@@ -926,7 +931,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kOzWsThreads, 1)
   const int S = a.S, nst = a.nst;
   const int slot_bytes = S * (kWsATile + kPairBTile);
   const int npass = (S + kPairDiag - 1) / kPairDiag;
-  int tm, tn;  // 256-row tile of the pair, 128-column tile
+  const int nt = a.nt;
+  int tm, tn;  // 256-row tile of the pair, nt-column tile
   {
     const int id = blockIdx.x >> 1;
     const int per_group = a.group_m * a.tiles_n;
@@ -983,7 +989,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kOzWsThreads, 1)
           }
           issued_all = itg + 1;
           // the even CTA expects the bytes of both CTAs' copies of this stage
-          if (rank == 0) mbar_expect_tx(&full[st], (uint32_t)(2 * nk * smax * (kWsATile + kPairBTile)));
+          if (rank == 0) mbar_expect_tx(&full[st], (uint32_t)(2 * nk * smax * (kWsATile + nt / 2 * kWsBox)));
           const uint32_t fbar = mapa_rank(smem_u32(&full[st]), 0);
           const uint32_t sst = sbase + (uint32_t)(st * slot_bytes);
           for (int j = 0; j < nk; ++j) {
@@ -992,7 +998,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kOzWsThreads, 1)
               const uint32_t sa = sst + (uint32_t)((j * smax + s) * kWsATile);
               const uint32_t sb = sst + (uint32_t)(S * kWsATile + (j * smax + s) * kPairBTile);
               tma_load_2d_pair(sa, &mapA, kx, (int)(s * a.Mp + tm * 256 + rank * 128), fbar);
-              tma_load_2d_pair(sb, &mapB, kx, (int)(s * a.Np + tn * kPairBN + rank * 128), fbar);
+              tma_load_2d_pair(sb, &mapB, kx, (int)(s * a.Np + tn * nt + rank * (nt / 2)), fbar);
             }
           }
         }
@@ -1029,7 +1035,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kOzWsThreads, 1)
                   const uint32_t sa = sst + (uint32_t)((j * smax + s1 - 1) * kWsATile + kk * kWsBK);
                   const uint32_t sb =
                       sst + (uint32_t)(S * kWsATile + (j * smax + g - s1 - 1) * kPairBTile + kk * kWsBK);
-                  FormMma<FORM>::mma_pair(dcol, make_desc_sw64(sa), make_desc_sw64(sb),
+                  FormMma<FORM>::mma_pair(dcol, make_desc_sw64(sa), make_desc_sw64(sb), idesc_n(nt),
                                           (it > 0 || j > 0 || kk > 0 || s1 > 1) ? 1u : 0u);
                 }
               }
@@ -1057,13 +1063,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kOzWsThreads, 1)
       const bool first = (p == 0);
       if (ok) {
         const bool rd = !(first && !a.beta);
-        for (int c = 0; c < kPairBN / 16; ++c) {
+        for (int c = 0; c < nt / 16; ++c) {
           double *ptr[16];
           double old[16];
           int esc[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            const int64_t n = (int64_t)tn * kPairBN + c * 16 + i;
+            const int64_t n = (int64_t)tn * nt + c * 16 + i;
             const bool okn = mrow && n < a.N;
             ptr[i] = okn ? a.D + dm + a.nD[n] : nullptr;
             esc[i] = okn ? em + a.eb[n] : 0;
@@ -1358,6 +1364,24 @@ int launch_pair_form(const CUtensorMap &mapA, const CUtensorMap &mapB, OzPairArg
   return TALSH_SUCCESS;
 }
 
+// Tile width of the CTA-pair kernel: the one with the least time for the
+// fullest pair of SMs, waves x (columns + 16 for a tile's epilogue and start).
+// 2640 x 2805: 121 256-wide tiles are two waves on 74 pairs, 143 224-wide ones
+// too, 12 % less work each (801 -> 757 us for the whole contraction, K = 2480,
+// six int8 slices).
+// Rows of B beyond N belong to the next slice or are zero-filled past the
+// last; they only reach columns that are not stored.
+int pair_tile_n(int64_t Mp, int64_t N) {
+  const int64_t pairs = std::max(1, current_sm_count() / 2), tm = Mp / 256;
+  int best = kPairBN;
+  int64_t least = 0;
+  for (int nt = kPairBN; nt >= 128; nt -= 32) {
+    const int64_t cost = (tm * ((N + nt - 1) / nt) + pairs - 1) / pairs * (nt + 16);
+    if (nt == kPairBN || cost < least) { least = cost; best = nt; }
+  }
+  return best;
+}
+
 // The warp-specialised GEMM of one form over K-step launches [0, nkb32) in
 // chunks of kc32 steps (32 bytes each).
 template <int FORM>
@@ -1438,10 +1462,11 @@ int contract_split_launch(int kind, const int *cptrn, int drank, const int *ddim
   CUtensorMap mapA, mapB;
   std::memset(&mapA, 0, sizeof(mapA));
   std::memset(&mapB, 0, sizeof(mapB));
+  const int nt = pair_tile_n(p.Mp, N);
   const bool pair = !simple && g_stall_test.load() == 0 && split_pair_wanted(p.Mp, p.Np) &&
-                    (int64_t)slices * p.Mp < 0x7fffffffLL && (int64_t)slices * p.Np < 0x7fffffffLL &&
+                    (int64_t)slices * p.Mp < 0x7fffffffLL && (int64_t)slices * p.Np + 512 < 0x7fffffffLL &&
                     make_slice_map(&mapA, As, Kbytes, slices * p.Mp, kOzBM) &&
-                    make_slice_map(&mapB, Bs, Kbytes, slices * p.Np, 128);
+                    make_slice_map(&mapB, Bs, Kbytes, slices * p.Np, nt / 2);
   const int tiled = (!simple && !pair) ? 1 : 0;
   auto split_float = [&](auto kern) {
     kern<<<(unsigned)p.Mp, 256, 0, st>>>(A64, M, K, p.Mp, p.Kp, slices, (unsigned char *)As, ea, tiled);
@@ -1492,7 +1517,8 @@ int contract_split_launch(int kind, const int *cptrn, int drank, const int *ddim
     w.Mp = p.Mp; w.Np = p.Np; w.S = slices;
     w.nst = std::max(2, std::min(8, kOzPairSmem / stage_bytes));
     w.tiles_m2 = (int)(p.Mp / (2 * kOzBM));
-    w.tiles_n = (int)(p.Np / kPairBN);
+    w.nt = nt;
+    w.tiles_n = (int)((N + nt - 1) / nt);
     w.group_m = std::max(1, ws_group_m() / 2);
     w.ea = ea; w.eb = eb; w.D = (double *)D; w.mD = mD; w.nD = nD; w.M = M; w.N = N;
     w.alpha = alpha_re; w.err = err;
