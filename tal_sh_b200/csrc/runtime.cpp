@@ -369,6 +369,7 @@ struct TaskRec {
   int nargs = 0;
   ArgRec a[MAX_TENSOR_OPERANDS];
   void *scratch = nullptr;
+  bool timed = true;     // the task's events also time it (a caller's task object can ask)
   int split_slices = 0;  // > 0: the contraction runs in the split-precision form
   int failed = 0;
   bool finalized = false;
@@ -386,7 +387,7 @@ int task_finalize(talsh_task_t *task, bool success) {
   TaskRec *tr = rec_of(task);
   if (tr == nullptr || tr->finalized) return TALSH_SUCCESS;
   int rc = TALSH_SUCCESS;
-  if (success) {
+  if (success && tr->timed) {
     float ms = 0.f;
     if (cudaEventElapsedTime(&ms, tr->ev[0], tr->ev[3]) == cudaSuccess) tr->times[0] = ms * 1e-3;
     if (cudaEventElapsedTime(&ms, tr->ev[1], tr->ev[2]) == cudaSuccess) tr->times[1] = ms * 1e-3;
@@ -726,12 +727,16 @@ int schedule(OpSpec &op, int dev_id, int dev_kind, talsh_task_t *user_task) {
   cudaStream_t st = G.stream;
   for (auto &e : tr->ev) e = event_get(gpu);
   int rc = TALSH_SUCCESS;
-  cudaEventRecord(tr->ev[0], st);  // after the staging buffers' stream-ordered allocation
   bool any_in = false, any_out = false;
   for (int k = 0; k < op.nt; ++k) {
     any_in = any_in || (tr->a[k].dalloc && tr->a[k].need_input);
     any_out = any_out || tr->a[k].copy_back;
   }
+  // A blocking call's task never leaves this function: its time marks would
+  // only cost (three records and four differences took 17 of the 43 us of a
+  // small call), so it records the events that order its copies and its last one.
+  tr->timed = user_task != nullptr;
+  if (tr->timed || any_in) cudaEventRecord(tr->ev[0], st);  // after the staging buffers' stream-ordered allocation
   if (any_in) {
     // Consecutive tasks stage on alternating streams.  Ordering stays safe: a
     // staging read waits for copies back into its Host range (wait_pending),
@@ -748,7 +753,7 @@ int schedule(OpSpec &op, int dev_id, int dev_kind, talsh_task_t *user_task) {
     }
     cudaEventRecord(tr->ev[1], hs);
     cudaStreamWaitEvent(st, tr->ev[1], 0);
-  } else {
+  } else if (tr->timed) {
     cudaEventRecord(tr->ev[1], st);
   }
   if (rc == TALSH_SUCCESS) {
@@ -808,7 +813,7 @@ int schedule(OpSpec &op, int dev_id, int dev_kind, talsh_task_t *user_task) {
         break;
     }
   }
-  cudaEventRecord(tr->ev[2], st);
+  if (tr->timed || any_out) cudaEventRecord(tr->ev[2], st);
   if (any_out) {
     cudaStreamWaitEvent(G.d2h, tr->ev[2], 0);
     for (int k = 0; k < op.nt && rc == TALSH_SUCCESS; ++k) {
