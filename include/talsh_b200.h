@@ -91,8 +91,11 @@ size_t tcTensorNorm1Scratch(size_t vol);
 int tcTensorNorm1(int data_kind, size_t vol, const void *src, double *result_dev, void *scratch,
                   size_t scratch_bytes, void *stream);
 
-/* Bytes of device scratch tcTensorContract needs for this shape (offset
- * tables of the gather-GEMM, plus the partial sums of a full contraction). */
+/* Bytes of device scratch tcTensorContract uses for this shape: the offset
+ * tables (16 bytes per value of each index group) and, where a long contracted
+ * range is split over CTAs, the partial sums.  A call given less, but at least
+ * the tables, or a scratch that is not 16-byte aligned, runs unsplit (another
+ * summation order); below the tables it is refused. */
 size_t tcTensorContractScratch(int data_kind, const int *cptrn, int drank, const int *ddims,
                                int lrank, const int *ldims, int rrank, const int *rdims);
 
@@ -219,17 +222,17 @@ typedef struct {
   int conj_bits, accumulative;
 } tcContractTask;
 
-/* Bytes of device scratch tcTensorContractBatch needs for these tasks (0 when
- * a task is invalid). */
+/* Bytes of device scratch tcTensorContractBatch uses for these tasks (0 when
+ * a task is invalid).  With less, as long as it holds all but the partial sums
+ * of split contracted ranges, the batch runs unsplit; below that it is refused. */
 size_t tcTensorContractBatchScratch(int ntasks, const tcContractTask *tasks);
 
 /* Runs every task with tcTensorContract's semantics.  The tasks' offset
  * tables are built by one launch and the GEMM tiles of all tasks run in one
  * persistent launch per tile configuration (FP64 tensor-pipe 64x64 or 32x32
- * tiles for R8 and C8, SIMT for R4/C4), each CTA finding its task from a tile
+ * tiles for R8 and C8, packed FP32 FMA for R4/C4), each CTA finding its task from a tile
  * prefix sum (a full
- * contraction is a 1 x 1 tile: its sum order differs from tcTensorContract's
- * two-pass dot product); scalar operands and hyper-indices take the
+ * contraction is a 1 x 1 tile: its sum order differs from tcTensorContract's); scalar operands and hyper-indices take the
  * single-task path.
  * Tasks must not write overlapping D regions (they run concurrently).  A
  * batched form of gpu_tensor_block_contract_dlf; no reference
@@ -347,7 +350,7 @@ void tcTensorContractBatchTuneReset(void);
  * not allowed).  Same arguments and results as tcTensorContract minus the
  * scratch pair.  Its scratch is one array of TC_CONTRACT_NOALLOC_SCRATCH_BYTES
  * compiled into the library, held on every GPU that loads the library until
- * exit.  Shapes whose tcTensorContractScratch(...) exceeds that size are
+ * exit.  Shapes whose offset tables exceed that size are
  * rejected with TALSH_LIMIT_EXCEEDED (tcLastErrorString says why).  The first
  * call on a device looks up the array's device address, so make that first
  * call before any stream capture; the address is kept for the life of the
