@@ -1233,9 +1233,14 @@ struct KSplit {
 constexpr int kSplitMinK = 256;
 KSplit k_split(int kind, int64_t M, int64_t N, int64_t K, int64_t H) {
   KSplit s;
+  // Shapes past 2^31 reach this only through the scratch queries (the launch
+  // refuses them): K first, then each factor of the tile count, so that neither
+  // the chunk nor the product leaves its type.
+  if (K > 0x7fffffffLL) return s;
+  const int64_t most = K / kSplitMinK, many = 8 * 148;
+  if (most < 2 || (M + 63) / 64 >= many || (N + 63) / 64 >= many || H >= many) return s;
   const int64_t tiles = ((M + 63) / 64) * ((N + 63) / 64) * std::max<int64_t>(H, 1);
-  const int64_t most = K / kSplitMinK;
-  if (most < 2 || tiles >= 8 * 148) return s;
+  if (tiles >= many) return s;
   int64_t want = std::min((kind == C8 ? 2 : kind == R4 ? 6 : 4) * 148 / tiles, most);
   if (tiles >= 148) {
     // Every SM has a tile, but not the same number of them: cut K when that

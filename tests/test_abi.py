@@ -751,3 +751,30 @@ def test_slice_views_without_gpu(built):
             assert x.destruct() == 0
     finally:
         assert L.talshShutdown() == 0
+
+
+def test_contraction_scratch_queries_past_32_bits(built):
+    """Shape queries answer for extents no launch takes: contracted ranges past 2^31 (a chunk of a split range would
+    leave 32 bits) and tile counts past 2^63 ask for the offset tables alone; at 2^31 - 1 the query still splits."""
+    L = T.lib()
+
+    def query(ks, ms=(40,), ns=(40,), hs=()):
+        """Bytes for D(m.., h.., n..) += L(k.., m.., h..) R(k.., n.., h..), and the offset tables alone."""
+        nk, nm, nh, nn = len(ks), len(ms), len(hs), len(ns)
+        con = [-(i + 1) for i in range(nk)]
+        cptrn = con + list(range(1, nm + nh + 1)) + con + list(range(nm + nh + 1, nm + nh + nn + 1)) + \
+            list(range(nm + 1, nm + nh + 1))
+        dims = [list(x) for x in (ms + hs + ns, ks + ms + hs, ks + ns + hs)]
+        need = L.tcTensorContractScratch(T.R8, T.ivec(cptrn), len(dims[0]), T.ivec(dims[0]), len(dims[1]),
+                                         T.ivec(dims[1]), len(dims[2]), T.ivec(dims[2]))
+        table = 16 * (np.prod(ms, dtype=object) + np.prod(ns, dtype=object) + np.prod(ks, dtype=object)) + \
+            (24 * np.prod(hs, dtype=object) if hs else 0)
+        return need, (table + 255) // 256 * 256
+
+    for ks, ms, ns, hs in [((592 << 10, 1 << 22), (40,), (40,), ()), ((1 << 17, 1 << 16), (1280,), (1024,), ()),
+                           ((1 << 17, 1 << 17), (1 << 13,), (64,), ()), ((1 << 31 >> 1, 2), (40,), (40,), ()),
+                           ((1024,), (1 << 16, 1 << 12), (1 << 16, 1 << 12), (1 << 16, 1 << 12))]:
+        need, table = query(ks, ms, ns, hs)
+        assert need == table, (ks, ms, ns, hs)
+    need, table = query((2147483647,))
+    assert need > table
