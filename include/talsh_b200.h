@@ -94,8 +94,10 @@ int tcTensorNorm1(int data_kind, size_t vol, const void *src, double *result_dev
 /* Bytes of device scratch tcTensorContract uses for this shape: the offset
  * tables (16 bytes per value of each index group) and, where a long contracted
  * range is split over CTAs, the partial sums.  A call given less, but at least
- * the tables, or a scratch that is not 16-byte aligned, runs unsplit (another
- * summation order); below the tables it is refused. */
+ * the tables, or a scratch that is not 16-byte aligned, computes the same sums
+ * on one CTA per output tile: the same bits, slower (a full contraction of two
+ * tensors with an unaligned scratch sums in another order); below the tables it
+ * is refused. */
 size_t tcTensorContractScratch(int data_kind, const int *cptrn, int drank, const int *ddims,
                                int lrank, const int *ldims, int rrank, const int *rdims);
 
@@ -224,7 +226,8 @@ typedef struct {
 
 /* Bytes of device scratch tcTensorContractBatch uses for these tasks (0 when
  * a task is invalid).  With less, as long as it holds all but the partial sums
- * of split contracted ranges, the batch runs unsplit; below that it is refused. */
+ * of split contracted ranges, the batch runs one CTA per output tile (the same
+ * bits); below that it is refused. */
 size_t tcTensorContractBatchScratch(int ntasks, const tcContractTask *tasks);
 
 /* Runs every task with tcTensorContract's semantics.  The tasks' offset

@@ -53,7 +53,7 @@ double cmplx8_to_real8(double re, double im);
 
 // Scratch of one tcTensorContract call: the size that lets it split a long
 // contracted range over CTAs, and in *least (may be null) the size below which
-// the call is refused.
+// the call is refused.  The result's bits do not depend on which it gets.
 size_t contract_scratch_bytes(int kind, const int *cptrn, int drank, const int *ddims, int lrank,
                               const int *ldims, int rrank, const int *rdims, size_t *least);
 

@@ -117,7 +117,8 @@ struct GemmArgs {
   int b_along_n;  // B tile loads: lanes along n (else along k)
   int conj_l, conj_r;
   // Split contracted range (nsplit > 1): CTA (tile, s) sums k in
-  // [s kchunk, (s+1) kchunk) and the partial tiles meet in `part`.
+  // [s kchunk, (s+1) kchunk) and the partial tiles meet in `part`; without room
+  // for them (part null) the CTA of a tile walks the splits itself (SeqSum).
   int nsplit, kchunk, gsz;
   int ncnt;   // arrival counters of this contraction (zeroed by the table kernel)
   void *part;
@@ -207,6 +208,27 @@ __device__ __forceinline__ bool split_combine(V (&acc)[NF], uint32_t mask, int p
   gather(0, ng, a.gsz);
   return true;
 }
+
+// The sum of split_combine where there is no room for partial tiles: one CTA
+// walks the splits in order and keeps the running group sum and the total, so
+// a short scratch costs time and changes no bit.
+template <int NF, typename V>
+struct SeqSum {
+  V group[NF], total[NF];
+  __device__ __forceinline__ void add(const V (&acc)[NF], const GemmArgs &a, int s) {
+    const int i = s % a.gsz;
+    const bool closes = i == a.gsz - 1 || s == a.nsplit - 1;
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      if (i == 0) group[f] = acc[f];
+      else vadd(group[f], acc[f]);
+      if (closes) {
+        if (s < a.gsz) total[f] = group[f];
+        else vadd(total[f], group[f]);
+      }
+    }
+  }
+};
 
 // ---------------------------------------------------------------- R8: DMMA
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
@@ -389,7 +411,7 @@ struct Side {
 // B's after the third): issued in one block after the barrier they left the
 // pipe idle in every warp at once.  Rows and columns beyond the tensor are neither loaded (their stale
 // shared values only reach outputs that are not stored) nor multiplied.
-template <int BM, int BN>
+template <int BM, int BN, bool SEQ>
 __device__ __forceinline__ void dmma_tile(const double *__restrict__ L, const double *__restrict__ R,
                                           double *D, const GemmArgs &a, const TileWork &w,
                                           unsigned char *smem) {
@@ -407,9 +429,6 @@ __device__ __forceinline__ void dmma_tile(const double *__restrict__ L, const do
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int m0 = w.tm * BM, n0 = w.tn * BN;
   const int mrem = a.M - m0, nrem = a.N - n0;
-  const int k0 = a.nsplit > 1 ? w.split * a.kchunk : 0;
-  const int K = a.nsplit > 1 ? min(a.kchunk, a.K - k0) : a.K;
-  const int64_t *kLg = a.kL + k0, *kRg = a.kR + k0;
   for (int i = tid; i < BM; i += NT) {
     const int m = m0 + i;
     mLs[i] = m < a.M ? a.mL[m] : 0;
@@ -420,85 +439,95 @@ __device__ __forceinline__ void dmma_tile(const double *__restrict__ L, const do
     nRs[i] = n < a.N ? a.nR[n] : 0;
     nDs[i] = n < a.N ? a.nD[n] : 0;
   }
-  kring_init<BK, ST>(kLg, kRg, K, kLs, kRs, tid, NT);
-  __syncthreads();
-
-  const int numK = (K + BK - 1) / BK;
-  // Portion Q of P of the loads of k-tile kt into stage s.
-  Side<BM, BK, NT, AP, 8, true> sa;
-  Side<BN, BK, NT, BP, 8, true> sb;
-  sa.init(L, mLs, As, a.a_along_m, mrem);
-  sb.init(R, nRs, Bs, a.b_along_n, nrem);
-  constexpr uint32_t SAB = BK * AP * 8, SBB = BK * BP * 8;  // bytes per stage
-  KRing<BK, ST> ring;
-  ring.init(kLg, kRg, kLs, kRs);
-  const uint32_t ksa = (uint32_t)__cvta_generic_to_shared(kLs), ksb = (uint32_t)__cvta_generic_to_shared(kRs);
-  auto load_a = [&](int kt, int s) { sa.load_tile(s * SAB, ksa + (kt % kKRing) * (BK * 8), K - kt * BK); };
-  auto load_b = [&](int kt, int s) { sb.load_tile(s * SBB, ksb + (kt % kKRing) * (BK * 8), K - kt * BK); };
   using Int0 = std::integral_constant<int, 0>;
   using Int1 = std::integral_constant<int, 1>;
   using Int2 = std::integral_constant<int, 2>;
   using Int3 = std::integral_constant<int, 3>;
-
   constexpr int FM = C::WM / 8, FN = C::WN / 8;
   double2 acc[FM * FN];
-#pragma unroll
-  for (int f = 0; f < FM * FN; ++f) acc[f] = make_double2(0.0, 0.0);
-
   // Ragged tiles give the low warp positions more fragments; rotating the
   // positions by CTA spreads them over the SM's four tensor pipes.
   const int wr = (warp + w.lin + w.split) % (C::WARPS_M * C::WARPS_N);
   const int wm = wr % C::WARPS_M, wn = wr / C::WARPS_M;
   const int fr = lane >> 2, fc = lane & 3;
   const int fm = frag_count(mrem, wm, C::WARPS_M, FM), fn = frag_count(nrem, wn, C::WARPS_N, FN);
+  SeqSum<FM * FN, double2> seq;
+  for (int split = SEQ ? 0 : w.split;; ++split) {
+    const int k0 = a.nsplit > 1 ? split * a.kchunk : 0;
+    const int K = a.nsplit > 1 ? min(a.kchunk, a.K - k0) : a.K;
+    const int64_t *kLg = a.kL + k0, *kRg = a.kR + k0;
+#pragma unroll
+    for (int f = 0; f < FM * FN; ++f) acc[f] = make_double2(0.0, 0.0);
+    kring_init<BK, ST>(kLg, kRg, K, kLs, kRs, tid, NT);
+    __syncthreads();
 
+    const int numK = (K + BK - 1) / BK;
+    Side<BM, BK, NT, AP, 8, true> sa;
+    Side<BN, BK, NT, BP, 8, true> sb;
+    sa.init(L, mLs, As, a.a_along_m, mrem);
+    sb.init(R, nRs, Bs, a.b_along_n, nrem);
+    constexpr uint32_t SAB = BK * AP * 8, SBB = BK * BP * 8;  // bytes per stage
+    KRing<BK, ST> ring;
+    ring.init(kLg, kRg, kLs, kRs);
+    const uint32_t ksa = (uint32_t)__cvta_generic_to_shared(kLs), ksb = (uint32_t)__cvta_generic_to_shared(kRs);
+    auto load_a = [&](int kt, int s) { sa.load_tile(s * SAB, ksa + (kt % kKRing) * (BK * 8), K - kt * BK); };
+    auto load_b = [&](int kt, int s) { sb.load_tile(s * SBB, ksb + (kt % kKRing) * (BK * 8), K - kt * BK); };
 #pragma unroll
-  for (int s = 0; s < ST - 1; ++s) {
-    load_a(s, s);
-    load_b(s, s);
-    cp_async_commit();
-  }
-  auto main_loop = [&](auto full_c) {
-    constexpr bool FULL = decltype(full_c)::value;
-    int st = 0, ps = ST - 1;  // stage of tile kt, stage filled during iteration kt
-    for (int kt = 0; kt < numK; ++kt) {
-      cp_async_wait<ST - 2>();
-      __syncthreads();
-      const double *as = As + (st * BK + fc) * AP + wm * 8;
-      const double *bs = Bs + (st * BK + fc) * BP + wn * 8;
-      auto step = [&](auto ksc) {
-        constexpr int ks = decltype(ksc)::value;
-        double af[FM], bf[FN];
-        const double *ap = as + (fr ^ ks), *bp = bs + (fr ^ ks);  // kswz(4 ks + fc) = ks
-#pragma unroll
-        for (int i = 0; i < FM; ++i) af[i] = ap[ks * 4 * AP + i * C::WARPS_M * 8];
-#pragma unroll
-        for (int j = 0; j < FN; ++j) bf[j] = bp[ks * 4 * BP + j * C::WARPS_N * 8];
-#pragma unroll
-        for (int i = 0; i < FM; ++i) {
-          if (!FULL && i >= fm) break;
-#pragma unroll
-          for (int j = 0; j < FN; ++j)
-            if (FULL || j < fn) dmma_8x8x4(acc[i * FN + j].x, acc[i * FN + j].y, af[i], bf[j]);
-        }
-        if constexpr (ks == 0) load_a(kt + ST - 1, ps);
-        if constexpr (ks == 2) load_b(kt + ST - 1, ps);
-      };
-      step(Int0{});
-      step(Int1{});
-      step(Int2{});
-      step(Int3{});
-      ring.step(kt, K);
+    for (int s = 0; s < ST - 1; ++s) {
+      load_a(s, s);
+      load_b(s, s);
       cp_async_commit();
-      ps = st;
-      st = st + 1 == ST ? 0 : st + 1;
     }
-  };
-  if (fm == FM && fn == FN) main_loop(std::true_type{});
-  else main_loop(std::false_type{});
-  cp_async_wait<0>();
+    auto main_loop = [&](auto full_c) {
+      constexpr bool FULL = decltype(full_c)::value;
+      int st = 0, ps = ST - 1;  // stage of tile kt, stage filled during iteration kt
+      for (int kt = 0; kt < numK; ++kt) {
+        cp_async_wait<ST - 2>();
+        __syncthreads();
+        const double *as = As + (st * BK + fc) * AP + wm * 8;
+        const double *bs = Bs + (st * BK + fc) * BP + wn * 8;
+        auto step = [&](auto ksc) {
+          constexpr int ks = decltype(ksc)::value;
+          double af[FM], bf[FN];
+          const double *ap = as + (fr ^ ks), *bp = bs + (fr ^ ks);  // kswz(4 ks + fc) = ks
+#pragma unroll
+          for (int i = 0; i < FM; ++i) af[i] = ap[ks * 4 * AP + i * C::WARPS_M * 8];
+#pragma unroll
+          for (int j = 0; j < FN; ++j) bf[j] = bp[ks * 4 * BP + j * C::WARPS_N * 8];
+#pragma unroll
+          for (int i = 0; i < FM; ++i) {
+            if (!FULL && i >= fm) break;
+#pragma unroll
+            for (int j = 0; j < FN; ++j)
+              if (FULL || j < fn) dmma_8x8x4(acc[i * FN + j].x, acc[i * FN + j].y, af[i], bf[j]);
+          }
+          if constexpr (ks == 0) load_a(kt + ST - 1, ps);
+          if constexpr (ks == 2) load_b(kt + ST - 1, ps);
+        };
+        step(Int0{});
+        step(Int1{});
+        step(Int2{});
+        step(Int3{});
+        ring.step(kt, K);
+        cp_async_commit();
+        ps = st;
+        st = st + 1 == ST ? 0 : st + 1;
+      }
+    };
+    if (fm == FM && fn == FN) main_loop(std::true_type{});
+    else main_loop(std::false_type{});
+    cp_async_wait<0>();
+    if constexpr (!SEQ) break;
+    seq.add(acc, a, split);
+    if (split + 1 == a.nsplit) break;
+    __syncthreads();  // the next split refills the stages and the offset ring
+  }
 
-  if (a.nsplit > 1) {
+  if constexpr (SEQ) {
+#pragma unroll
+    for (int f = 0; f < FM * FN; ++f) acc[f] = seq.total[f];
+  }
+  if (!SEQ && a.nsplit > 1) {
     uint32_t mask = 0;
 #pragma unroll
     for (int f = 0; f < FM * FN; ++f)
@@ -559,7 +588,7 @@ struct ZmmaCfg {
                                  (size_t)(2 * BM + 2 * BN + 2 * kKRing * BK) * sizeof(int64_t);
 };
 
-template <int BM, int BN>
+template <int BM, int BN, bool SEQ>
 __device__ __forceinline__ void zmma_tile(const double2 *__restrict__ L, const double2 *__restrict__ R,
                                           double2 *D, const GemmArgs &a, const TileWork &w,
                                           unsigned char *smem) {
@@ -576,9 +605,6 @@ __device__ __forceinline__ void zmma_tile(const double2 *__restrict__ L, const d
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int m0 = w.tm * BM, n0 = w.tn * BN;
   const int mrem = a.M - m0, nrem = a.N - n0;
-  const int k0 = a.nsplit > 1 ? w.split * a.kchunk : 0;
-  const int K = a.nsplit > 1 ? min(a.kchunk, a.K - k0) : a.K;
-  const int64_t *kLg = a.kL + k0, *kRg = a.kR + k0;
   for (int i = tid; i < BM; i += NT) {
     const int m = m0 + i;
     mLs[i] = m < a.M ? a.mL[m] : 0;
@@ -589,28 +615,12 @@ __device__ __forceinline__ void zmma_tile(const double2 *__restrict__ L, const d
     nRs[i] = n < a.N ? a.nR[n] : 0;
     nDs[i] = n < a.N ? a.nD[n] : 0;
   }
-  kring_init<BK, ST>(kLg, kRg, K, kLs, kRs, tid, NT);
-  __syncthreads();
-  const int numK = (K + BK - 1) / BK;
-  Side<BM, BK, NT, AP, 16, false> sa;
-  Side<BN, BK, NT, BP, 16, false> sb;
-  sa.init(L, mLs, As, a.a_along_m, mrem);
-  sb.init(R, nRs, Bs, a.b_along_n, nrem);
-  constexpr uint32_t SAB = BK * AP * 16, SBB = BK * BP * 16;  // bytes per stage
-  KRing<BK, ST> ring;
-  ring.init(kLg, kRg, kLs, kRs);
-  const uint32_t ksa = (uint32_t)__cvta_generic_to_shared(kLs), ksb = (uint32_t)__cvta_generic_to_shared(kRs);
-  auto load_a = [&](int kt, int s) { sa.load_tile(s * SAB, ksa + (kt % kKRing) * (BK * 8), K - kt * BK); };
-  auto load_b = [&](int kt, int s) { sb.load_tile(s * SBB, ksb + (kt % kKRing) * (BK * 8), K - kt * BK); };
   using Int0 = std::integral_constant<int, 0>;
   using Int1 = std::integral_constant<int, 1>;
   using Int2 = std::integral_constant<int, 2>;
   using Int3 = std::integral_constant<int, 3>;
-
   constexpr int FM = C::WM / 8, FN = C::WN / 8;
   double2 acc[2 * FM * FN];  // fragment f: real parts at 2 f, imaginary parts at 2 f + 1
-#pragma unroll
-  for (int f = 0; f < 2 * FM * FN; ++f) acc[f] = make_double2(0.0, 0.0);
   // Ragged tiles give the low warp positions more fragments; rotating the
   // positions by CTA spreads them over the SM's four tensor pipes.
   const int wr = (warp + w.lin + w.split) % (C::WARPS_M * C::WARPS_N);
@@ -620,67 +630,96 @@ __device__ __forceinline__ void zmma_tile(const double2 *__restrict__ L, const d
   // conjugation flips the sign bit of the imaginary part
   const int ml = a.conj_l ? (int)0x80000000 : 0, mr = a.conj_r ? (int)0x80000000 : 0;
   auto flip = [](double x, int m) { return __hiloint2double(__double2hiint(x) ^ m, __double2loint(x)); };
+  SeqSum<2 * FM * FN, double2> seq;
+  for (int split = SEQ ? 0 : w.split;; ++split) {
+    const int k0 = a.nsplit > 1 ? split * a.kchunk : 0;
+    const int K = a.nsplit > 1 ? min(a.kchunk, a.K - k0) : a.K;
+    const int64_t *kLg = a.kL + k0, *kRg = a.kR + k0;
 #pragma unroll
-  for (int s = 0; s < ST - 1; ++s) {
-    load_a(s, s);
-    load_b(s, s);
-    cp_async_commit();
-  }
-  auto main_loop = [&](auto full_c) {
-    constexpr bool FULL = decltype(full_c)::value;
-    int st = 0, ps = ST - 1;
-    for (int kt = 0; kt < numK; ++kt) {
-      cp_async_wait<ST - 2>();
-      __syncthreads();
-      const double2 *as = As + (st * BK + fc) * AP + wm * 8 + fr;
-      const double2 *bs = Bs + (st * BK + fc) * BP + wn * 8 + fr;
-      auto step = [&](auto ksc) {
-        constexpr int ks = decltype(ksc)::value;
-        double ar[FM], ai[FM], br[FN], bi[FN], nbi[FN];
+    for (int f = 0; f < 2 * FM * FN; ++f) acc[f] = make_double2(0.0, 0.0);
+    kring_init<BK, ST>(kLg, kRg, K, kLs, kRs, tid, NT);
+    __syncthreads();
+    const int numK = (K + BK - 1) / BK;
+    Side<BM, BK, NT, AP, 16, false> sa;
+    Side<BN, BK, NT, BP, 16, false> sb;
+    sa.init(L, mLs, As, a.a_along_m, mrem);
+    sb.init(R, nRs, Bs, a.b_along_n, nrem);
+    constexpr uint32_t SAB = BK * AP * 16, SBB = BK * BP * 16;  // bytes per stage
+    KRing<BK, ST> ring;
+    ring.init(kLg, kRg, kLs, kRs);
+    const uint32_t ksa = (uint32_t)__cvta_generic_to_shared(kLs), ksb = (uint32_t)__cvta_generic_to_shared(kRs);
+    auto load_a = [&](int kt, int s) { sa.load_tile(s * SAB, ksa + (kt % kKRing) * (BK * 8), K - kt * BK); };
+    auto load_b = [&](int kt, int s) { sb.load_tile(s * SBB, ksb + (kt % kKRing) * (BK * 8), K - kt * BK); };
 #pragma unroll
-        for (int i = 0; i < FM; ++i) {
-          const double2 v = as[ks * 4 * AP + i * C::WARPS_M * 8];
-          ar[i] = v.x;
-          ai[i] = flip(v.y, ml);
-        }
+    for (int s = 0; s < ST - 1; ++s) {
+      load_a(s, s);
+      load_b(s, s);
+      cp_async_commit();
+    }
+    auto main_loop = [&](auto full_c) {
+      constexpr bool FULL = decltype(full_c)::value;
+      int st = 0, ps = ST - 1;
+      for (int kt = 0; kt < numK; ++kt) {
+        cp_async_wait<ST - 2>();
+        __syncthreads();
+        const double2 *as = As + (st * BK + fc) * AP + wm * 8 + fr;
+        const double2 *bs = Bs + (st * BK + fc) * BP + wn * 8 + fr;
+        auto step = [&](auto ksc) {
+          constexpr int ks = decltype(ksc)::value;
+          double ar[FM], ai[FM], br[FN], bi[FN], nbi[FN];
 #pragma unroll
-        for (int j = 0; j < FN; ++j) {
-          const double2 v = bs[ks * 4 * BP + j * C::WARPS_N * 8];
-          br[j] = v.x;
-          bi[j] = flip(v.y, mr);
-          nbi[j] = -bi[j];
-        }
-#pragma unroll
-        for (int i = 0; i < FM; ++i) {
+          for (int i = 0; i < FM; ++i) {
+            const double2 v = as[ks * 4 * AP + i * C::WARPS_M * 8];
+            ar[i] = v.x;
+            ai[i] = flip(v.y, ml);
+          }
 #pragma unroll
           for (int j = 0; j < FN; ++j) {
-            double2 &cr = acc[2 * (i * FN + j)], &ci = acc[2 * (i * FN + j) + 1];
+            const double2 v = bs[ks * 4 * BP + j * C::WARPS_N * 8];
+            br[j] = v.x;
+            bi[j] = flip(v.y, mr);
+            nbi[j] = -bi[j];
+          }
+#pragma unroll
+          for (int i = 0; i < FM; ++i) {
+#pragma unroll
+            for (int j = 0; j < FN; ++j) {
+              double2 &cr = acc[2 * (i * FN + j)], &ci = acc[2 * (i * FN + j) + 1];
 #pragma unroll 1
-            for (int x = FULL ? 1 : one_if(i < fm && j < fn); x > 0; --x) {
-              dmma_8x8x4(cr.x, cr.y, ar[i], br[j]);
-              dmma_8x8x4(cr.x, cr.y, ai[i], nbi[j]);
-              dmma_8x8x4(ci.x, ci.y, ar[i], bi[j]);
-              dmma_8x8x4(ci.x, ci.y, ai[i], br[j]);
+              for (int x = FULL ? 1 : one_if(i < fm && j < fn); x > 0; --x) {
+                dmma_8x8x4(cr.x, cr.y, ar[i], br[j]);
+                dmma_8x8x4(cr.x, cr.y, ai[i], nbi[j]);
+                dmma_8x8x4(ci.x, ci.y, ar[i], bi[j]);
+                dmma_8x8x4(ci.x, ci.y, ai[i], br[j]);
+              }
             }
           }
-        }
-        if constexpr (ks == 0) load_a(kt + ST - 1, ps);
-        if constexpr (ks == 2) load_b(kt + ST - 1, ps);
-      };
-      step(Int0{});
-      step(Int1{});
-      step(Int2{});
-      step(Int3{});
-      ring.step(kt, K);
-      cp_async_commit();
-      ps = st;
-      st = st + 1 == ST ? 0 : st + 1;
-    }
-  };
-  if (fm == FM && fn == FN) main_loop(std::true_type{});
-  else main_loop(std::false_type{});
-  cp_async_wait<0>();
-  if (a.nsplit > 1) {
+          if constexpr (ks == 0) load_a(kt + ST - 1, ps);
+          if constexpr (ks == 2) load_b(kt + ST - 1, ps);
+        };
+        step(Int0{});
+        step(Int1{});
+        step(Int2{});
+        step(Int3{});
+        ring.step(kt, K);
+        cp_async_commit();
+        ps = st;
+        st = st + 1 == ST ? 0 : st + 1;
+      }
+    };
+    if (fm == FM && fn == FN) main_loop(std::true_type{});
+    else main_loop(std::false_type{});
+    cp_async_wait<0>();
+    if constexpr (!SEQ) break;
+    seq.add(acc, a, split);
+    if (split + 1 == a.nsplit) break;
+    __syncthreads();
+  }
+  if constexpr (SEQ) {
+#pragma unroll
+    for (int f = 0; f < 2 * FM * FN; ++f) acc[f] = seq.total[f];
+  }
+  if (!SEQ && a.nsplit > 1) {
     uint32_t mask = 0;
 #pragma unroll
     for (int f = 0; f < FM * FN; ++f)
@@ -716,26 +755,26 @@ template <int BM, int BN> struct GemmOcc { static constexpr int D = 1, Z = 1; };
 template <> struct GemmOcc<64, 64> { static constexpr int D = 4, Z = 2; };
 template <> struct GemmOcc<32, 32> { static constexpr int D = 6, Z = 5; };
 
-template <int BM, int BN>
-__global__ void __launch_bounds__(ZmmaCfg<BM, BN>::THREADS, GemmOcc<BM, BN>::Z)
+template <int BM, int BN, bool SEQ>
+__global__ void __launch_bounds__(ZmmaCfg<BM, BN>::THREADS, SEQ ? 1 : GemmOcc<BM, BN>::Z)
     zgemm_gather_kernel(const double2 *__restrict__ L, const double2 *__restrict__ R, double2 *D,
                         const GemmArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const double2 *Lp = L, *Rp = R;
   double2 *Dp = D;
   const TileWork w = block_work(a, Lp, Rp, Dp);
-  zmma_tile<BM, BN>(Lp, Rp, Dp, a, w, smem);
+  zmma_tile<BM, BN, SEQ>(Lp, Rp, Dp, a, w, smem);
 }
 
-template <int BM, int BN>
-__global__ void __launch_bounds__(DmmaCfg<BM, BN>::THREADS, GemmOcc<BM, BN>::D)
+template <int BM, int BN, bool SEQ>
+__global__ void __launch_bounds__(DmmaCfg<BM, BN>::THREADS, SEQ ? 1 : GemmOcc<BM, BN>::D)
     dgemm_gather_kernel(const double *__restrict__ L, const double *__restrict__ R, double *D,
                         const GemmArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const double *Lp = L, *Rp = R;
   double *Dp = D;
   const TileWork w = block_work(a, Lp, Rp, Dp);
-  dmma_tile<BM, BN>(Lp, Rp, Dp, a, w, smem);
+  dmma_tile<BM, BN, SEQ>(Lp, Rp, Dp, a, w, smem);
 }
 
 // ------------------------------------------------- R4 / C4: packed FP32 FMA
@@ -772,7 +811,7 @@ struct FmmaCfg {
                                  (size_t)(2 * BM + 2 * BN + 2 * kKRing * BK) * sizeof(int64_t);
 };
 
-template <typename T, int BM, int BN>
+template <typename T, int BM, int BN, bool SEQ>
 __device__ __forceinline__ void fmma_tile(const T *__restrict__ L, const T *__restrict__ R, T *D, const GemmArgs &a,
                                           const TileWork &w, unsigned char *smem) {
   using C = FmmaCfg<T, BM, BN>;
@@ -790,9 +829,6 @@ __device__ __forceinline__ void fmma_tile(const T *__restrict__ L, const T *__re
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int m0 = w.tm * BM, n0 = w.tn * BN;
   const int mrem = a.M - m0, nrem = a.N - n0;
-  const int k0 = a.nsplit > 1 ? w.split * a.kchunk : 0;
-  const int K = a.nsplit > 1 ? min(a.kchunk, a.K - k0) : a.K;
-  const int64_t *kLg = a.kL + k0, *kRg = a.kR + k0;
   for (int i = tid; i < BM; i += NT) {
     const int m = m0 + i;
     mLs[i] = m < a.M ? a.mL[m] : 0;
@@ -803,20 +839,6 @@ __device__ __forceinline__ void fmma_tile(const T *__restrict__ L, const T *__re
     nRs[i] = n < a.N ? a.nR[n] : 0;
     nDs[i] = n < a.N ? a.nD[n] : 0;
   }
-  kring_init<BK, ST>(kLg, kRg, K, kLs, kRs, tid, NT);
-  __syncthreads();
-  const int numK = (K + BK - 1) / BK;
-  Side<BM, BK, NT, AP, ES, false> sa;
-  Side<BN, BK, NT, BP, ES, false> sb;
-  sa.init(L, mLs, As, a.a_along_m, mrem);
-  sb.init(R, nRs, Bs, a.b_along_n, nrem);
-  constexpr uint32_t SAB = BK * AP * ES, SBB = BK * BP * ES;
-  KRing<BK, ST> ring;
-  ring.init(kLg, kRg, kLs, kRs);
-  const uint32_t ksa = (uint32_t)__cvta_generic_to_shared(kLs), ksb = (uint32_t)__cvta_generic_to_shared(kRs);
-  auto load_a = [&](int kt, int s) { sa.load_tile(s * SAB, ksa + (kt % kKRing) * (BK * 8), K - kt * BK); };
-  auto load_b = [&](int kt, int s) { sb.load_tile(s * SBB, ksb + (kt % kKRing) * (BK * 8), K - kt * BK); };
-
   const int tm = (lane & 3) + 4 * (warp % (C::TMN / 4)), tn = (lane >> 2) + 8 * (warp / (C::TMN / 4));
   // Accumulator pairs.  Complex: acc[i][j] is element (i, j), (re, im).  Real:
   // a pair of rows meets a pair of columns as they come from shared memory, and
@@ -826,114 +848,148 @@ __device__ __forceinline__ void fmma_tile(const T *__restrict__ L, const T *__re
   // cost two moves per row.
   constexpr int NP = CPLX ? TN : TN / 2;
   uint64_t acc[TM][NP];
-#pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < NP; ++j) acc[i][j] = 0;
   const uint32_t cl = a.conj_l ? 0x80000000u : 0u, cr = a.conj_r ? 0x80000000u : 0u;
+  constexpr int NF = TM * NP / 2;  // 16-byte units: two accumulator pairs of a row
+  auto to_units = [&](float4(&u)[NF]) {
 #pragma unroll
-  for (int s = 0; s < ST - 1; ++s) {
-    load_a(s, s);
-    load_b(s, s);
-    cp_async_commit();
-  }
-  int st = 0, ps = ST - 1;
-  for (int kt = 0; kt < numK; ++kt) {
-    cp_async_wait<ST - 2>();
+    for (int f = 0; f < NF; ++f) {
+      const int i = f / (NP / 2), j = f % (NP / 2);
+      const float2 x = unpack2(acc[i][2 * j]), y = unpack2(acc[i][2 * j + 1]);
+      u[f] = make_float4(x.x, x.y, y.x, y.y);
+    }
+  };
+  auto from_units = [&](const float4(&u)[NF]) {
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      const int i = f / (NP / 2), j = f % (NP / 2);
+      acc[i][2 * j] = pack2(u[f].x, u[f].y);
+      acc[i][2 * j + 1] = pack2(u[f].z, u[f].w);
+    }
+  };
+  SeqSum<NF, float4> seq;
+  for (int split = SEQ ? 0 : w.split;; ++split) {
+    const int k0 = a.nsplit > 1 ? split * a.kchunk : 0;
+    const int K = a.nsplit > 1 ? min(a.kchunk, a.K - k0) : a.K;
+    const int64_t *kLg = a.kL + k0, *kRg = a.kR + k0;
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < NP; ++j) acc[i][j] = 0;
+    kring_init<BK, ST>(kLg, kRg, K, kLs, kRs, tid, NT);
     __syncthreads();
-    const T *as = As + st * BK * AP + tm * VE;
-    const T *bs = Bs + st * BK * BP + tn * VE;
+    const int numK = (K + BK - 1) / BK;
+    Side<BM, BK, NT, AP, ES, false> sa;
+    Side<BN, BK, NT, BP, ES, false> sb;
+    sa.init(L, mLs, As, a.a_along_m, mrem);
+    sb.init(R, nRs, Bs, a.b_along_n, nrem);
+    constexpr uint32_t SAB = BK * AP * ES, SBB = BK * BP * ES;
+    KRing<BK, ST> ring;
+    ring.init(kLg, kRg, kLs, kRs);
+    const uint32_t ksa = (uint32_t)__cvta_generic_to_shared(kLs), ksb = (uint32_t)__cvta_generic_to_shared(kRs);
+    auto load_a = [&](int kt, int s) { sa.load_tile(s * SAB, ksa + (kt % kKRing) * (BK * 8), K - kt * BK); };
+    auto load_b = [&](int kt, int s) { sb.load_tile(s * SBB, ksb + (kt % kKRing) * (BK * 8), K - kt * BK); };
 #pragma unroll
-    for (int k = 0; k < BK; ++k) {
-      uint64_t av[C::MC * 2], bv[C::NC * 2];
+    for (int s = 0; s < ST - 1; ++s) {
+      load_a(s, s);
+      load_b(s, s);
+      cp_async_commit();
+    }
+    int st = 0, ps = ST - 1;
+    for (int kt = 0; kt < numK; ++kt) {
+      cp_async_wait<ST - 2>();
+      __syncthreads();
+      const T *as = As + st * BK * AP + tm * VE;
+      const T *bs = Bs + st * BK * BP + tn * VE;
 #pragma unroll
-      for (int c = 0; c < C::MC; ++c) {
-        const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(as + k * AP + c * (C::TMN * VE));
-        av[2 * c] = v.x;
-        av[2 * c + 1] = v.y;
-      }
+      for (int k = 0; k < BK; ++k) {
+        uint64_t av[C::MC * 2], bv[C::NC * 2];
 #pragma unroll
-      for (int c = 0; c < C::NC; ++c) {
-        const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(bs + k * BP + c * (C::TNN * VE));
-        bv[2 * c] = v.x;
-        bv[2 * c + 1] = v.y;
-      }
-      if constexpr (CPLX) {
-        // (re, im) += x.re (y.re, y.im), then += x.im (-y.im, y.re)
-        uint64_t by[TN], bx[TN];
-#pragma unroll
-        for (int j = 0; j < TN; ++j) {
-          const float2 y = unpack2(bv[j]);
-          const float yi = __uint_as_float(__float_as_uint(y.y) ^ cr);
-          by[j] = pack2(y.x, yi);
-          bx[j] = pack2(-yi, y.x);
+        for (int c = 0; c < C::MC; ++c) {
+          const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(as + k * AP + c * (C::TMN * VE));
+          av[2 * c] = v.x;
+          av[2 * c + 1] = v.y;
         }
 #pragma unroll
-        for (int i = 0; i < TM; ++i) {
-          const float2 x = unpack2(av[i]);
-          const float xi = __uint_as_float(__float_as_uint(x.y) ^ cl);
-          const uint64_t xr2 = pack2(x.x, x.x), xi2 = pack2(xi, xi);
+        for (int c = 0; c < C::NC; ++c) {
+          const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(bs + k * BP + c * (C::TNN * VE));
+          bv[2 * c] = v.x;
+          bv[2 * c + 1] = v.y;
+        }
+        if constexpr (CPLX) {
+          // (re, im) += x.re (y.re, y.im), then += x.im (-y.im, y.re)
+          uint64_t by[TN], bx[TN];
 #pragma unroll
           for (int j = 0; j < TN; ++j) {
-            ffma2(acc[i][j], xr2, by[j]);
-            ffma2(acc[i][j], xi2, bx[j]);
+            const float2 y = unpack2(bv[j]);
+            const float yi = __uint_as_float(__float_as_uint(y.y) ^ cr);
+            by[j] = pack2(y.x, yi);
+            bx[j] = pack2(-yi, y.x);
           }
-        }
-      } else {
-        uint64_t bs2[NP];
 #pragma unroll
-        for (int j = 0; j < NP; ++j) {
-          const float2 y = unpack2(bv[j]);
-          bs2[j] = pack2(y.y, y.x);
-        }
+          for (int i = 0; i < TM; ++i) {
+            const float2 x = unpack2(av[i]);
+            const float xi = __uint_as_float(__float_as_uint(x.y) ^ cl);
+            const uint64_t xr2 = pack2(x.x, x.x), xi2 = pack2(xi, xi);
 #pragma unroll
-        for (int i = 0; i < TM; i += 2)
+            for (int j = 0; j < TN; ++j) {
+              ffma2(acc[i][j], xr2, by[j]);
+              ffma2(acc[i][j], xi2, bx[j]);
+            }
+          }
+        } else {
+          uint64_t bs2[NP];
 #pragma unroll
           for (int j = 0; j < NP; ++j) {
-            ffma2(acc[i][j], av[i / 2], bv[j]);
-            ffma2(acc[i + 1][j], av[i / 2], bs2[j]);
+            const float2 y = unpack2(bv[j]);
+            bs2[j] = pack2(y.y, y.x);
           }
+#pragma unroll
+          for (int i = 0; i < TM; i += 2)
+#pragma unroll
+            for (int j = 0; j < NP; ++j) {
+              ffma2(acc[i][j], av[i / 2], bv[j]);
+              ffma2(acc[i + 1][j], av[i / 2], bs2[j]);
+            }
+        }
+        if (k == 1) load_a(kt + ST - 1, ps);
+        if (k == BK / 2 + 1) load_b(kt + ST - 1, ps);
       }
-      if (k == 1) load_a(kt + ST - 1, ps);
-      if (k == BK / 2 + 1) load_b(kt + ST - 1, ps);
+      ring.step(kt, K);
+      cp_async_commit();
+      ps = st;
+      st = st + 1 == ST ? 0 : st + 1;
     }
-    ring.step(kt, K);
-    cp_async_commit();
-    ps = st;
-    st = st + 1 == ST ? 0 : st + 1;
-  }
-  cp_async_wait<0>();
+    cp_async_wait<0>();
 
-  if constexpr (!CPLX) {  // back to rows: acc[i][j/2] = (c(i,j), c(i,j+1))
+    if constexpr (!CPLX) {  // back to rows: acc[i][j/2] = (c(i,j), c(i,j+1))
 #pragma unroll
-    for (int i = 0; i < TM; i += 2)
+      for (int i = 0; i < TM; i += 2)
 #pragma unroll
-      for (int j = 0; j < NP; ++j) {
-        const float2 d = unpack2(acc[i][j]), x = unpack2(acc[i + 1][j]);
-        acc[i][j] = pack2(d.x, x.x);
-        acc[i + 1][j] = pack2(x.y, d.y);
-      }
+        for (int j = 0; j < NP; ++j) {
+          const float2 d = unpack2(acc[i][j]), x = unpack2(acc[i + 1][j]);
+          acc[i][j] = pack2(d.x, x.x);
+          acc[i + 1][j] = pack2(x.y, d.y);
+        }
+    }
+    if constexpr (!SEQ) break;
+    float4 u[NF];
+    to_units(u);
+    seq.add(u, a, split);
+    if (split + 1 == a.nsplit) break;
+    __syncthreads();
   }
+  if constexpr (SEQ) from_units(seq.total);
   auto row_of = [&](int i) { return (i / VE) * (C::TMN * VE) + tm * VE + i % VE; };
   auto col_of = [&](int j) { return (j / VE) * (C::TNN * VE) + tn * VE + j % VE; };
-  if (a.nsplit > 1) {
-    constexpr int NF = TM * NP / 2;  // 16-byte units: two accumulator pairs of a row
+  if (!SEQ && a.nsplit > 1) {
     float4 part[NF];
     uint32_t mask = 0;
+    to_units(part);
 #pragma unroll
-    for (int f = 0; f < NF; ++f) {
-      const int i = f / (NP / 2), j = f % (NP / 2);
-      const float2 u = unpack2(acc[i][2 * j]), v = unpack2(acc[i][2 * j + 1]);
-      part[f] = make_float4(u.x, u.y, v.x, v.y);
-      if (row_of(i) < mrem && col_of(j * (TN * 2 / NP)) < nrem) mask |= 1u << f;
-    }
+    for (int f = 0; f < NF; ++f)
+      if (row_of(f / (NP / 2)) < mrem && col_of(f % (NP / 2) * (TN * 2 / NP)) < nrem) mask |= 1u << f;
     if (!split_combine<NF, NT>(part, mask, tid, a, w.lin, w.split)) return;
-#pragma unroll
-    for (int f = 0; f < NF; ++f) {
-      const int i = f / (NP / 2), j = f % (NP / 2);
-      acc[i][2 * j] = pack2(part[f].x, part[f].y);
-      acc[i][2 * j + 1] = pack2(part[f].z, part[f].w);
-    }
+    from_units(part);
   }
   const float alr = (float)a.alpha_re, ali = (float)a.alpha_im;
 #pragma unroll
@@ -968,14 +1024,14 @@ template <typename T, int BM> struct FmmaOcc { static constexpr int N = 4; };
 template <> struct FmmaOcc<float, 64> { static constexpr int N = 6; };  // 7: 5 % slower (spills)
 template <> struct FmmaOcc<float, 128> { static constexpr int N = 2; };
 
-template <typename T, int BM, int BN>
-__global__ void __launch_bounds__(FmmaCfg<T, BM, BN>::THREADS, FmmaOcc<T, BM>::N)
+template <typename T, int BM, int BN, bool SEQ>
+__global__ void __launch_bounds__(FmmaCfg<T, BM, BN>::THREADS, SEQ ? 1 : FmmaOcc<T, BM>::N)
     fgemm_gather_kernel(const T *__restrict__ L, const T *__restrict__ R, T *D, const GemmArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const T *Lp = L, *Rp = R;
   T *Dp = D;
   const TileWork w = block_work(a, Lp, Rp, Dp);
-  fmma_tile<T, BM, BN>(Lp, Rp, Dp, a, w, smem);
+  fmma_tile<T, BM, BN, SEQ>(Lp, Rp, Dp, a, w, smem);
 }
 
 // ------------------------------------------------------ full contraction
@@ -1226,7 +1282,7 @@ size_t table_bytes(const TableParams &T) {
 // two), each at least 256 long (16 pipeline steps; 512 makes short ranges up to
 // 15 % slower).  The cut depends on the
 // shape alone, so the same contraction sums in the same order alone and in any
-// batch, whatever tile runs it.
+// batch, whatever tile runs it and whatever scratch it has.
 struct KSplit {
   int nsplit = 1, kchunk = 0, gsz = 1;
 };
@@ -1284,60 +1340,76 @@ int gemm_edge(int kind, int64_t M, int64_t N, int64_t H, const KSplit &s) {
   return tiles(64) * s.nsplit >= sms ? 64 : 32;
 }
 
+// A split contracted range without room for partial tiles.
+bool sequential(const GemmArgs &ga) { return ga.nsplit > 1 && ga.part == nullptr; }
+
 // Grid of a gather-GEMM launch: tiles of one GEMM times hyper combinations
-// times splits.
+// times the splits that run in CTAs of their own.
 int gemm_grid(GemmArgs &ga, int bm, int bn, int64_t *blocks) {
   ga.tiles_m = (ga.M + bm - 1) / bm;
   const int64_t per = (int64_t)ga.tiles_m * ((ga.N + bn - 1) / bn);
-  const int64_t all = per * std::max(ga.H, 1) * std::max(ga.nsplit, 1);
+  const int64_t all = per * std::max(ga.H, 1) * (sequential(ga) ? 1 : std::max(ga.nsplit, 1));
   if (per > 0x7fffffffLL || all > 0x7fffffffLL) return TALSH_LIMIT_EXCEEDED;
   ga.tiles_mn = (int)per;
   *blocks = all;
   return TALSH_SUCCESS;
 }
 
-template <int BM, int BN>
-int launch_dmma(const double *L, const double *R, double *D, GemmArgs ga, cudaStream_t st) {
+template <int BM, int BN, bool SEQ>
+int launch_dmma_as(const double *L, const double *R, double *D, GemmArgs ga, cudaStream_t st) {
   using C = DmmaCfg<BM, BN>;
   static std::atomic<uint64_t> attr_set{0};
   once_per_device(attr_set, [] {
-    cudaFuncSetAttribute(dgemm_gather_kernel<BM, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(dgemm_gather_kernel<BM, BN, SEQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)C::SMEM);
   });
   int64_t tiles = 0;
   if (gemm_grid(ga, BM, BN, &tiles)) return TALSH_LIMIT_EXCEEDED;
-  dgemm_gather_kernel<BM, BN><<<(unsigned)tiles, C::THREADS, C::SMEM, st>>>(L, R, D, ga);
+  dgemm_gather_kernel<BM, BN, SEQ><<<(unsigned)tiles, C::THREADS, C::SMEM, st>>>(L, R, D, ga);
   note_launch();
   return check_launch("dgemm_gather_kernel");
 }
-
 template <int BM, int BN>
-int launch_zmma(const double2 *L, const double2 *R, double2 *D, GemmArgs ga, cudaStream_t st) {
+int launch_dmma(const double *L, const double *R, double *D, const GemmArgs &ga, cudaStream_t st) {
+  return sequential(ga) ? launch_dmma_as<BM, BN, true>(L, R, D, ga, st) : launch_dmma_as<BM, BN, false>(L, R, D, ga, st);
+}
+
+template <int BM, int BN, bool SEQ>
+int launch_zmma_as(const double2 *L, const double2 *R, double2 *D, GemmArgs ga, cudaStream_t st) {
   using Z = ZmmaCfg<BM, BN>;
   static std::atomic<uint64_t> attr_set{0};
   once_per_device(attr_set, [] {
-    cudaFuncSetAttribute(zgemm_gather_kernel<BM, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(zgemm_gather_kernel<BM, BN, SEQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)Z::SMEM);
   });
   int64_t tiles = 0;
   if (gemm_grid(ga, BM, BN, &tiles)) return TALSH_LIMIT_EXCEEDED;
-  zgemm_gather_kernel<BM, BN><<<(unsigned)tiles, Z::THREADS, Z::SMEM, st>>>(L, R, D, ga);
+  zgemm_gather_kernel<BM, BN, SEQ><<<(unsigned)tiles, Z::THREADS, Z::SMEM, st>>>(L, R, D, ga);
   note_launch();
   return check_launch("zgemm_gather_kernel");
 }
+template <int BM, int BN>
+int launch_zmma(const double2 *L, const double2 *R, double2 *D, const GemmArgs &ga, cudaStream_t st) {
+  return sequential(ga) ? launch_zmma_as<BM, BN, true>(L, R, D, ga, st) : launch_zmma_as<BM, BN, false>(L, R, D, ga, st);
+}
 
-template <typename T, int BM, int BN>
-int launch_fmma(const void *L, const void *R, void *D, GemmArgs ga, cudaStream_t st) {
+template <typename T, int BM, int BN, bool SEQ>
+int launch_fmma_as(const void *L, const void *R, void *D, GemmArgs ga, cudaStream_t st) {
   using C = FmmaCfg<T, BM, BN>;
   static std::atomic<uint64_t> attr_set{0};
   once_per_device(attr_set, [] {
-    cudaFuncSetAttribute(fgemm_gather_kernel<T, BM, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+    cudaFuncSetAttribute(fgemm_gather_kernel<T, BM, BN, SEQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
   });
   int64_t tiles = 0;
   if (gemm_grid(ga, BM, BN, &tiles)) return TALSH_LIMIT_EXCEEDED;
-  fgemm_gather_kernel<T, BM, BN><<<(unsigned)tiles, C::THREADS, C::SMEM, st>>>((const T *)L, (const T *)R, (T *)D, ga);
+  fgemm_gather_kernel<T, BM, BN, SEQ><<<(unsigned)tiles, C::THREADS, C::SMEM, st>>>((const T *)L, (const T *)R, (T *)D, ga);
   note_launch();
   return check_launch("fgemm_gather_kernel");
+}
+template <typename T, int BM, int BN>
+int launch_fmma(const void *L, const void *R, void *D, const GemmArgs &ga, cudaStream_t st) {
+  return sequential(ga) ? launch_fmma_as<T, BM, BN, true>(L, R, D, ga, st)
+                        : launch_fmma_as<T, BM, BN, false>(L, R, D, ga, st);
 }
 
 template <typename T>
@@ -1398,8 +1470,9 @@ int check_args(int kind, const int *cptrn, int drank, const int *ddims, int lran
 
 // Scratch bytes of tcTensorContract for this shape (0 when none): the offset
 // tables and, for a split contracted range, the partial sums and counters.
-// `least`, when given, receives what the unsplit form needs: a call with less
-// than the full size but at least that runs unsplit.
+// `least`, when given, receives what the form without partial sums needs: a call
+// with less than the full size but at least that computes the same bits on one
+// CTA per tile.
 size_t contract_scratch_bytes(int kind, const int *cptrn, int drank, const int *ddims, int lrank,
                               const int *ldims, int rrank, const int *rdims, size_t *least) {
   if (least) *least = 0;
@@ -1511,17 +1584,19 @@ int contract_launch(int kind, const int *cptrn, int drank, const int *ddims, int
   }
   KSplit ks;
   int edge = 64;
+  void *part = nullptr;
   if (drank > 0) {
     ks = k_split(kind, T.M, T.N, T.K, T.H);
     edge = gemm_edge(kind, T.M, T.N, T.H, ks);
     const int64_t extra = split_bytes(ks, kind, T.M, T.N, T.H, edge);
-    if (scratch_bytes < need + (size_t)extra || !vec_scratch) {  // no room for partial sums: one CTA per tile
-      ks = KSplit();
-      edge = gemm_edge(kind, T.M, T.N, T.H, ks);
+    if (ks.nsplit > 1 && scratch_bytes >= need + (size_t)extra && vec_scratch) {
+      const int64_t tiles = ((T.M + edge - 1) / edge) * ((T.N + edge - 1) / edge) * T.H;
+      T.ncnt = split_counters(ks, tiles);
+      T.cnt = (int *)((char *)scratch + need);
+      part = (char *)T.cnt + align_up(4 * T.ncnt, 256);
+    } else {  // one CTA per tile
+      edge = gemm_edge(kind, T.M, T.N, T.H, KSplit());
     }
-    const int64_t tiles = ((T.M + edge - 1) / edge) * ((T.N + edge - 1) / edge) * T.H;
-    T.ncnt = split_counters(ks, tiles);
-    T.cnt = (int *)((char *)scratch + need);
   }
   {
     const int64_t total = T.M + T.N + T.K + (T.nh > 0 ? T.H : 0);
@@ -1553,7 +1628,7 @@ int contract_launch(int kind, const int *cptrn, int drank, const int *ddims, int
   }
   ga.nsplit = ks.nsplit; ga.kchunk = ks.kchunk; ga.gsz = ks.gsz;
   ga.cnt = T.cnt;
-  ga.part = (char *)scratch + need + align_up(4 * T.ncnt, 256);
+  ga.part = part;
   switch (kind) {
     case R8: {
       const double *l = (const double *)L, *r = (const double *)R;
@@ -1646,9 +1721,10 @@ struct BatchDesc {
 
 // Tile configurations of the batch: 0 = DMMA 64x64, 1 = DMMA 32x32 (R8),
 // Z = complex on the DMMA pipe, S4 / S14 = packed FP32 FMA 64x64 (R4 / C4).
-enum : int { kCfgD64 = 0, kCfgD32 = 1, kCfgZ64 = 2, kCfgZ32 = 3, kCfgS4 = 4, kCfgS14 = 5, kNumCfg = 6 };
+// From kCfgSeq on: the same for tasks whose split range has no partial sums.
+enum : int { kCfgD64 = 0, kCfgD32 = 1, kCfgZ64 = 2, kCfgZ32 = 3, kCfgS4 = 4, kCfgS14 = 5, kCfgSeq = 6, kNumCfg = 12 };
 // Square tile edge of a configuration.
-inline int cfg_tile(int c) { return (c == kCfgD32 || c == kCfgZ32) ? 32 : 64; }
+inline int cfg_tile(int c) { return (c % kCfgSeq == kCfgD32 || c % kCfgSeq == kCfgZ32) ? 32 : 64; }
 
 __global__ void __launch_bounds__(256) batch_tables_kernel(const BatchDesc *descs) {
   const BatchDesc &d = descs[blockIdx.y];
@@ -1716,8 +1792,8 @@ __device__ __forceinline__ int64_t next_item(unsigned long long *ctr) {
   return item;
 }
 
-template <int BM, int BN>
-__global__ void __launch_bounds__(DmmaCfg<BM, BN>::THREADS, GemmOcc<BM, BN>::D)
+template <int BM, int BN, bool SEQ>
+__global__ void __launch_bounds__(DmmaCfg<BM, BN>::THREADS, SEQ ? 1 : GemmOcc<BM, BN>::D)
     dmma_batch_kernel(const BatchDesc *descs, const int32_t *list, const int64_t *prefix, int n,
                       int64_t total, unsigned long long *ctr) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -1726,13 +1802,13 @@ __global__ void __launch_bounds__(DmmaCfg<BM, BN>::THREADS, GemmOcc<BM, BN>::D)
     const int j = find_task(prefix, n, w);
     const BatchDesc &d = descs[list[j]];
     stage_args(a, d.a);
-    dmma_tile<BM, BN>((const double *)d.L, (const double *)d.R, (double *)d.D, a, item_work(a, (int)(w - prefix[j])),
+    dmma_tile<BM, BN, SEQ>((const double *)d.L, (const double *)d.R, (double *)d.D, a, item_work(a, (int)(w - prefix[j])),
                       smem);
   }
 }
 
-template <int BM, int BN>
-__global__ void __launch_bounds__(ZmmaCfg<BM, BN>::THREADS, GemmOcc<BM, BN>::Z)
+template <int BM, int BN, bool SEQ>
+__global__ void __launch_bounds__(ZmmaCfg<BM, BN>::THREADS, SEQ ? 1 : GemmOcc<BM, BN>::Z)
     zmma_batch_kernel(const BatchDesc *descs, const int32_t *list, const int64_t *prefix, int n,
                       int64_t total, unsigned long long *ctr) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -1741,13 +1817,13 @@ __global__ void __launch_bounds__(ZmmaCfg<BM, BN>::THREADS, GemmOcc<BM, BN>::Z)
     const int j = find_task(prefix, n, w);
     const BatchDesc &d = descs[list[j]];
     stage_args(a, d.a);
-    zmma_tile<BM, BN>((const double2 *)d.L, (const double2 *)d.R, (double2 *)d.D, a,
+    zmma_tile<BM, BN, SEQ>((const double2 *)d.L, (const double2 *)d.R, (double2 *)d.D, a,
                       item_work(a, (int)(w - prefix[j])), smem);
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(FmmaCfg<T, 64, 64>::THREADS, FmmaOcc<T, 64>::N)
+template <typename T, bool SEQ>
+__global__ void __launch_bounds__(FmmaCfg<T, 64, 64>::THREADS, SEQ ? 1 : FmmaOcc<T, 64>::N)
     fmma_batch_kernel(const BatchDesc *descs, const int32_t *list, const int64_t *prefix, int n,
                       int64_t total, unsigned long long *ctr) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -1756,7 +1832,7 @@ __global__ void __launch_bounds__(FmmaCfg<T, 64, 64>::THREADS, FmmaOcc<T, 64>::N
     const int j = find_task(prefix, n, w);
     const BatchDesc &d = descs[list[j]];
     stage_args(a, d.a);
-    fmma_tile<T, 64, 64>((const T *)d.L, (const T *)d.R, (T *)d.D, a, item_work(a, (int)(w - prefix[j])), smem);
+    fmma_tile<T, 64, 64, SEQ>((const T *)d.L, (const T *)d.R, (T *)d.D, a, item_work(a, (int)(w - prefix[j])), smem);
   }
 }
 
@@ -1796,8 +1872,8 @@ int batch_cfg_of(int kind, int64_t M, int64_t N) {
   }
 }
 
-// `lean` (one flag per task, or null): no partial sums for that task, whose
-// contracted range then is not split.
+// `lean` (one flag per task, or null): no partial sums for that task; each CTA
+// of a tile then walks the task's splits itself.
 int batch_plan(int ntasks, const tcContractTask *tasks, BatchPlan &bp, const std::vector<char> *lean = nullptr) {
   if (ntasks < 0 || ntasks > 65535 || (ntasks > 0 && tasks == nullptr)) return TALSH_INVALID_ARGS;
   bp.descs.assign(ntasks, BatchDesc());
@@ -1854,16 +1930,17 @@ int batch_plan(int ntasks, const tcContractTask *tasks, BatchPlan &bp, const std
     a.b_along_n = an.b_along_n ? 1 : 0;
     a.conj_l = cl; a.conj_r = cr;
     d.L = x.L; d.R = x.R; d.D = x.D;
-    const int c = batch_cfg_of(x.data_kind, T.M, T.N);
+    int c = batch_cfg_of(x.data_kind, T.M, T.N);
     const int bm = cfg_tile(c), bn = bm;
     a.tiles_m = (int)((T.M + bm - 1) / bm);
     const int64_t tiles = (int64_t)a.tiles_m * ((T.N + bn - 1) / bn);
     if (tiles > 0x7fffffffLL) return TALSH_LIMIT_EXCEEDED;
     a.tiles_mn = (int)tiles;
-    a.nsplit = 1;
-    if (!(lean && (*lean)[t])) {
-      const KSplit ks = k_split(x.data_kind, T.M, T.N, T.K, 1);
-      a.nsplit = ks.nsplit; a.kchunk = ks.kchunk; a.gsz = ks.gsz;
+    const KSplit ks = k_split(x.data_kind, T.M, T.N, T.K, 1);
+    a.nsplit = ks.nsplit; a.kchunk = ks.kchunk; a.gsz = ks.gsz;
+    if (lean && (*lean)[t]) {
+      if (ks.nsplit > 1) c += kCfgSeq;
+    } else {
       a.ncnt = (int)split_counters(ks, tiles);
       bp.part_off[t] = part;
       part += (size_t)align_up(split_bytes(ks, x.data_kind, T.M, T.N, 1, bm), 256);
@@ -1874,10 +1951,8 @@ int batch_plan(int ntasks, const tcContractTask *tasks, BatchPlan &bp, const std
     bp.list[c].push_back(t);
   }
   // Longest items (largest K, or K chunk) first, then the item prefix sums.
-  auto span = [&](int t) {
-    const GemmArgs &a = bp.descs[t].a;
-    return a.nsplit > 1 ? a.kchunk : a.K;
-  };
+  auto splits = [&](int t) { return bp.cfg[t] >= kCfgSeq ? 1 : bp.descs[t].a.nsplit; };  // CTAs that share a tile
+  auto span = [&](int t) { return splits(t) > 1 ? bp.descs[t].a.kchunk : bp.descs[t].a.K; };
   for (int c = 0; c < kNumCfg; ++c) {
     auto &l = bp.list[c];
     std::stable_sort(l.begin(), l.end(), [&](int x, int y) { return span(x) > span(y); });
@@ -1885,23 +1960,26 @@ int batch_plan(int ntasks, const tcContractTask *tasks, BatchPlan &bp, const std
     if (l.empty()) continue;
     pl.push_back(0);
     for (int t : l) {
-      const GemmArgs &a = bp.descs[t].a;
-      pl.push_back(pl.back() + (int64_t)a.tiles_mn * a.nsplit);
+      pl.push_back(pl.back() + (int64_t)bp.descs[t].a.tiles_mn * splits(t));
     }
   }
   size_t off = 0;
-  auto take = [&](size_t bytes) { const size_t o = off; off = (off + bytes + 255) & ~size_t(255); return o; };
+  auto take = [&](size_t bytes, size_t unit = 256) {
+    const size_t o = off = (off + unit - 1) / unit * unit;
+    off += bytes;
+    return o;
+  };
   bp.off_desc = take(sizeof(BatchDesc) * (size_t)std::max(ntasks, 1));
   for (int c = 0; c < kNumCfg; ++c) {
-    bp.off_list[c] = take(sizeof(int32_t) * bp.list[c].size());
-    bp.off_prefix[c] = take(sizeof(int64_t) * bp.prefix[c].size());
+    bp.off_list[c] = take(sizeof(int32_t) * bp.list[c].size(), 16);
+    bp.off_prefix[c] = take(sizeof(int64_t) * bp.prefix[c].size(), 16);
   }
   bp.off_tab = take(sizeof(int64_t) * (size_t)tab);
   bp.off_ctr = take(sizeof(unsigned long long) * kNumCfg);
   for (int t = 0; t < ntasks; ++t)
     if (bp.cfg[t] < 0) bp.fb_off[t] = take(bp.fb_scratch[t]);
   bp.off_part = take(part);
-  bp.total = off;
+  bp.total = (off + 255) & ~size_t(255);
   return TALSH_SUCCESS;
 }
 
@@ -1924,37 +2002,53 @@ int launch_tc_batch(BatchKernel k, int threads, size_t smem, const char *name, c
   return check_launch(name);
 }
 
-template <int BM, int BN>
+template <int BM, int BN, bool SEQ>
 int launch_dmma_batch(const BatchPlan &bp, int c, char *base, cudaStream_t st) {
   using C = DmmaCfg<BM, BN>;
   static std::atomic<uint64_t> attr{0};
   once_per_device(attr, [] {
-    cudaFuncSetAttribute(dmma_batch_kernel<BM, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
-    cudaFuncSetAttribute(dmma_batch_kernel<BM, BN>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    cudaFuncSetAttribute(dmma_batch_kernel<BM, BN, SEQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+    cudaFuncSetAttribute(dmma_batch_kernel<BM, BN, SEQ>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   });
-  return launch_tc_batch(dmma_batch_kernel<BM, BN>, C::THREADS, C::SMEM, "dmma_batch_kernel", bp, c, base, st);
+  return launch_tc_batch(dmma_batch_kernel<BM, BN, SEQ>, C::THREADS, C::SMEM, "dmma_batch_kernel", bp, c, base, st);
 }
 
-template <int BM, int BN>
+template <int BM, int BN, bool SEQ>
 int launch_zmma_batch(const BatchPlan &bp, int c, char *base, cudaStream_t st) {
   using Z = ZmmaCfg<BM, BN>;
   static std::atomic<uint64_t> attr{0};
   once_per_device(attr, [] {
-    cudaFuncSetAttribute(zmma_batch_kernel<BM, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Z::SMEM);
-    cudaFuncSetAttribute(zmma_batch_kernel<BM, BN>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    cudaFuncSetAttribute(zmma_batch_kernel<BM, BN, SEQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Z::SMEM);
+    cudaFuncSetAttribute(zmma_batch_kernel<BM, BN, SEQ>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   });
-  return launch_tc_batch(zmma_batch_kernel<BM, BN>, Z::THREADS, Z::SMEM, "zmma_batch_kernel", bp, c, base, st);
+  return launch_tc_batch(zmma_batch_kernel<BM, BN, SEQ>, Z::THREADS, Z::SMEM, "zmma_batch_kernel", bp, c, base, st);
 }
 
-template <typename T>
+template <typename T, bool SEQ>
 int launch_fmma_batch(const BatchPlan &bp, int c, char *base, cudaStream_t st) {
   using C = FmmaCfg<T, 64, 64>;
   static std::atomic<uint64_t> attr{0};
   once_per_device(attr, [] {
-    cudaFuncSetAttribute(fmma_batch_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
-    cudaFuncSetAttribute(fmma_batch_kernel<T>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    cudaFuncSetAttribute(fmma_batch_kernel<T, SEQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+    cudaFuncSetAttribute(fmma_batch_kernel<T, SEQ>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   });
-  return launch_tc_batch(fmma_batch_kernel<T>, C::THREADS, C::SMEM, "fmma_batch_kernel", bp, c, base, st);
+  return launch_tc_batch(fmma_batch_kernel<T, SEQ>, C::THREADS, C::SMEM, "fmma_batch_kernel", bp, c, base, st);
+}
+
+// The persistent launch of configuration c.
+template <bool SEQ>
+int launch_cfg_as(const BatchPlan &bp, int c, char *base, cudaStream_t st) {
+  switch (c % kCfgSeq) {
+    case kCfgD64: return launch_dmma_batch<64, 64, SEQ>(bp, c, base, st);
+    case kCfgD32: return launch_dmma_batch<32, 32, SEQ>(bp, c, base, st);
+    case kCfgZ64: return launch_zmma_batch<64, 64, SEQ>(bp, c, base, st);
+    case kCfgZ32: return launch_zmma_batch<32, 32, SEQ>(bp, c, base, st);
+    case kCfgS4: return launch_fmma_batch<float, SEQ>(bp, c, base, st);
+    default: return launch_fmma_batch<float2, SEQ>(bp, c, base, st);
+  }
+}
+int launch_cfg(const BatchPlan &bp, int c, char *base, cudaStream_t st) {
+  return c < kCfgSeq ? launch_cfg_as<false>(bp, c, base, st) : launch_cfg_as<true>(bp, c, base, st);
 }
 
 }  // namespace
@@ -1985,7 +2079,7 @@ int64_t batch_bind(BatchPlan &bp, char *base) {
     int64_t *p = tabs + bp.tab_off[t];
     a.mL = p; a.mD = p + a.M; a.nR = a.mD + a.M; a.nD = a.nR + a.N; a.kL = a.nD + a.N; a.kR = a.kL + a.K;
     a.cnt = (int *)(base + bp.off_part + bp.part_off[t]);
-    a.part = (char *)a.cnt + align_up(4 * (int64_t)a.ncnt, 256);
+    a.part = bp.cfg[t] < kCfgSeq ? (char *)a.cnt + align_up(4 * (int64_t)a.ncnt, 256) : nullptr;
     max_entries = std::max<int64_t>(max_entries, (int64_t)a.M + a.N + a.K);
   }
   return max_entries;
@@ -2026,12 +2120,8 @@ int batch_run(int ntasks, const tcContractTask *tasks, BatchPlan &bp, void *scra
     note_launch();
     if ((rc = check_launch("batch_tables_kernel")) != 0) return rc;
   }
-  if (!bp.list[kCfgD64].empty() && (rc = launch_dmma_batch<64, 64>(bp, kCfgD64, base, st)) != 0) return rc;
-  if (!bp.list[kCfgD32].empty() && (rc = launch_dmma_batch<32, 32>(bp, kCfgD32, base, st)) != 0) return rc;
-  if (!bp.list[kCfgZ64].empty() && (rc = launch_zmma_batch<64, 64>(bp, kCfgZ64, base, st)) != 0) return rc;
-  if (!bp.list[kCfgZ32].empty() && (rc = launch_zmma_batch<32, 32>(bp, kCfgZ32, base, st)) != 0) return rc;
-  if (!bp.list[kCfgS4].empty() && (rc = launch_fmma_batch<float>(bp, kCfgS4, base, st)) != 0) return rc;
-  if (!bp.list[kCfgS14].empty() && (rc = launch_fmma_batch<float2>(bp, kCfgS14, base, st)) != 0) return rc;
+  for (int c = 0; c < kNumCfg; ++c)
+    if (!bp.list[c].empty() && (rc = launch_cfg(bp, c, base, st)) != 0) return rc;
   for (int t = 0; t < ntasks; ++t) {
     if (bp.cfg[t] >= 0) continue;
     const tcContractTask &x = tasks[t];
@@ -2066,7 +2156,9 @@ size_t batch_task_scratch_bound(const tcContractTask &x, bool lean) {
   return sizeof(BatchDesc) + sizeof(int32_t) + sizeof(int64_t) + fb + 256;
 }
 
-size_t batch_fixed_scratch() { return (size_t)(2 * kNumCfg + 4) * 256 + sizeof(unsigned long long) * kNumCfg; }
+// Rounding of the blocks (lists and prefix sums to 16 bytes, the others to 256) and the counters.
+size_t batch_fixed_scratch() { return (size_t)16 * 256 + 48; }
+static_assert(kNumCfg * (2 * 16 + 8 + 8) + 6 * 256 <= 16 * 256 + 48, "the roundings fit");
 
 // Plans a batch, asks `get` for device scratch and a pinned staging block of
 // the sizes the plan needs (get returns nullptr to refuse: TRY_LATER), and
@@ -2185,16 +2277,7 @@ extern "C" int tcContractBatchGraphCreate(int ntasks, const tcContractTask *task
   for (int b = 0; b < nbr; ++b) cudaStreamWaitEvent(br[b], ev[nbr], 0);
   const unsigned before = (unsigned)tcKernelLaunchCount();
   for (size_t b = 0; b < used.size() && rc == TALSH_SUCCESS && e == cudaSuccess; ++b) {
-    const int c = used[b];
-    cudaStream_t s2 = br[b];
-    switch (c) {
-      case kCfgD64: rc = launch_dmma_batch<64, 64>(bp, c, base, s2); break;
-      case kCfgD32: rc = launch_dmma_batch<32, 32>(bp, c, base, s2); break;
-      case kCfgZ64: rc = launch_zmma_batch<64, 64>(bp, c, base, s2); break;
-      case kCfgZ32: rc = launch_zmma_batch<32, 32>(bp, c, base, s2); break;
-      case kCfgS4: rc = launch_fmma_batch<float>(bp, c, base, s2); break;
-      default: rc = launch_fmma_batch<float2>(bp, c, base, s2); break;
-    }
+    rc = launch_cfg(bp, used[b], base, br[b]);
   }
   for (int t = 0; t < ntasks && fallbacks && rc == TALSH_SUCCESS && e == cudaSuccess; ++t) {
     if (bp.cfg[t] >= 0) continue;

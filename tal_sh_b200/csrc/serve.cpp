@@ -74,7 +74,7 @@ struct STask {
   size_t out_bytes = 0;    // server-held output bytes (0: caller's D)
   void *scratch = nullptr; // large tasks: scratch allocated at admission
   size_t scratch_bytes = 0;
-  bool lean = false;       // no room in the budget for partial sums: contracted range not split
+  bool lean = false;       // no room in the budget for partial sums: one CTA per output tile, same bits
   size_t reserve = 0;      // small tasks: budget held for their share of a batch's scratch
   int consumers_left = 0;  // declared consumers that have not completed
   int readers = 0;         // submitted consumers that have not completed
@@ -280,8 +280,8 @@ void admit(tcServer *s, int cls) {
     };
     size_up();
     if (need > s->cfg.budget_bytes && !t.lean) {
-      // A task that fits only without partial sums runs unsplit.  This depends
-      // on the budget alone, so its result does not depend on the other tasks.
+      // A task that fits only without partial sums runs without them: the same
+      // bits on fewer CTAs.
       t.lean = true;
       if (t.large) t.scratch_bytes = large_scratch(t, s->cfg.r8_slices);
       size_up();

@@ -283,6 +283,30 @@ def test_admission_under_budget(talsh):
         assert _rel(_host(d, (256, 4)), ref) <= TOL_FP64
 
 
+@pytest.mark.parametrize("large_flop", [1, 1 << 40])
+def test_budget_without_room_for_partial_sums(talsh, large_flop):
+    """A long contracted range (1.8 MB of partial sums) under a 1.5 MB budget runs without them, as
+    a large task and in a batch of small ones: the bits of a roomy server."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(21)
+    p, e = "D(a,b)+=L(k,a)*R(b,k)", dict(a=33, k=30001, b=18)
+    Lh, Rh = rand([30001, 33], T.R8, rng), rand([18, 30001], T.R8, rng)
+    l, r = _cuda(torch, Lh), _cuda(torch, Rh)
+    got = []
+    for budget in (1 << 30, 3 << 19):
+        out = [torch.zeros(33 * 18, dtype=torch.float64, device="cuda") for _ in range(3)]
+        srv = Server(budget_bytes=budget, large_flop=large_flop)
+        for d in out:
+            assert srv.submit(_task(T.R8, p, e, L=l.data_ptr(), R=r.data_ptr(), D=d.data_ptr()))[0] == 0
+        srv.drain()
+        st = srv.stats()
+        assert st.failed == 0 and st.bytes_peak <= budget and st.bytes_in_use == 0
+        srv.close()
+        got += out
+    assert all(torch.equal(x, got[0]) for x in got)
+    assert _rel(_host(got[0], (33, 18)), Lh.T @ Rh.T) <= TOL_FP64
+
+
 def test_keep_output_and_release(talsh):
     torch = pytest.importorskip("torch")
     rng = np.random.default_rng(3)
