@@ -24,6 +24,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstring>
 #include <type_traits>
 #include <vector>
@@ -1236,17 +1237,56 @@ int analyze(const int *cptrn, int drank, const int *ddims, int lrank, const int 
   return TALSH_SUCCESS;
 }
 
+// Elements of one 64-row (or 64-column) tile that lie next to each other in a
+// tensor: its stride-1 dimension as far as the tile covers it, and the next one
+// where it is covered whole.  A group's dimension is covered as far as 64 rows
+// reach past the dimensions before it; contracted dimensions are walked whole.
+struct GroupView {
+  int n;
+  const int64_t *ext, *str;
+  bool whole;
+};
+int64_t tile_run(const GroupView &a, const GroupView &b) {
+  int64_t run = 1;
+  for (;;) {
+    int64_t covered = 0, extent = 0;
+    for (const GroupView *g : {&a, &b}) {
+      int64_t before = 1;
+      for (int d = 0; d < g->n && before <= 64; ++d) {
+        if (g->str[d] == run) {
+          extent = g->ext[d];
+          covered = g->whole ? extent : std::min(extent, 64 / before);
+        }
+        if (!g->whole) before *= g->ext[d];
+      }
+    }
+    if (covered < 2) return run;
+    run *= covered;
+    if (covered < extent) return run;
+  }
+}
+
 // Order of the free indices for the GEMM tiles.  `analyze` lists them in their
 // operand's order, which makes that operand's loads contiguous when its
 // stride-1 index is free, but may scatter D, whose sectors then cross the L2
-// once per element, read and written.  When the stride-1 index is contracted
+// once per element, read and written.  Where the stride-1 index is contracted
 // anyway, or K < 384 and D's fastest index belongs to the group but does not
-// lead it, the group follows D's order (D(a,b,c,d) += L(e,b,a,d) R(c,e), 101 x 69
-// x 105 x 58, K = 51 in R4: 997 -> 307 us; D(a,b,c,d,e,f) += L(d,e,g,a) R(g,f,b,c),
-// 4608 x 4896 outputs in R8: operand's order / D's order 775 / 283 us at K = 64,
-// 1076 / 880 at 300, 1343 / 1395 at 500).  The order moves elements between tiles
+// lead it, the group takes D's order if that moves fewer sectors: L is read
+// ceil(N / 64) times, R ceil(M / 64) times, D read and written once, at es / 32
+// sectors per element and about one more per run.  One sector of D weighs as
+// much as `w` of an operand, fitted to where the two orders met on
+// D(e,m,i) += L(m,k,e,c) R(c,k,i), 131328 x i outputs (us, operand's / D's order):
+//   R8  i = 1:  44 / 65 at K = 20, 186 / 650 at 300;   8: 84 / 69, 217 / 660
+//      24: 207 / 241 at 100;   64: 344 / 249 at 100, 453 / 660 at 300
+//   R4  i = 8: 98 / 124 at 100;  64: 317 / 237 at 200, 355 / 355 at 300
+//   C8  i = 8: 152 / 154 at 100, 290 / 353 at 300;  64: 848 / 692 at 300
+//   C4  i = 8: 120 / 124 at 20;  64: 411 / 398 at 100, 573 / 699 at 200
+// (K < 384 alone chose D's order in all of these).  Outputs wide both ways gain
+// most: D(a,b,c,d) += L(e,b,a,d) R(c,e), 101 x 69 x 105 x 58, K = 51 in R4: 997
+// -> 307 us; D(a,b,c,d,e,f) += L(d,e,g,a) R(g,f,b,c), 4608 x 4896 in R8: 728 ->
+// 230 us at K = 64, 993 -> 776 at 300.  The order moves elements between tiles
 // only: every element's sum is unchanged.
-void order_by_output(Analysis &an) {
+void order_by_output(Analysis &an, int es, bool cplx) {
   TableParams &T = an.T;
   auto smallest = [](const int64_t *str, int n) {
     int64_t s = INT64_MAX;
@@ -1254,19 +1294,51 @@ void order_by_output(Analysis &an) {
     return s;
   };
   const int64_t dm = smallest(T.mstrD, T.nm), dn = smallest(T.nstrD, T.nn);
-  auto sort_group = [](int n, int64_t *ext, int64_t *op, int64_t *d) {
-    for (int i = 1; i < n; ++i)
-      for (int j = i; j > 0 && d[j] < d[j - 1]; --j) {
-        std::swap(ext[j], ext[j - 1]);
-        std::swap(op[j], op[j - 1]);
-        std::swap(d[j], d[j - 1]);
-      }
-  };
   const bool short_k = T.K < 384;
-  if (!an.a_along_m || (short_k && dm < dn && T.nm > 0 && T.mstrD[0] != dm))
-    sort_group(T.nm, T.mext, T.mstrL, T.mstrD);
-  if (!an.b_along_n || (short_k && dn < dm && T.nn > 0 && T.nstrD[0] != dn))
-    sort_group(T.nn, T.next, T.nstrR, T.nstrD);
+  const bool may_m = !an.a_along_m || (short_k && dm < dn && T.nm > 0 && T.mstrD[0] != dm);
+  const bool may_n = !an.b_along_n || (short_k && dn < dm && T.nn > 0 && T.nstrD[0] != dn);
+  if (!may_m && !may_n) return;
+  struct Group {
+    int64_t ext[kMaxGR], op[kMaxGR], d[kMaxGR];
+  };
+  auto take = [](Group &g, int n, const int64_t *ext, const int64_t *op, const int64_t *d, bool sorted) {
+    for (int i = 0; i < n; ++i) {
+      int j = i;
+      for (; sorted && j > 0 && d[i] < g.d[j - 1]; --j) {
+        g.ext[j] = g.ext[j - 1];
+        g.op[j] = g.op[j - 1];
+        g.d[j] = g.d[j - 1];
+      }
+      g.ext[j] = ext[i];
+      g.op[j] = op[i];
+      g.d[j] = d[i];
+    }
+  };
+  const double w = cplx ? (es == 16 ? 12.0 : 2.0) : (es == 8 ? 3.0 : 5.0);
+  const double M = (double)T.M, N = (double)T.N, K = (double)T.K;
+  auto sectors = [&](int64_t run) { return es / 32.0 + (1.0 - es / 32.0) / (double)run; };
+  double least = 0.0;
+  Group m, n;
+  for (int c = 0; c < 4; ++c) {  // bit 0: m in D's order, bit 1: n
+    if (((c & 1) && !may_m) || ((c & 2) && !may_n)) continue;
+    Group gm, gn;
+    take(gm, T.nm, T.mext, T.mstrL, T.mstrD, c & 1);
+    take(gn, T.nn, T.next, T.nstrR, T.nstrD, c & 2);
+    // where both move as much, D's order is the faster one under a contracted stride-1 index
+    const double even = ((c & 1) && !an.a_along_m ? 0.98 : 1.0) * ((c & 2) && !an.b_along_n ? 0.98 : 1.0);
+    const double cost =
+        even *
+        (M * K * std::ceil(N / 64) * sectors(tile_run({T.nm, gm.ext, gm.op, false}, {T.nk, T.kext, T.kstrL, true})) +
+        N * K * std::ceil(M / 64) * sectors(tile_run({T.nn, gn.ext, gn.op, false}, {T.nk, T.kext, T.kstrR, true})) +
+        w * M * N * sectors(tile_run({T.nm, gm.ext, gm.d, false}, {T.nn, gn.ext, gn.d, false})));
+    if (c == 0 || cost < least) {
+      least = cost;
+      m = gm;
+      n = gn;
+    }
+  }
+  std::copy(m.ext, m.ext + T.nm, T.mext); std::copy(m.op, m.op + T.nm, T.mstrL); std::copy(m.d, m.d + T.nm, T.mstrD);
+  std::copy(n.ext, n.ext + T.nn, T.next); std::copy(n.op, n.op + T.nn, T.nstrR); std::copy(n.d, n.d + T.nn, T.nstrD);
 }
 
 int sm_count_dev() { return current_sm_count(); }
@@ -1557,7 +1629,7 @@ int contract_launch(int kind, const int *cptrn, int drank, const int *ddims, int
   }
   Analysis an;
   if ((rc = analyze(cptrn, drank, ddims, lrank, ldims, rrank, rdims, an)) != 0) return rc;
-  order_by_output(an);
+  order_by_output(an, kind_size(kind), kind_is_complex(kind));
   TableParams T = an.T;
   const size_t need = table_bytes(T) + (drank == 0 ? (size_t)dot_blocks(T.K) * sizeof(double2) : 0);
   if (scratch == nullptr || scratch_bytes < need) return TALSH_INVALID_ARGS;
@@ -1906,7 +1978,7 @@ int batch_plan(int ntasks, const tcContractTask *tasks, BatchPlan &bp, const std
       if (lean && (*lean)[t]) bp.fb_scratch[t] = least;
       continue;
     }
-    order_by_output(an);
+    order_by_output(an, kind_size(x.data_kind), kind_is_complex(x.data_kind));
     const TableParams &T = an.T;
     BatchDesc &d = bp.descs[t];
     d.nm = T.nm; d.nn = T.nn; d.nk = T.nk; d.es = kind_size(x.data_kind);

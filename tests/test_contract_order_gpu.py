@@ -1,6 +1,6 @@
 """Contractions whose free indices are walked in D's order (the operand's stride-1 index is contracted, or K is
-short and D's fastest index does not lead its group): against numpy in 64 bits on both sides of the rule, alone and
-bit for bit in a batch."""
+short and D's fastest index does not lead its group, where that moves fewer sectors): against numpy in 64 bits on both
+sides of the rule, alone and bit for bit in a batch."""
 import re
 
 import numpy as np
@@ -18,7 +18,14 @@ CASES = [("D(a,b,c,d)+=L(e,b,a,d)*R(c,e)", dict(a=13, b=9, c=11, d=7, e=17)),
          ("D(a,b,c,d,e,f)+=L(d,e,g,a)*R(g,f,b,c)", dict(a=9, b=3, c=5, d=7, e=2, f=6, g=383)),
          ("D(a,b,c,d,e,f)+=L(d,e,g,a)*R(g,f,b,c)", dict(a=9, b=3, c=5, d=7, e=2, f=6, g=384)),
          ("D(b,a,d,c)+=L(c,k,d)*R(a,k,b)", dict(a=21, b=13, c=11, d=9, k=15)),
-         ("D(b,a,h,d,c)+=L(c,k,h,d)*R(a,k,h,b)", dict(a=11, b=13, c=8, d=9, k=15, h=3))]
+         ("D(b,a,h,d,c)+=L(c,k,h,d)*R(a,k,h,b)", dict(a=11, b=13, c=8, d=9, k=15, h=3)),
+         # outputs thin one way, where the line moves with the width: operand's order and D's
+         ("D(e,m)+=L(m,k,e,c)*R(c,k)", dict(m=17, k=15, e=70, c=20)),
+         ("D(e,m,i)+=L(m,k,e,c)*R(c,k,i)", dict(m=17, k=2, e=70, c=3, i=8)),
+         ("D(e,m,i)+=L(m,k,e,c)*R(c,k,i)", dict(m=17, k=15, e=70, c=20, i=8)),
+         ("D(e,m,i)+=L(m,k,e,c)*R(c,k,i)", dict(m=17, k=4, e=70, c=5, i=65)),
+         ("D(e,m,i)+=L(k,m,e,c)*R(c,k,i)", dict(m=17, k=2, e=70, c=100, i=3)),
+         ("D(j,i,a)+=L(k,a)*R(i,j,k)", dict(i=70, j=33, k=40, a=2))]
 
 
 @pytest.mark.parametrize("kind", [T.R4, T.R8, T.C4, T.C8])
