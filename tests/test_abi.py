@@ -706,7 +706,7 @@ def test_every_reference_header_function_is_exported(built):
     only; this core does not use cuTENSOR).  Skipped where the reference sources
     are absent."""
     ref = _reference_tree()
-    if ref is None:
+    if ref is None or not os.path.exists(os.path.join(ref, "talsh.h")):
         pytest.skip("reference sources not present")
     L = T.lib()
     names = set()
