@@ -803,7 +803,7 @@ __device__ __forceinline__ float2 unpack2(uint64_t v) {
 template <typename T, int BM, int BN>
 struct FmmaCfg {
   static constexpr int VE = 16 / (int)sizeof(T);
-  static constexpr int MC = sizeof(T) == 4 ? 2 : 4, NC = 2;
+  static constexpr int MC = sizeof(T) == 4 || BM <= 32 ? 2 : 4, NC = 2;
   static constexpr int TMN = BM / (MC * VE), TNN = BN / (NC * VE);  // threads along m and n
   static constexpr int THREADS = TMN * TNN;
   static constexpr int BK = 16, STAGES = 3;
@@ -1024,6 +1024,7 @@ __device__ __forceinline__ void fmma_tile(const T *__restrict__ L, const T *__re
 template <typename T, int BM> struct FmmaOcc { static constexpr int N = 4; };
 template <> struct FmmaOcc<float, 64> { static constexpr int N = 6; };  // 7: 5 % slower (spills)
 template <> struct FmmaOcc<float, 128> { static constexpr int N = 2; };
+template <> struct FmmaOcc<float2, 32> { static constexpr int N = 8; };
 
 template <typename T, int BM, int BN, bool SEQ>
 __global__ void __launch_bounds__(FmmaCfg<T, BM, BN>::THREADS, SEQ ? 1 : FmmaOcc<T, BM>::N)
@@ -1402,13 +1403,17 @@ int64_t split_bytes(const KSplit &s, int kind, int64_t M, int64_t N, int64_t H, 
 // CTA tile edge of a single contraction.  R8, C8: 64, or 32 when even the split
 // 64 x 64 tiles do not give every SM one.  (128 x 128 R8 tiles, one CTA of 16
 // warps per SM, were 1.5 % slower than four 64 x 64 CTAs on 3072 x 3072 x 3072:
-// independent CTAs fill each other's barrier gaps.)  R4: 128 when two of those
-// per SM exist and are mostly filled, else 64.  Results do not depend on it.
+// independent CTAs fill each other's barrier gaps.)  C4: 32, whose two warps
+// leave eight CTAs per SM to hide a k step's latency behind (64 / 32, us: 18
+// tiles of 64, K = 169: 55 / 25, 45 before the packed kernel; 105 tiles, K =
+// 459: 125 / 76; 131000 x 1, K = 20: 98 / 53; 3000 x 3000 x 3000: 5847 / 5799).
+// R4: 128 when two of those per SM exist and are mostly filled, else 64.
+// Results do not depend on it.
 int gemm_edge(int kind, int64_t M, int64_t N, int64_t H, const KSplit &s) {
   auto tiles = [&](int64_t e) { return ((M + e - 1) / e) * ((N + e - 1) / e) * std::max<int64_t>(H, 1); };
   const int64_t sms = sm_count_dev();
   if (kind == R4) return tiles(128) >= 2 * sms && tiles(64) >= 3 * tiles(128) ? 128 : 64;
-  if (kind == C4) return 64;
+  if (kind == C4) return 32;
   return tiles(64) * s.nsplit >= sms ? 64 : 32;
 }
 
@@ -1710,7 +1715,7 @@ int contract_launch(int kind, const int *cptrn, int drank, const int *ddims, int
     case R4:
       if (edge == 128) return launch_fmma<float, 128, 128>(L, R, D, ga, st);
       return launch_fmma<float, 64, 64>(L, R, D, ga, st);
-    case C4: return launch_fmma<float2, 64, 64>(L, R, D, ga, st);
+    case C4: return launch_fmma<float2, 32, 32>(L, R, D, ga, st);
     default:
       if (edge == 64) return launch_zmma<64, 64>((const double2 *)L, (const double2 *)R, (double2 *)D, ga, st);
       return launch_zmma<32, 32>((const double2 *)L, (const double2 *)R, (double2 *)D, ga, st);
