@@ -330,12 +330,12 @@ int tcServerReplay(tcServer *srv, int n, const tcServeTask *tasks, const double 
  * each class present among `tasks`, runs that class's tasks as one batch with
  * 32x32 and with 64x64 tiles (`reps` timed runs each after one warm-up, CUDA
  * events on `stream`) and keeps the faster tile for the class; later batches
- * (tcTensorContractBatch, the contraction server) use it, so query
- * tcTensorContractBatchScratch again afterwards (the scratch size depends on
- * the tiles).  The tasks are executed several times, so their D contents are
- * unspecified afterwards.
- * scratch: at least tcTensorContractBatchScratch(ntasks, tasks) bytes.  Not to
- * run concurrently with other batch launches. */
+ * (tcTensorContractBatch, the contraction server) use it.  The scratch size
+ * does not depend on the choice.  The tasks are executed several times, so
+ * their D contents are unspecified afterwards.
+ * scratch: as for tcTensorContractBatch (without room for partial sums both
+ * tiles are timed without them).  Not to run concurrently with other batch
+ * launches. */
 int tcTensorContractBatchTune(int ntasks, const tcContractTask *tasks, void *scratch, size_t scratch_bytes,
                               void *stream, int reps);
 /* Tile edge chosen for a class (0: not tuned, the shape rule applies; -1: bad class). */

@@ -1949,6 +1949,15 @@ int batch_cfg_of(int kind, int64_t M, int64_t N) {
   }
 }
 
+// Bytes of a task's partial sums and counters for whichever tile edge it gets, so
+// that the scratch of a batch does not depend on what was tuned, when, or on the
+// edge the autotuner is trying.
+size_t batch_part_bytes(const KSplit &ks, int kind, int64_t M, int64_t N) {
+  const int64_t wide = split_bytes(ks, kind, M, N, 1, 64);
+  const bool narrow = kind == R8 || kind == C8;
+  return (size_t)align_up(narrow ? std::max(wide, split_bytes(ks, kind, M, N, 1, 32)) : wide, 256);
+}
+
 // `lean` (one flag per task, or null): no partial sums for that task; each CTA
 // of a tile then walks the task's splits itself.
 int batch_plan(int ntasks, const tcContractTask *tasks, BatchPlan &bp, const std::vector<char> *lean = nullptr) {
@@ -2020,7 +2029,7 @@ int batch_plan(int ntasks, const tcContractTask *tasks, BatchPlan &bp, const std
     } else {
       a.ncnt = (int)split_counters(ks, tiles);
       bp.part_off[t] = part;
-      part += (size_t)align_up(split_bytes(ks, x.data_kind, T.M, T.N, 1, bm), 256);
+      part += batch_part_bytes(ks, x.data_kind, T.M, T.N);
     }
     bp.cfg[t] = c;
     bp.tab_off[t] = tab;
@@ -2047,10 +2056,13 @@ int batch_plan(int ntasks, const tcContractTask *tasks, BatchPlan &bp, const std
     return o;
   };
   bp.off_desc = take(sizeof(BatchDesc) * (size_t)std::max(ntasks, 1));
+  // The lists take the same room however the tasks fall into them.
+  const size_t lists = off + (size_t)ntasks * (sizeof(int32_t) + sizeof(int64_t)) + kNumCfg * (sizeof(int64_t) + 2 * 16);
   for (int c = 0; c < kNumCfg; ++c) {
     bp.off_list[c] = take(sizeof(int32_t) * bp.list[c].size(), 16);
     bp.off_prefix[c] = take(sizeof(int64_t) * bp.prefix[c].size(), 16);
   }
+  off = lists;
   bp.off_tab = take(sizeof(int64_t) * (size_t)tab);
   bp.off_ctr = take(sizeof(unsigned long long) * kNumCfg);
   for (int t = 0; t < ntasks; ++t)
@@ -2225,9 +2237,8 @@ size_t batch_task_scratch_bound(const tcContractTask &x, bool lean) {
     const TableParams &T = an.T;
     if (an.hyper) {  // single-task path inside the batch
       fb = full;
-    } else {         // either tile edge of the batch kernels
-      const KSplit ks = k_split(x.data_kind, T.M, T.N, T.K, 1);
-      fb += (size_t)std::max(split_bytes(ks, x.data_kind, T.M, T.N, 1, 32), split_bytes(ks, x.data_kind, T.M, T.N, 1, 64)) + 256;
+    } else {
+      fb += batch_part_bytes(k_split(x.data_kind, T.M, T.N, T.K, 1), x.data_kind, T.M, T.N);
     }
   }
   return sizeof(BatchDesc) + sizeof(int32_t) + sizeof(int64_t) + fb + 256;
@@ -2419,7 +2430,12 @@ extern "C" int tcTensorContractBatchTune(int ntasks, const tcContractTask *tasks
                                          size_t scratch_bytes, void *stream, int reps) {
   using namespace tb;
   if (ntasks < 0 || (ntasks > 0 && tasks == nullptr) || reps < 1) return TALSH_INVALID_ARGS;
-  if (scratch_bytes < tcTensorContractBatchScratch(ntasks, tasks)) return TALSH_INVALID_ARGS;
+  {  // as tcTensorContractBatch: partial sums are optional, and both edges have them or neither
+    BatchPlan bp;
+    const std::vector<char> lean((size_t)ntasks, 1);
+    if (ntasks > 0 && (batch_plan(ntasks, tasks, bp, &lean) != TALSH_SUCCESS || scratch_bytes < bp.total))
+      return TALSH_INVALID_ARGS;
+  }
   std::vector<int> cls[2][kTuneBuckets][kTuneBuckets];
   for (int t = 0; t < ntasks; ++t) {
     const tcContractTask &x = tasks[t];

@@ -184,8 +184,8 @@ def test_autotune_chooses_tiles_and_keeps_results(talsh):
         tuned = [lib.tcTensorContractBatchTuned(k, mb, nb) for k in (T.R8, T.C8) for mb in range(4) for nb in range(4)]
         assert set(tuned) <= {0, 32, 64} and any(t in (32, 64) for t in tuned), tuned
         assert lib.tcTensorContractBatchTuned(T.R4, 0, 0) == -1
-        # a fresh batch after tuning equals one tcTensorContract per task (the
-        # scratch size depends on the tiles chosen: query it again)
+        # a fresh batch after tuning equals one tcTensorContract per task; its
+        # scratch does not depend on the tiles chosen
         tasks, keep = build(specs, 2)
         need = lib.tcTensorContractBatchScratch(len(specs), tasks)
         sc = torch.empty(need, dtype=torch.uint8, device="cuda")
@@ -207,6 +207,42 @@ def test_autotune_chooses_tiles_and_keeps_results(talsh):
         lib.tcTensorContractBatchTuneReset()
     assert all(lib.tcTensorContractBatchTuned(k, mb, nb) == 0 for k in (T.R8, T.C8) for mb in range(4)
                for nb in range(4))
+
+
+@pytest.mark.parametrize("kind", [T.R8, T.C8])
+def test_tuning_long_ranges_keeps_the_scratch(talsh, kind):
+    """Split contracted ranges, whose partial sums differ in size between the tile edges: the scratch query answers the
+    same before and after tuning, tuning takes any scratch that a batch takes, and the bits stay."""
+    torch = pytest.importorskip("torch")
+    lib, rng = T.lib(), np.random.default_rng(31)
+    s = torch.cuda.current_stream().cuda_stream
+    shapes = [(20, 20, 5000), (33, 17, 3001), (10, 60, 4000), (70, 9, 2000)]
+    tasks, keep = (T.ContractTask * len(shapes))(), []
+    for t, (m, n, k) in zip(tasks, shapes):
+        l, r = (torch.from_numpy(rnd(rng, x, kind).ravel(order="F").copy()).cuda() for x in ([k, m], [n, k]))
+        d = torch.empty(m * n, dtype=l.dtype, device="cuda")
+        t.data_kind, t.drank, t.lrank, t.rrank = kind, 2, 2, 2
+        for to, v in ((t.cptrn, [-2, 1, 2, -1]), (t.ddims, [m, n]), (t.ldims, [k, m]), (t.rdims, [n, k])):
+            for i, x in enumerate(v):
+                to[i] = x
+        t.D, t.L, t.R, t.alpha_re, t.accumulative = d.data_ptr(), l.data_ptr(), r.data_ptr(), 1.0, 0
+        keep.append((l, r, d))
+    lib.tcTensorContractBatchTuneReset()
+    try:
+        need = lib.tcTensorContractBatchScratch(len(shapes), tasks)
+        buf = torch.empty(need, dtype=torch.uint8, device="cuda")
+        assert lib.tcTensorContractBatch(len(shapes), tasks, buf.data_ptr(), need, s) == 0
+        torch.cuda.synchronize()
+        first = [d.clone() for _, _, d in keep]
+        for size in (need, need - 256):
+            assert lib.tcTensorContractBatchTune(len(shapes), tasks, buf.data_ptr(), size, s, 1) == 0
+            assert lib.tcTensorContractBatchScratch(len(shapes), tasks) == need
+            assert lib.tcTensorContractBatch(len(shapes), tasks, buf.data_ptr(), size, s) == 0
+            torch.cuda.synchronize()
+            assert all(torch.equal(d, f) for (_, _, d), f in zip(keep, first))
+        assert lib.tcTensorContractBatchTune(len(shapes), tasks, buf.data_ptr(), 4096, s, 1) == T.TALSH_INVALID_ARGS
+    finally:
+        lib.tcTensorContractBatchTuneReset()
 
 
 def test_batch_graph_replays_equal_the_batch(talsh):
