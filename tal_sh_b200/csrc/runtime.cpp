@@ -155,6 +155,19 @@ int dev_alloc(int gpu, size_t bytes, void **p) {
   return TALSH_SUCCESS;
 }
 
+// Scratch of a contraction: `bytes`, or `least` (0: none) where the pool has no
+// more; the task is deferred only when that fails too.
+int scratch_alloc(int gpu, size_t &bytes, size_t least, void **p) {
+  const unsigned long long deferred = R.gpu[gpu].try_later;
+  int rc = dev_alloc(gpu, bytes, p);
+  if (rc != TALSH_SUCCESS && least > 0 && least < bytes) {
+    R.gpu[gpu].try_later = deferred;
+    bytes = least;
+    rc = dev_alloc(gpu, bytes, p);
+  }
+  return rc;
+}
+
 // Frees library-owned memory (host or device); unknown pointers are ignored.
 int mem_free(void *p) {
   if (p == nullptr) return TALSH_SUCCESS;
@@ -647,11 +660,7 @@ int schedule(OpSpec &op, int dev_id, int dev_kind, talsh_task_t *user_task) {
     scratch = tcTensorNorm1Scratch(shape_volume(op.t[0]->shape_p)) + 256;
   }
   if (scratch > 0) {
-    int rc = dev_alloc(gpu, scratch, &tr->scratch);
-    if (rc != TALSH_SUCCESS && scratch_least > 0 && scratch_least < scratch) {
-      scratch = scratch_least;
-      rc = dev_alloc(gpu, scratch, &tr->scratch);
-    }
+    const int rc = scratch_alloc(gpu, scratch, scratch_least, &tr->scratch);
     if (rc != TALSH_SUCCESS) {
       for (int j = 0; j < op.nt; ++j) if (tr->a[j].dalloc) mem_free(tr->a[j].dptr);
       delete tr;
@@ -2514,13 +2523,7 @@ int talshTensorContractXL(const char *cptrn, talsh_tens_t *d, talsh_tens_t *l, t
   };
   cudaSetDevice(gpu);
   for (int a = 0; a < 3 && rc == TALSH_SUCCESS; ++a) rc = dev_alloc(gpu, bb[a], &db[a]);
-  if (rc == TALSH_SUCCESS && scratch_bytes) {
-    rc = dev_alloc(gpu, scratch_bytes, &scr);
-    if (rc != TALSH_SUCCESS && scratch_least < scratch_bytes) {
-      scratch_bytes = scratch_least;
-      rc = dev_alloc(gpu, scratch_bytes, &scr);
-    }
-  }
+  if (rc == TALSH_SUCCESS && scratch_bytes) rc = scratch_alloc(gpu, scratch_bytes, scratch_least, &scr);
   for (int a = 0; a < 3 && rc == TALSH_SUCCESS; ++a) {
     const size_t whole = shape_volume(ts[a]->shape_p) * (size_t)es;
     mp[a] = xl_map(hp[a], whole, reg[a]);

@@ -121,7 +121,7 @@ def test_split_k_with_hyper_indices(talsh):
 @pytest.mark.parametrize("kind,xl,dims", [(T.R8, 0, (40, 33, 20001)), (T.R4, 0, (40, 33, 20001)), (T.R4, 1, (2, 3, 230000))])
 def test_short_device_memory_changes_no_bits(kind, xl, dims):
     """talshTensorContract and the out-of-core form in a pool that holds the operands and the offset tables but not
-    the partial sums: the bits of a roomy pool."""
+    the partial sums: the bits of a roomy pool, and no deferred task on record."""
     code = r"""
 import ctypes as C, hashlib, sys
 import numpy as np
@@ -157,6 +157,6 @@ assert L.talshShutdown() == 0
     for budget in (1 << 30, short + 4096):
         p = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, TALSH_B200_GPU_BUDGET_BYTES=str(budget)),
                            stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True, timeout=300)
-        assert p.returncode == 0, p.stdout
+        assert p.returncode == 0 and " deferred 0;" in p.stdout, p.stdout
         sums.append([x for x in p.stdout.splitlines() if x.startswith("sum")])
     assert len(sums[0]) == 1 and sums[0] == sums[1]
