@@ -1317,8 +1317,8 @@ size_t contract_split_scratch(int kind, const int *cptrn, int drank, const int *
 
 namespace {
 
-// Which GEMM runs: the CTA-pair kernel (256 x 256 tiles) when its tiles give
-// every SM work (two CTAs per tile), else the single-CTA kernel (128 x 128
+// Which GEMM runs: the CTA-pair kernel (tiles of 256 rows by up to 256 columns)
+// when 256 x 256 tiles give every SM work (two CTAs per tile), else the single-CTA kernel (128 x 128
 // tiles, four times as many); TALSH_B200_SPLIT_PAIR=1 / 0 forces one.
 int split_pair_mode() {
   static const int v = [] {
@@ -1365,18 +1365,29 @@ int launch_pair_form(const CUtensorMap &mapA, const CUtensorMap &mapB, OzPairArg
 }
 
 // Tile width of the CTA-pair kernel: the one with the least time for the
-// fullest pair of SMs, waves x (columns + 16 for a tile's epilogue and start).
+// fullest pair of SMs, waves x (columns + 128 for what a tile costs at any width:
+// its rows of A, its passes' epilogues, its start).  Over 28 shapes and all five
+// widths any constant from 64 to 320 chooses within 0.7 % of the fastest; 16, the
+// epilogue's share alone, lost up to 15 % where narrow tiles cost another wave
+// (3264 x 3465, K = 3311, int8: 160-wide 1436 us, 224-wide 1269, 256-wide 1346).
 // 2640 x 2805: 121 256-wide tiles are two waves on 74 pairs, 143 224-wide ones
-// too, 12 % less work each (801 -> 757 us for the whole contraction, K = 2480,
+// too, 12 % less work each (810 -> 773 us for the whole contraction, K = 2480,
 // six int8 slices).
 // Rows of B beyond N belong to the next slice or are zero-filled past the
 // last; they only reach columns that are not stored.
+// TALSH_B200_SPLIT_PAIR_N=128, 160, 192, 224 or 256 forces one.
 int pair_tile_n(int64_t Mp, int64_t N) {
+  static const int forced = [] {
+    const char *e = std::getenv("TALSH_B200_SPLIT_PAIR_N");
+    const int v = e ? std::atoi(e) : 0;
+    return v >= 128 && v <= kPairBN && v % 32 == 0 ? v : 0;
+  }();
+  if (forced) return forced;
   const int64_t pairs = std::max(1, current_sm_count() / 2), tm = Mp / 256;
   int best = kPairBN;
   int64_t least = 0;
   for (int nt = kPairBN; nt >= 128; nt -= 32) {
-    const int64_t cost = (tm * ((N + nt - 1) / nt) + pairs - 1) / pairs * (nt + 16);
+    const int64_t cost = (tm * ((N + nt - 1) / nt) + pairs - 1) / pairs * (nt + 128);
     if (nt == kPairBN || cost < least) { least = cost; best = nt; }
   }
   return best;

@@ -217,9 +217,9 @@ def test_split_complex_through_talsh_contract(talsh):
 
 
 def test_cta_pair_kernel_accuracy(talsh):
-    """The CTA-pair kernel (TALSH_B200_SPLIT_PAIR=1: cta_group::2 MMAs of
-    256 x 256 over a 2-CTA cluster), in a child process, meets the same bound
-    on every case, real and complex."""
+    """The CTA-pair kernel (TALSH_B200_SPLIT_PAIR=1: cta_group::2 MMAs over a
+    2-CTA cluster; 256 x 128 tiles, the width chosen for shapes of one wave), in
+    a child process, meets the same bound on every case, real and complex."""
     import os
     import subprocess
     import sys
@@ -243,3 +243,37 @@ print("ERR", t._run(torch, "D(a,b)+=L(a,k)*R(k,b)", dict(a=130, b=70, k=200), 6,
     errs = [float(line.split()[1]) for line in p.stdout.splitlines() if line.startswith("ERR ")]
     assert len(errs) == len(CASES) + len(COMPLEX_CASES) + 1, p.stdout
     assert max(errs) <= TOL_SPLIT6, errs
+
+
+@pytest.mark.parametrize("width", [128, 160, 192, 224, 256])
+def test_cta_pair_tile_widths(talsh, width):
+    """Every tile width of the CTA-pair kernel, in a child process: the int8 form and a bf16 one within their bounds,
+    the int8 one with the errors of the 256-wide tiles to the last digit (exact int32 sums, recombined in the
+    same order), with N below, at, just past and not a multiple of the width."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    code = r"""
+import sys
+sys.path.insert(0, %r); sys.path.insert(0, %r)
+import torch
+import test_split_forms_gpu as f
+import test_split_gpu as t
+w = %d
+for n in (w - 1, w, w + 1, 2 * w + 37, 333):
+    print("ERR", t._run(torch, "D(a,b)+=L(a,k)*R(k,b)", dict(a=300, b=n, k=200), 6))
+print("ERR", t._run(torch, "D(a,b)+=L(a,k)*R(k,b)", dict(a=130, b=w + 3, k=200), 6, alpha=-0.75, acc=False,
+                    scale_rows=True))
+print("ERRF", f._run(torch, "D(a,b)+=L(a,k)*R(k,b)", dict(a=300, b=2 * w + 37, k=300), "bf16", 3))
+""" % (root, os.path.join(root, "tests"), width)
+    errs = []
+    for n in (width, 256):
+        env = dict(TALSH_B200_SPLIT_PAIR="1", TALSH_B200_SPLIT_PAIR_N=str(n))
+        p = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, **env), stdout=subprocess.PIPE,
+                           stderr=subprocess.STDOUT, text=True, timeout=600)
+        assert p.returncode == 0, p.stdout
+        errs.append([x.split() for x in p.stdout.splitlines() if x.startswith("ERR")])
+    assert len(errs[0]) == 7 and max(float(e) for k, e in errs[0] if k == "ERR") <= TOL_SPLIT6, errs
+    assert max(float(e) for k, e in errs[0] if k == "ERRF") <= 5e-6, errs
+    assert [e for k, e in errs[0] if k == "ERR"] == [e for k, e in errs[1] if k == "ERR"], errs
