@@ -160,3 +160,44 @@ assert L.talshShutdown() == 0
         assert p.returncode == 0 and " deferred 0;" in p.stdout, p.stdout
         sums.append([x for x in p.stdout.splitlines() if x.startswith("sum")])
     assert len(sums[0]) == 1 and sums[0] == sums[1]
+
+
+# 128 x 128 R4 tiles (at least two per SM): K whole, and cut in two; both remainders
+@pytest.mark.parametrize("m,n,k", [(2209, 2241, 300), (4665, 957, 4001)])
+def test_large_r4_tiles(talsh, m, n, k):
+    """The wide R4 tiles against 64 bits for both load directions of both operands, accumulating and overwriting, and
+    bit for bit against a batch (64 x 64 tiles)."""
+    torch = pytest.importorskip("torch")
+    lib = T.lib()
+    g = torch.Generator(device="cuda")
+    g.manual_seed(17)
+    s = torch.cuda.current_stream().cuda_stream
+    mk = lambda *x: torch.rand(*x, device="cuda", generator=g).mul_(2.0).sub_(1.0)  # noqa: E731
+    for l_along_k, r_along_k, acc in [(0, 0, 1), (1, 1, 0), (0, 1, 0), (1, 0, 1)]:
+        # row-major (cols, rows) is the column-major (rows, cols) body
+        l, r, d0 = mk(m, k) if l_along_k else mk(k, m), mk(n, k) if r_along_k else mk(k, n), mk(n, m)
+        ld, rd = ([k, m] if l_along_k else [m, k]), ([k, n] if r_along_k else [n, k])
+        cptrn = ([-(1 if r_along_k else 2), 1] if l_along_k else [1, -(1 if r_along_k else 2)]) + \
+            ([-(1 if l_along_k else 2), 2] if r_along_k else [2, -(1 if l_along_k else 2)])
+        args = (T.R4, T.ivec(cptrn), 2, T.ivec([m, n]), 2, T.ivec(ld), 2, T.ivec(rd))
+        need = lib.tcTensorContractScratch(*args)
+        assert (need > (16 * (m + n + k) + 255) // 256 * 256) == (k > 1000)  # cut or whole
+        buf = torch.empty(need, dtype=torch.uint8, device="cuda")
+        d, d2 = d0.clone(), d0.clone()
+        assert lib.tcTensorContract(*args, d.data_ptr(), l.data_ptr(), r.data_ptr(), 0.5, 0.0, 0, acc, buf.data_ptr(),
+                                    need, s) == 0
+        a, b = (l if l_along_k else l.T).double(), (r if r_along_k else r.T).double()
+        ref = 0.5 * (b @ a.T) + (d0.double() if acc else 0.0)
+        assert float(torch.linalg.norm(d.double() - ref) / torch.linalg.norm(ref)) <= TOL[T.R4]
+        t = (T.ContractTask * 1)()
+        t[0].data_kind, t[0].drank, t[0].lrank, t[0].rrank = T.R4, 2, 2, 2
+        for to, v in ((t[0].cptrn, cptrn), (t[0].ddims, [m, n]), (t[0].ldims, ld), (t[0].rdims, rd)):
+            for i, x in enumerate(v):
+                to[i] = x
+        t[0].D, t[0].L, t[0].R = d2.data_ptr(), l.data_ptr(), r.data_ptr()
+        t[0].alpha_re, t[0].accumulative = 0.5, acc
+        need = lib.tcTensorContractBatchScratch(1, t)
+        buf = torch.empty(need, dtype=torch.uint8, device="cuda")
+        assert lib.tcTensorContractBatch(1, t, buf.data_ptr(), need, s) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(d, d2)

@@ -133,3 +133,30 @@ def test_slice_insert_units(talsh, kind):
                 torch.cuda.synchronize()
                 assert rc == 0 and bufs[1].cpu().numpy().tobytes() == ref.tobytes(order="F"), (full, sl, off, shift,
                                                                                                   insert, acc)
+
+
+def test_slice_insert_past_32_bits(talsh):
+    """More than 2^31 one-element units (64-bit unit numbers): a 2 x 1100000000 R4 slice of a 3 x 1100000001 tensor and
+    its insertion, bit-exact."""
+    torch = pytest.importorskip("torch")
+    L, n = T.lib(), 1100000000
+    s = torch.cuda.current_stream().cuda_stream
+    full = torch.empty(3 * (n + 1), dtype=torch.int32, device="cuda")
+    step = 1 << 27
+    pieces = range(0, n, step)  # filled and compared in pieces: the temporaries stay small
+    for lo in range(0, full.numel(), step):
+        hi = min(lo + step, full.numel())
+        full[lo:hi] = torch.arange(lo, hi, device="cuda") % 2000000011
+    part = torch.zeros(2 * n, dtype=torch.int32, device="cuda")
+    args = (T.R4, 2, T.ivec([3, n + 1]), T.ivec([2, n]), T.ivec([1, 0]))
+    assert L.tcTensorSlice(*args, full.data_ptr(), part.data_ptr(), 0, s) == 0
+    want = full.view(n + 1, 3)[:n, 1:]
+    got = part.view(n, 2)
+    assert all(torch.equal(got[lo:lo + step], want[lo:lo + step]) for lo in pieces)
+    part.bitwise_not_()
+    assert L.tcTensorInsert(*args, part.data_ptr(), full.data_ptr(), 0, s) == 0
+    rows = full.view(n + 1, 3)
+    for lo in pieces:
+        hi = min(lo + step, n)
+        assert torch.equal(rows[lo:hi, 1:], got[lo:hi])
+        assert torch.equal(rows[lo:hi, 0].long(), torch.arange(3 * lo, 3 * hi, 3, device="cuda") % 2000000011)
