@@ -1383,10 +1383,21 @@ int build_plan(int esize, const Fused &F, Plan &plan, int op = kOpCopy, const Pl
   // times as fast; 279 x 37 x 196 x 31 R8: 256 -> 200 us).  Plans with vector
   // output are left alone: they pay less per slot, and one lost 11 %.  Scalars
   // only, a few microseconds of planning, and only where the copy takes longer.
-  if (F.vol >= (1 << 21) && cfg.grow < 0 && cfg.longrun == 0 && !cfg.small && vec_width(G, nb) == 1) {
+  // The result is taken where it saves enough slots (330 random shapes per
+  // launch, both tiles; a smaller saving does not pay for the output runs it
+  // cuts off the 32-lane grid): 15 % for adds and for copies read element by
+  // element, of which none then lost (geometric mean 1.09-1.17; without the
+  // line down to 0.92).  Bulk-read copies spend less per slot: of 8-byte ones
+  // those whose runs share no dimension and that save 45 % (1.15, worst 0.99;
+  // without the line 0.86), 16-byte ones never (1.01 on average, worst 0.85).
+  const bool bulk_copy =
+      op != kOpAdd && (cfg.bulk < 0 ? permute_bulk_wanted(esize, op, 1) : cfg.bulk == 1);
+  const bool shared_runs = G.V < G.Li * G.Lo;  // a dimension in both groups
+  if (F.vol >= (1 << 21) && cfg.grow < 0 && cfg.longrun == 0 && !cfg.small && vec_width(G, nb) == 1 &&
+      !(bulk_copy && (esize >= 16 || shared_runs))) {
+    auto slots = [&](double V) { return V <= kThreads * 4 ? kThreads * 4.0 : kThreads * 8.0; };
     auto cost = [&](double tiles, double V, double Li, double Lo) {
-      const double slots = V <= kThreads * 4 ? kThreads * 4 : kThreads * 8;
-      return 0.3 * tiles * slots / (double)F.vol + 32.0 / (Li * esize) + (op == kOpAdd ? 2.0 : 1.0) * 32.0 / (Lo * esize);
+      return 0.3 * tiles * slots(V) / (double)F.vol + 32.0 / (Li * esize) + (op == kOpAdd ? 2.0 : 1.0) * 32.0 / (Lo * esize);
     };
     double tiles = 1.0;
     for (int i = 0; i < n; ++i) tiles *= (double)((P.ext[i] + G.tl[i] - 1) / G.tl[i]);
@@ -1432,7 +1443,9 @@ int build_plan(int esize, const Fused &F, Plan &plan, int op = kOpCopy, const Pl
       Geo X;
       geometry(best_a, best_ta, best_b, best_tb, X);
       cur_na = best_a; cur_nb = best_b;
-      if (acceptable(X)) { G = X; na = best_a; nb = best_b; }
+      double fewer = tiles * slots((double)G.V) / slots((double)X.V);
+      for (int i = 0; i < n; ++i) fewer /= (double)((P.ext[i] + X.tl[i] - 1) / X.tl[i]);
+      if (acceptable(X) && fewer >= (bulk_copy ? 1.45 : 1.15)) { G = X; na = best_a; nb = best_b; }
       cur_na = na; cur_nb = nb;
     }
   }

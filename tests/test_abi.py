@@ -420,6 +420,21 @@ def test_transpose_plan_invariants(built):
     assert n_tiled > 1000
 
 
+@pytest.mark.parametrize("kind,dims,o2n,tile,runs", [
+    (T.C8, [903, 75, 93, 6], [2, 4, 1, 3], 651, (21, 31)),        # 16-byte copies keep the grown tile
+    (T.R8, [55, 818099], [2, 1], 1760, (55, 32)),                 # 8-byte: too few slots saved
+    (T.R8, [29, 8, 191, 525], [1, 4, 2, 3], 1160, (232, 145)),    # 8-byte: a dimension in both runs
+    (T.R4, [677, 70951], [2, 1], 1984, (62, 32)),                 # 4-byte: too few slots saved
+    (T.R8, [279, 37, 196, 31], [3, 1, 4, 2], 1924, (26, 74)),     # refined
+    (T.C4, [385, 48877], [2, 1], 2035, (55, 37)),                 # refined
+    (T.R4, [35, 15, 7, 11661], [2, 1, 4, 3], 1575, (525, 1575))])  # refined
+def test_tile_refinement_only_where_it_pays(built, kind, dims, o2n, tile, runs):
+    """Tile and run lengths of shapes timed both ways: the refined tile only where it was the faster one."""
+    info = (C.c_int * 12)()
+    assert T.lib().tcPermutePlanInfo(kind, len(dims), T.ivec(dims), T.ivec(o2n), info) == 0
+    assert (info[2], (info[3], info[4])) == (tile, runs)
+
+
 def test_contraction_scratch_queries_on_malformed_and_valid_patterns(built):
     """Host-side pattern analysis without a GPU: random (mostly malformed) digital
     patterns are analysed without crashing; valid random contractions get
