@@ -122,10 +122,11 @@ struct PermParams {
   int64_t istr[kMaxFR];
   int64_t ostr[kMaxFR];
   int64_t ntile[kMaxFR];
-  uint32_t mg_ts[kMaxFR], sh_ts[kMaxFR];  // magic divisors of the tile-index stride of each dimension
-  uint32_t mg_nt[kMaxFR], sh_nt[kMaxFR];  // and of its tile count
+  uint32_t mg_ts[kMaxFR];  // magic divisors of the tile-index stride of each dimension,
+  uint32_t mg_nt[kMaxFR];  // of its tile count
+  uint32_t mg_tl[kMaxFR];  // and of its tile extent
+  uint8_t sh_ts[kMaxFR], sh_nt[kMaxFR], sh_tl[kMaxFR];  // bytes: a small copy's launch pays for its parameters
   int32_t tl[kMaxFR];
-  uint32_t mg_tl[kMaxFR], sh_tl[kMaxFR];  // magic divisors of the tile extents
   uint32_t mg_ap, sh_ap, mg_bp, sh_bp;    // of a_pre, b_pre
   uint32_t mg_ba, sh_ba, mg_ab, sh_ab;    // of pre_bA, pre_aB
   int32_t smstr[kMaxFR];
@@ -142,11 +143,11 @@ struct TileSetup {
 };
 
 // Fast unsigned division for n < 2^31 (Granlund-Montgomery round-up method).
-void make_magic(uint32_t d, uint32_t &mg, uint32_t &sh) {
-  uint32_t s = 0;
-  while ((1ull << s) < d) ++s;
-  mg = (uint32_t)(((1ull << 32) * ((1ull << s) - d)) / d + 1ull);
-  sh = s;
+template <typename S>
+void make_magic(uint32_t d, uint32_t &mg, S &sh) {
+  const uint32_t s = d > 1 ? 32 - __builtin_clz(d - 1) : 0;  // ceil(log2 d)
+  mg = d > 1 ? (uint32_t)(((1ull << 32) * ((1ull << s) - d)) / d + 1ull) : 1u;
+  sh = (S)s;
 }
 __device__ __forceinline__ uint32_t fast_div(uint32_t n, uint32_t mg, uint32_t sh) {
   return (__umulhi(n, mg) + n) >> sh;
