@@ -65,3 +65,28 @@ def test_full_contraction(talsh, kind):
             run(dims, perm, conj if kind in (T.C4, T.C8) else 0, conj // 2 % 2)
         if kind != T.C8:  # bodies aligned to the element only
             run(dims, perm, 0, 1, offset=1)
+
+
+def test_long_sums_are_summed_in_parts(talsh):
+    """Rounding of 41 M products, 8 draws.  A thread adds about 270 of them: in one chain the error is about
+    0.6 u sqrt(n v 270 / 2), v = 1/9 the products' variance (2.6e-16 sqrt(n)); as sums of 8 and then of those, about
+    1e-16 sqrt(n).  The line lies at their geometric mean."""
+    torch = pytest.importorskip("torch")
+    lib = T.lib()
+    dims = [80, 64, 100, 80]  # D += L(a,b,i,j) R(b,a,i,j)
+    n = int(np.prod(dims))
+    args = (T.R8, T.ivec([-2, -1, -3, -4, -2, -1, -3, -4]), 0, None, 4, T.ivec(dims), 4, T.ivec([64, 80, 100, 80]))
+    need = lib.tcTensorContractScratch(*args)
+    buf = torch.empty(need, dtype=torch.uint8, device="cuda")
+    square = 0.0
+    for seed in range(8):
+        g = torch.Generator(device="cuda")
+        g.manual_seed(seed)
+        l, r = (torch.rand(n, dtype=torch.float64, device="cuda", generator=g).mul_(2.0).sub_(1.0) for _ in range(2))
+        d = torch.zeros(1, dtype=torch.float64, device="cuda")
+        assert lib.tcTensorContract(*args, d.data_ptr(), l.data_ptr(), r.data_ptr(), 1.0, 0.0, 0, 0, buf.data_ptr(),
+                                    need, torch.cuda.current_stream().cuda_stream) == 0
+        x = l.view(80, 100, 64, 80).cpu().numpy().astype(np.longdouble)
+        x *= r.view(80, 100, 80, 64).transpose(2, 3).cpu().numpy()
+        square += float((d.cpu().numpy()[0] - x.sum()) ** 2) / n / 8
+    assert np.sqrt(square) <= 1.6e-16, np.sqrt(square)
