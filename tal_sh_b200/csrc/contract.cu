@@ -446,8 +446,11 @@ __device__ __forceinline__ void dmma_tile(const double *__restrict__ L, const do
   using Int3 = std::integral_constant<int, 3>;
   constexpr int FM = C::WM / 8, FN = C::WN / 8;
   double2 acc[FM * FN];
-  // Ragged tiles give the low warp positions more fragments; rotating the
-  // positions by CTA spreads them over the SM's four tensor pipes.
+  // Ragged tiles give the low warp positions more fragments; the positions turn
+  // with the CTA's number.  CTAs of one launch that share an SM are mostly a
+  // multiple of 148 = 4 x 37 apart and turn alike, so little comes of it: 40 x 40
+  // outputs 167.4 -> 165.7 us, batch of 768 4324 -> 4302.  (Turning by the number
+  // over 148 as well, 162 -> 177 us, was not kept.)
   const int wr = (warp + w.lin + w.split) % (C::WARPS_M * C::WARPS_N);
   const int wm = wr % C::WARPS_M, wn = wr / C::WARPS_M;
   const int fr = lane >> 2, fc = lane & 3;
@@ -622,8 +625,7 @@ __device__ __forceinline__ void zmma_tile(const double2 *__restrict__ L, const d
   using Int3 = std::integral_constant<int, 3>;
   constexpr int FM = C::WM / 8, FN = C::WN / 8;
   double2 acc[2 * FM * FN];  // fragment f: real parts at 2 f, imaginary parts at 2 f + 1
-  // Ragged tiles give the low warp positions more fragments; rotating the
-  // positions by CTA spreads them over the SM's four tensor pipes.
+  // Warp positions turn with the CTA's number, as in the real tile.
   const int wr = (warp + w.lin + w.split) % (C::WARPS_M * C::WARPS_N);
   const int wm = wr % C::WARPS_M, wn = wr / C::WARPS_M;
   const int fr = lane >> 2, fc = lane & 3;
@@ -803,7 +805,7 @@ __device__ __forceinline__ float2 unpack2(uint64_t v) {
 template <typename T, int BM, int BN>
 struct FmmaCfg {
   static constexpr int VE = 16 / (int)sizeof(T);
-  static constexpr int MC = sizeof(T) == 4 || BM <= 32 ? 2 : 4, NC = 2;
+  static constexpr int MC = (sizeof(T) == 4 ? 2 : 4) / (BM <= 32 ? 2 : 1), NC = sizeof(T) == 4 && BN <= 32 ? 1 : 2;
   static constexpr int TMN = BM / (MC * VE), TNN = BN / (NC * VE);  // threads along m and n
   static constexpr int THREADS = TMN * TNN;
   static constexpr int BK = 16, STAGES = 3;
@@ -1024,6 +1026,7 @@ __device__ __forceinline__ void fmma_tile(const T *__restrict__ L, const T *__re
 template <typename T, int BM> struct FmmaOcc { static constexpr int N = 4; };
 template <> struct FmmaOcc<float, 64> { static constexpr int N = 6; };  // 7: 5 % slower (spills)
 template <> struct FmmaOcc<float, 128> { static constexpr int N = 2; };
+template <> struct FmmaOcc<float, 32> { static constexpr int N = 16; };
 template <> struct FmmaOcc<float2, 32> { static constexpr int N = 8; };
 
 template <typename T, int BM, int BN, bool SEQ>
@@ -1407,11 +1410,16 @@ int64_t split_bytes(const KSplit &s, int kind, int64_t M, int64_t N, int64_t H, 
 // leave eight CTAs per SM to hide a k step's latency behind (64 / 32, us: 18
 // tiles of 64, K = 169: 55 / 25, 45 before the packed kernel; 105 tiles, K =
 // 459: 125 / 76; 131000 x 1, K = 20: 98 / 53; 3000 x 3000 x 3000: 5847 / 5799).
-// R4: 128 when two of those per SM exist and are mostly filled, else 64.
-// Results do not depend on it.
+// R4: 32 (4 x 4 sub-tiles) when one side is no wider, or when 64 x 64 tiles are
+// fewer than three for two SMs (64 / 32, us: 131000 x 1, K = 20: 37 / 23; 300 x
+// 300, K = 30: 18.4 / 11.1, 13.0 before the packed kernel; 512 x 512, K = 400: 41
+// / 25; 900 x 900 x 900, 225 tiles: 77 / 70 and, loads along k, 78 / 86), else 128
+// when two of those per SM exist and are mostly filled, else 64.  Results do not
+// depend on it.
 int gemm_edge(int kind, int64_t M, int64_t N, int64_t H, const KSplit &s) {
   auto tiles = [&](int64_t e) { return ((M + e - 1) / e) * ((N + e - 1) / e) * std::max<int64_t>(H, 1); };
   const int64_t sms = sm_count_dev();
+  if (kind == R4 && (std::min(M, N) <= 32 || 2 * tiles(64) * s.nsplit < 3 * sms)) return 32;
   if (kind == R4) return tiles(128) >= 2 * sms && tiles(64) >= 3 * tiles(128) ? 128 : 64;
   if (kind == C4) return 32;
   return tiles(64) * s.nsplit >= sms ? 64 : 32;
@@ -1714,7 +1722,8 @@ int contract_launch(int kind, const int *cptrn, int drank, const int *ddims, int
     }
     case R4:
       if (edge == 128) return launch_fmma<float, 128, 128>(L, R, D, ga, st);
-      return launch_fmma<float, 64, 64>(L, R, D, ga, st);
+      if (edge == 64) return launch_fmma<float, 64, 64>(L, R, D, ga, st);
+      return launch_fmma<float, 32, 32>(L, R, D, ga, st);
     case C4: return launch_fmma<float2, 32, 32>(L, R, D, ga, st);
     default:
       if (edge == 64) return launch_zmma<64, 64>((const double2 *)L, (const double2 *)R, (double2 *)D, ga, st);

@@ -118,7 +118,8 @@ def test_split_k_with_hyper_indices(talsh):
     assert torch.equal(d, d2)
 
 
-@pytest.mark.parametrize("kind,xl,dims", [(T.R8, 0, (40, 33, 20001)), (T.R4, 0, (40, 33, 20001)), (T.R4, 1, (2, 3, 230000))])
+@pytest.mark.parametrize("kind,xl,dims", [(T.R8, 0, (40, 33, 20001)), (T.R4, 0, (40, 33, 20001)),
+                                          (T.R4, 1, (1, 1, 230000))])
 def test_short_device_memory_changes_no_bits(kind, xl, dims):
     """talshTensorContract and the out-of-core form in a pool that holds the operands and the offset tables but not
     the partial sums: the bits of a roomy pool, and no deferred task on record."""
