@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <cstring>
 
 #include "common.h"
@@ -35,6 +36,7 @@ struct SliceParams {
   int64_t run;                    // contiguous units per run
   int64_t total;                  // units of the slice
   int64_t base;                   // full-tensor offset of the slice origin
+  int64_t full;                   // units of the full tensor
   int64_t rext[kMaxRank];         // slice extents of the run dimensions
   int64_t rstr[kMaxRank];         // full-tensor strides of the run dimensions
   uint32_t mg_run, sh_run, mg[kMaxRank], sh[kMaxRank];  // magic divisors (totals below 2^31)
@@ -42,9 +44,8 @@ struct SliceParams {
 
 // Round-up magic division of n < 2^31 (Granlund and Montgomery).
 void magic(int64_t d, uint32_t &mg, uint32_t &sh) {
-  uint32_t s = 0;
-  while ((1ull << s) < (uint64_t)d) ++s;
-  mg = (uint32_t)(((1ull << 32) * ((1ull << s) - (uint64_t)d)) / (uint64_t)d + 1ull);
+  const uint32_t s = d > 1 ? 64 - __builtin_clzll((uint64_t)d - 1) : 0;  // ceil(log2 d)
+  mg = d > 1 ? (uint32_t)(((1ull << 32) * ((1ull << s) - (uint64_t)d)) / (uint64_t)d + 1ull) : 1u;
   sh = s;
 }
 __device__ __forceinline__ uint32_t mdiv(uint32_t n, uint32_t mg, uint32_t sh) { return (__umulhi(n, mg) + n) >> sh; }
@@ -52,9 +53,12 @@ __device__ __forceinline__ uint32_t mdiv(uint32_t n, uint32_t mg, uint32_t sh) {
 // A unit: VEC values of a real type (complex values are two).
 template <typename R, int VEC> struct alignas(sizeof(R) * VEC) Unit { R v[VEC]; };
 
-template <bool WIDE>
+// Arithmetic of unit numbers and full-tensor offsets: 32 bits for both, 32 and
+// 64, or 64 for both.
+enum : int { kNarrow = 0, kMixed = 1, kWide = 2 };
+template <int MODE>
 __device__ __forceinline__ int64_t full_offset(const SliceParams &p, int64_t e) {
-  if constexpr (WIDE) {
+  if constexpr (MODE == kWide) {
     int64_t r = e / p.run;
     int64_t off = p.base + (e - r * p.run);
     for (int d = 0; d < p.nrow; ++d) {
@@ -64,19 +68,20 @@ __device__ __forceinline__ int64_t full_offset(const SliceParams &p, int64_t e) 
     }
     return off;
   } else {
+    using O = std::conditional_t<MODE == kNarrow, uint32_t, int64_t>;
     uint32_t r = mdiv((uint32_t)e, p.mg_run, p.sh_run);
-    int64_t off = p.base + ((uint32_t)e - r * (uint32_t)p.run);
-    for (int d = 0; d < p.nrow; ++d) {
+    O off = (O)p.base + ((uint32_t)e - r * (uint32_t)p.run);
+    for (int d = 0; d + 1 < p.nrow; ++d) {
       const uint32_t q = mdiv(r, p.mg[d], p.sh[d]);
-      off += (int64_t)(r - q * (uint32_t)p.rext[d]) * p.rstr[d];
+      off += (O)(r - q * (uint32_t)p.rext[d]) * (O)p.rstr[d];
       r = q;
     }
-    return off;
+    return p.nrow > 0 ? off + (O)r * (O)p.rstr[p.nrow - 1] : off;  // r is below the last extent
   }
 }
 
 // INSERT = false: slice[e] (+)= full[map(e)]; true: full[map(e)] (+)= slice[e].
-template <typename R, int VEC, bool INSERT, bool ACC, bool WIDE>
+template <typename R, int VEC, bool INSERT, bool ACC, int MODE>
 __global__ void __launch_bounds__(kSliceThreads) slice_kernel(const Unit<R, VEC> *__restrict__ src,
                                                               Unit<R, VEC> *dst, const SliceParams p) {
   constexpr int U = 4;
@@ -88,7 +93,7 @@ __global__ void __launch_bounds__(kSliceThreads) slice_kernel(const Unit<R, VEC>
     for (int u = 0; u < U; ++u) {
       const int64_t e = e0 + u * kSliceThreads;
       if (e >= p.total) continue;
-      f[u] = full_offset<WIDE>(p, e);
+      f[u] = full_offset<MODE>(p, e);
       x[u] = src[INSERT ? e : f[u]];
       if (ACC) y[u] = dst[INSERT ? f[u] : e];
     }
@@ -111,8 +116,10 @@ int launch(const void *src, void *dst, const SliceParams &p, cudaStream_t st) {
   const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)current_sm_count() * 32));
   const auto *s = (const Unit<R, VEC> *)src;
   auto *d = (Unit<R, VEC> *)dst;
-  if (p.total >= (int64_t(1) << 31)) slice_kernel<R, VEC, INSERT, ACC, true><<<blocks, kSliceThreads, 0, st>>>(s, d, p);
-  else slice_kernel<R, VEC, INSERT, ACC, false><<<blocks, kSliceThreads, 0, st>>>(s, d, p);
+  const int64_t lim = int64_t(1) << 31;
+  if (p.total >= lim) slice_kernel<R, VEC, INSERT, ACC, kWide><<<blocks, kSliceThreads, 0, st>>>(s, d, p);
+  else if (p.full >= lim) slice_kernel<R, VEC, INSERT, ACC, kMixed><<<blocks, kSliceThreads, 0, st>>>(s, d, p);
+  else slice_kernel<R, VEC, INSERT, ACC, kNarrow><<<blocks, kSliceThreads, 0, st>>>(s, d, p);
   note_launch();
   return check_launch(INSERT ? "tensor insert" : "tensor slice");
 }
@@ -176,9 +183,10 @@ int slice_op(bool insert, int kind, int rank, const int *full_dims, const int *s
   p.run /= vec;
   p.base /= vec;
   p.total /= vec;
+  p.full = stride / vec;
   for (int k = 0; k < p.nrow; ++k) p.rstr[k] /= vec;
   magic(p.run, p.mg_run, p.sh_run);
-  for (int k = 0; k < p.nrow; ++k) magic(p.rext[k], p.mg[k], p.sh[k]);
+  for (int k = 0; k + 1 < p.nrow; ++k) magic(p.rext[k], p.mg[k], p.sh[k]);
   const bool acc = accumulative != 0;
   cudaStream_t st = (cudaStream_t)stream;
   // values per unit: float 1, 2, 4; double 1, 2

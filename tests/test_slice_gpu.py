@@ -153,6 +153,11 @@ def test_slice_insert_past_32_bits(talsh):
     want = full.view(n + 1, 3)[:n, 1:]
     got = part.view(n, 2)
     assert all(torch.equal(got[lo:lo + step], want[lo:lo + step]) for lo in pieces)
+    # few units at offsets past 2^31
+    few = torch.zeros(2 * 1000, dtype=torch.int32, device="cuda")
+    assert L.tcTensorSlice(T.R4, 2, T.ivec([3, n + 1]), T.ivec([2, 1000]), T.ivec([1, n - 999]), full.data_ptr(),
+                           few.data_ptr(), 0, s) == 0
+    assert torch.equal(few.view(1000, 2), full.view(n + 1, 3)[n - 999:, 1:])
     part.bitwise_not_()
     assert L.tcTensorInsert(*args, part.data_ptr(), full.data_ptr(), 0, s) == 0
     rows = full.view(n + 1, 3)
