@@ -286,3 +286,34 @@ def test_device_resource_memory_from_caller_streams(talsh):
     finally:
         L.tensDevRsc_release_all(d)
         assert L.tensDevRsc_destroy(d) == 0
+
+
+@pytest.mark.parametrize("kind", [T.R4, T.R8, T.C4, T.C8])
+def test_init_and_scale_at_every_alignment(talsh, kind):
+    """tcTensorInit / tcTensorScale on bodies that start at each element of a 16-byte unit, of fewer elements than a
+    unit up to more than one unit per thread: every element exact, none beside the body touched."""
+    torch = pytest.importorskip("torch")
+    L, rng = talsh, np.random.default_rng(19)
+    s = torch.cuda.current_stream().cuda_stream
+    unit = max(1, 16 // T.NP_DTYPE[kind]().itemsize)
+    alpha = (0.75, -1.5) if kind in (T.C4, T.C8) else (0.75, 0.0)
+    for n in (1, 2, 3, 4, 5, 7, 8, 9, 255, 1027, 65537, 2500003):
+        for shift in range(unit):
+            x = rand((n + 2 * unit + shift,), kind, rng)
+            lo = unit + shift
+            body = x[lo:lo + n]
+            buf = torch.from_numpy(x.copy()).cuda()
+            at = buf.data_ptr() + lo * x.itemsize
+            assert L.tcTensorScale(kind, n, at, alpha[0], alpha[1], s) == 0
+            want = x.copy()
+            if kind in (T.C4, T.C8):
+                re, im = (body.real.dtype.type(a) for a in alpha)
+                want[lo:lo + n] = (body.real * re - body.imag * im) + 1j * (body.real * im + body.imag * re)
+            else:
+                want[lo:lo + n] = body * body.dtype.type(alpha[0])
+            torch.cuda.synchronize()
+            assert buf.cpu().numpy().tobytes() == want.tobytes(), (n, shift)
+            assert L.tcTensorInit(kind, n, at, 0.25, -0.5, s) == 0
+            want[lo:lo + n] = 0.25 - 0.5j if kind in (T.C4, T.C8) else 0.25
+            torch.cuda.synchronize()
+            assert buf.cpu().numpy().tobytes() == want.tobytes(), (n, shift)
