@@ -994,29 +994,88 @@ __device__ __forceinline__ void fmma_tile(const T *__restrict__ L, const T *__re
     if (!split_combine<NF, NT>(part, mask, tid, a, w.lin, w.split)) return;
     from_units(part);
   }
+  // Epilogue through the stage buffers, so that the lanes of a warp meet D along
+  // its neighbours: straight from the sub-tiles a store filled half of each sector
+  // it touched, which showed where D is most of the traffic (R4, us: outer product
+  // 3000 x 1001 20.2 -> 16.5, 3000 x 3000 at K = 16 42 -> 31, 131000 x 64 at K = 30
+  // 49 -> 35; 3249 x 576 x 3249 307 -> 304).
+  constexpr int CP = BM + VE;                                       // column pitch
+  constexpr int CW = BN * CP <= ST * BK * (AP + BP) ? BN : BN / 2;  // columns per part
+  static_assert(CW * CP <= ST * BK * (AP + BP) && C::TNN * VE <= CW && NT % BM == 0 && NT % CW == 0, "parts fit the stages");
+  T *Cs = As;
   const float alr = (float)a.alpha_re, ali = (float)a.alpha_im;
-#pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    const int ml = row_of(i);
-    if (ml >= mrem) continue;
-    T *p[TN], d[TN];
-#pragma unroll
-    for (int j = 0; j < TN; ++j) {
-      const int nl = col_of(j);
-      p[j] = nl < nrem ? D + mDs[ml] + nDs[nl] : nullptr;
-      d[j] = (a.beta && p[j]) ? *p[j] : T();
+  const bool along_n = nrem > 1 && (mrem <= 1 || nDs[1] - nDs[0] < mDs[1] - mDs[0]);
+  auto emit = [&](T c, T d) {
+    if constexpr (CPLX) {
+      const float vr = c.x * alr - c.y * ali, vi = c.x * ali + c.y * alr;
+      return a.beta ? make_float2(d.x + vr, d.y + vi) : make_float2(vr, vi);
+    } else {
+      const float v = c * alr;
+      return a.beta ? d + v : v;
     }
+  };
+#pragma unroll
+  for (int c0 = 0; c0 < BN; c0 += CW) {
+    __syncthreads();  // every warp is done with the stages, or with the part before
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
-      if (!p[j]) continue;
-      if constexpr (CPLX) {
-        const float2 c = unpack2(acc[i][j]);
-        const float vr = c.x * alr - c.y * ali, vi = c.x * ali + c.y * alr;
-        *p[j] = a.beta ? make_float2(d[j].x + vr, d[j].y + vi) : make_float2(vr, vi);
-      } else {
-        const float2 c = unpack2(acc[i][j / 2]);
-        const float v = ((j & 1) ? c.y : c.x) * alr;
-        *p[j] = a.beta ? d[j] + v : v;
+      if ((j / VE) * (C::TNN * VE) / CW != c0 / CW) continue;
+#pragma unroll
+      for (int i = 0; i < TM; i += VE) {
+        T *to = Cs + (col_of(j) - c0) * CP + row_of(i);
+        if constexpr (CPLX) {
+          *reinterpret_cast<ulonglong2 *>(to) = make_ulonglong2(acc[i][j], acc[i + 1][j]);
+        } else {
+          float4 v;
+          float *e = &v.x;
+#pragma unroll
+          for (int q = 0; q < VE; ++q) {
+            const float2 c = unpack2(acc[i + q][j / 2]);
+            e[q] = (j & 1) ? c.y : c.x;
+          }
+          *reinterpret_cast<float4 *>(to) = v;
+        }
+      }
+    }
+    __syncthreads();
+    const int cols = min(CW, nrem - c0);
+    constexpr int U = 8;
+    if (!along_n) {
+      const int row = tid % BM;
+      if (row < mrem) {
+        T *dm = D + mDs[row];
+        for (int c = tid / BM; c < cols; c += U * (NT / BM)) {
+          T d[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int n = c + u * (NT / BM);
+            d[u] = a.beta && n < cols ? dm[nDs[c0 + n]] : T();
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int n = c + u * (NT / BM);
+            if (n < cols) dm[nDs[c0 + n]] = emit(Cs[n * CP + row], d[u]);
+          }
+        }
+      }
+    } else {
+      const int n = tid % CW;
+      if (n < cols) {
+        T *dn = D + nDs[c0 + n];
+        const int rows = min(BM, mrem);
+        for (int r = tid / CW; r < rows; r += U * (NT / CW)) {
+          T d[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int m = r + u * (NT / CW);
+            d[u] = a.beta && m < rows ? dn[mDs[m]] : T();
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int m = r + u * (NT / CW);
+            if (m < rows) dn[mDs[m]] = emit(Cs[n * CP + m], d[u]);
+          }
+        }
       }
     }
   }
@@ -1411,9 +1470,9 @@ int64_t split_bytes(const KSplit &s, int kind, int64_t M, int64_t N, int64_t H, 
 // tiles of 64, K = 169: 55 / 25, 45 before the packed kernel; 105 tiles, K =
 // 459: 125 / 76; 131000 x 1, K = 20: 98 / 53; 3000 x 3000 x 3000: 5847 / 5799).
 // R4: 32 (4 x 4 sub-tiles) when one side is no wider, or when 64 x 64 tiles are
-// fewer than three for two SMs (64 / 32, us: 131000 x 1, K = 20: 37 / 23; 300 x
-// 300, K = 30: 18.4 / 11.1, 13.0 before the packed kernel; 512 x 512, K = 400: 41
-// / 25; 900 x 900 x 900, 225 tiles: 77 / 70 and, loads along k, 78 / 86), else 128
+// fewer than three for two SMs (64 / 32, us: 131000 x 1, K = 20: 25 / 21; 300 x
+// 300, K = 30: 14.6 / 10.5, 13.0 before the packed kernel; 512 x 512, K = 400: 39
+// / 25; 900 x 900 x 900, 225 tiles: 74 / 70 and, loads along k, 76 / 86), else 128
 // when two of those per SM exist and are mostly filled, else 64.  Results do not
 // depend on it.
 int gemm_edge(int kind, int64_t M, int64_t N, int64_t H, const KSplit &s) {
